@@ -2,18 +2,26 @@
 // which restates the reference's CgrCompressor (src/compressor.cpp:306-515).
 //
 // The host keeps the cheap O(n) parts (position order, prefix sum of the bit
-// lengths, small CSR); the device does the per-vertex work, one thread per
+// lengths, small CSR); the device does the per-vertex work, one warp per
 // compressed position:
-//   pass 1  walks the neighbour list once and plans both sections' 256-bit
-//           segments with the reference's rule (a segment closes when
-//           gamma(cnt + 1) + its bits + the next item's bits exceed 256; the
-//           final partial segment joins the last closed one, unpadded), giving
-//           the vertex's bit length, its segment counts and the interval
-//           section's length;
-//   pass 2  plans again and writes each segment once the next one has closed
-//           (so it is known not to be the last), re-reading its items from
-//           the neighbour list: no per-thread item buffers.  Non-last segments
-//           sit at fixed 256-bit steps, so every segment's position is known.
+//   pass 1  splits the neighbour list, 32 ids a step, into residuals and
+//           intervals (maximal runs of >= 4 consecutive ids), kept in a work
+//           array in the vertex's own range (residuals from its front,
+//           (left, end) pairs from its back; 4 ids or more make 2 words), then
+//           plans both sections' 256-bit segments with the reference's rule (a
+//           segment closes when gamma(cnt + 1) + its bits + the next item's
+//           bits exceed 256; the final partial segment joins the last closed
+//           one, unpadded): a warp scan of the items' bits finds how many fit.
+//           It gives the vertex's bit length, its item and segment counts and
+//           the interval section's length;
+//   pass 2  finds the same segments again and writes each: the lanes place
+//           their codes in the warp's shared words, which then go to the
+//           stream.  Non-last segments sit at fixed 256-bit steps and the last
+//           is known from pass 1, so every segment's position is known.
+// Bound by the chain of segments of the largest vertex (each start depends on
+// the segment before), about 300 cycles a segment.  One thread per position,
+// walking its list alone, held the GPU for the largest vertex's every id: R-MAT
+// scale 20 took 45 + 120 ms in the two passes (largest degree 64,612).
 // Words shared with the neighbouring vertices are OR-ed atomically into a
 // zeroed stream.  Only the reference's parameters (zeta k = 3, intervals of
 // >= 4, 256-bit segments for both sections) are supported.
@@ -39,250 +47,313 @@ __device__ __forceinline__ uint64_t int_2_nat(int64_t x) {
   return x >= 0 ? uint64_t(x) << 1 : uint64_t(-((x << 1) + 1));
 }
 
-// Items of one section in neighbour order: intervals (maximal runs of >= 4
-// consecutive ids: left, len) or residuals (the other ids one by one).  idx is
-// where a later scan restarts to yield this item first: an interval's run
-// start, or a residual's own index (a run entered in its middle is shorter,
-// so still residual).
-struct Scan {
-  const uint32_t *nb;
-  uint64_t deg, k, rk, re;
-  bool itv;
-  __device__ Scan(const uint32_t *nb_, uint64_t deg_, uint64_t k0, bool itv_)
-      : nb(nb_), deg(deg_), k(k0), rk(0), re(0), itv(itv_) {}
-  __device__ bool next(uint32_t &a, uint32_t &len, uint64_t &idx) {
-    for (;;) {
-      if (rk < re) {
-        idx = rk;
-        a = nb[rk++];
-        len = 1;
-        return true;
-      }
-      if (k >= deg) return false;
-      const uint64_t l = k;
-      uint64_t r = l + 1;
-      while (r < deg && uint64_t(nb[r - 1]) + 1 == uint64_t(nb[r])) r++;
-      k = r;
-      if (r - l >= kMinItv) {
-        if (itv) {
-          idx = l;
-          a = nb[l];
-          len = uint32_t(r - l);
-          return true;
-        }
-      } else if (!itv) {
-        rk = l;
-        re = r;
-      }
-    }
-  }
-};
+constexpr uint32_t kFull = 0xFFFFFFFFu;
+constexpr int kEncThreads = 256;
+constexpr uint32_t kEncWarps = kEncThreads / 32;
+// shared words per warp of a segment being written: below 512 bits plus the
+// longer count, from any bit of its first word
+constexpr uint32_t kSegWords = 24;
 
-// Code values of an item: first of its segment (relative to the node) or a
-// gap from the previous item of the section.
-struct Codes {
-  uint64_t first, gap;
+__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, uint32_t lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(kFull, v, o);
+    if (lane >= uint32_t(o)) v += t;
+  }
+  return v;
+}
+
+// Positions a warp takes from the work counter: the large ones (first in
+// position order, a hub can hold a warp for long) one by one, the others
+// kEncClaim at a time.
+constexpr uint32_t kEncClaim = 8;
+struct Claim {
+  uint64_t p, e;
 };
-__device__ __forceinline__ Codes item_codes(bool itv, uint32_t a, uint32_t len, uint32_t pa, uint32_t plen,
-                                            uint32_t node, bool has_prev) {
-  Codes c;
-  c.first = int_2_nat(int64_t(a) - int64_t(node));
-  if (!has_prev) c.gap = 0;
-  else if (itv) c.gap = uint64_t(int64_t(a) - int64_t(pa) - int64_t(plen) - 1);
-  else c.gap = uint64_t(int64_t(a) - int64_t(pa) - 1);
+__device__ __forceinline__ Claim claim_positions(unsigned long long *ctr, uint64_t n_large, uint64_t n_c,
+                                                 uint32_t lane) {
+  unsigned long long u = 0;
+  if (lane == 0) u = atomicAdd(ctr, 1ull);
+  u = __shfl_sync(kFull, u, 0);
+  Claim c;
+  if (u < n_large) {
+    c.p = u;
+    c.e = u + 1;
+  } else {
+    c.p = n_large + (u - n_large) * kEncClaim;
+    c.e = c.p + kEncClaim;
+  }
+  if (c.e > n_c) c.e = n_c;
   return c;
 }
-__device__ __forceinline__ uint32_t item_bits(bool itv, uint64_t code, uint32_t len) {
-  return itv ? gamma_size(code) + gamma_size(uint64_t(len) - kMinItv) : zeta3_size(code);
-}
 
-// plan_segments (cgr_format.cpp) as a stream.  close(start, cnt) is called
-// for every segment the rule closes.
-struct Plan {
-  uint32_t cnt = 0, nclosed = 0, last_cnt = 0;
-  uint64_t cur = 0, start = 0, last_bits = 0, tail_gap = 0;
-  template <class Close>
-  __device__ void feed(uint32_t fs, uint32_t gs, uint64_t idx, Close &&close) {
-    uint32_t sz = cnt == 0 ? fs : gs;
-    if (gamma_size(uint64_t(cnt) + 1) + cur + sz > kSegLen) {
-      close(start, cnt);
-      last_cnt = cnt;
-      last_bits = gamma_size(cnt) + cur;
-      nclosed++;
-      cnt = 0;
-      cur = 0;
-      tail_gap = 0;
-      sz = fs;
-    }
-    if (cnt == 0) start = idx;
-    cnt++;
-    cur += sz;
-    tail_gap += gs;
+// The items of one section of a vertex in the work array.
+struct Section {
+  const uint32_t *t;  // residuals: ids from the front; intervals: from the back
+  uint64_t deg, n;    // ids of the vertex, items of the section
+  uint32_t node;
+  bool itv;
+  __device__ __forceinline__ uint32_t left(uint64_t k) const { return itv ? t[deg - 1 - 2 * k] : t[k]; }
+  __device__ __forceinline__ uint32_t end(uint64_t k) const { return itv ? t[deg - 2 - 2 * k] : 0u; }
+  // item k's code value as the first of a segment or after item k - 1, and
+  // (intervals) its length code
+  __device__ __forceinline__ void codes(uint64_t k, bool first, uint64_t &code, uint64_t &len) const {
+    const uint32_t l = left(k);
+    len = itv ? uint64_t(end(k)) - l - kMinItv + 1 : 0;  // end: the last id
+    if (first) code = int_2_nat(int64_t(l) - int64_t(node));
+    else code = itv ? uint64_t(l) - end(k - 1) - 2 : uint64_t(l) - left(k - 1) - 1;
   }
-  __device__ uint32_t nseg() const { return nclosed ? nclosed : 1u; }
-  // section bits after its header: 256 per non-last segment, then the last
-  // (the last closed one with the tail's items appended as gaps)
-  __device__ uint64_t bits() const {
-    if (nclosed == 0) return gamma_size(cnt) + cur;
-    return uint64_t(nclosed - 1) * kSegLen + gamma_size(uint64_t(last_cnt) + cnt) + (last_bits - gamma_size(last_cnt)) +
-           tail_gap;
+  __device__ __forceinline__ uint32_t bits(uint64_t code, uint64_t len) const {
+    return itv ? gamma_size(code) + gamma_size(len) : zeta3_size(code);
   }
 };
 
-// Plans one section over the neighbour list; close is forwarded.
-template <class Close>
-__device__ Plan plan_section(const uint32_t *nb, uint64_t deg, uint32_t node, bool itv, Close &&close) {
-  Plan pl;
-  Scan sc(nb, deg, 0, itv);
-  uint32_t a, len, pa = 0, plen = 0;
-  uint64_t idx;
-  bool has_prev = false;
-  while (sc.next(a, len, idx)) {
-    const Codes c = item_codes(itv, a, len, pa, plen, node, has_prev);
-    pl.feed(item_bits(itv, c.first, len), has_prev ? item_bits(itv, c.gap, len) : 0u, idx, close);
-    pa = a;
-    plen = len;
-    has_prev = true;
+// The segment of the section that starts at item s: how many items fit it, and
+// their bits without the count.  Called by all lanes, same result in each.
+__device__ __forceinline__ uint32_t fit_segment(const Section &sec, uint64_t s, uint32_t lane, uint32_t &bits) {
+  uint32_t sum = 0, cnt = 0;
+  for (;;) {
+    const uint64_t k = s + cnt + lane;
+    const bool has = k < sec.n;
+    uint32_t b = 0;
+    if (has) {
+      uint64_t code, len;
+      sec.codes(k, k == s, code, len);
+      b = sec.bits(code, len);
+    }
+    const uint32_t incl = sum + warp_incl_scan(b, lane);
+    const uint32_t fits = __ballot_sync(kFull, has && gamma_size(uint64_t(cnt) + lane + 1) + incl <= kSegLen);
+    const uint32_t f = __popc(fits);  // the bits grow with every item: a prefix fits
+    if (f) sum = __shfl_sync(kFull, incl, f - 1);
+    cnt += f;
+    if (f < 32) break;
   }
-  return pl;
+  bits = sum;
+  return cnt;
 }
 
-// MSB-first bit writer into a zeroed word array; each word is OR-ed once,
-// atomically (the first and last words of a vertex are shared).
-struct Writer {
-  uint32_t *w;
-  uint64_t nwords;  // words outside the stream are never touched (bad is set)
-  uint64_t pos;
-  uint64_t word;
-  uint32_t acc;
-  bool has, bad;
-  __device__ void flush() {
-    if (has && acc) {
-      if (word < nwords) atomicOr(w + word, acc);
-      else bad = true;
-    }
-    has = false;
+// Bits of items [s, e) all coded as gaps.
+__device__ __forceinline__ uint64_t gap_bits(const Section &sec, uint64_t s, uint64_t e, uint32_t lane) {
+  uint32_t mine = 0;
+  for (uint64_t k = s + lane; k < e; k += 32) {
+    uint64_t code, len;
+    sec.codes(k, false, code, len);
+    mine += sec.bits(code, len);
   }
-  __device__ void emit(uint64_t wi, uint32_t bits) {
-    if (has && wi == word) {
-      acc |= bits;
-      return;
-    }
-    flush();
-    word = wi;
-    acc = bits;
-    has = true;
-  }
-  __device__ void put(uint64_t x, int len) {  // the low len (<= 64) bits of x
-    while (len > 0) {
-      const uint64_t wi = pos >> 5;
-      const int off = int(pos & 31);
-      const int take = min(32 - off, len);
-      const uint64_t chunk = (x >> (len - take)) & ((1ull << take) - 1);
-      emit(wi, uint32_t(chunk << (32 - off - take)));
-      pos += uint64_t(take);
-      len -= take;
-    }
-  }
-  __device__ void gamma(uint64_t x) {
-    const uint64_t y = x + 1;
-    const int len = sig_bit(y);
-    pos += uint64_t(len);
-    put(y, len + 1);
-  }
-  __device__ void zeta3(uint64_t x) {
-    const uint64_t y = x + 1;
-    const int h = sig_bit(y) / 3;
-    pos += uint64_t(h);
-    put(1, 1);
-    put(y, (h + 1) * 3);
-  }
-};
+  return __reduce_add_sync(kFull, mine);
+}
 
-// Writes the segment of cnt items starting at scan index start at position
-// at: gamma(cnt), the first item coded against the node, the rest as gaps.
-__device__ void write_segment(Writer &wr, uint64_t at, const uint32_t *nb, uint64_t deg, uint32_t node, bool itv,
-                              uint64_t start, uint32_t cnt) {
-  wr.pos = at;
-  wr.gamma(cnt);
-  Scan sc(nb, deg, start, itv);
-  uint32_t a, len, pa = 0, plen = 0;
-  uint64_t idx;
-  for (uint32_t i = 0; i < cnt && sc.next(a, len, idx); i++) {
-    const Codes c = item_codes(itv, a, len, pa, plen, node, i > 0);
-    const uint64_t code = i == 0 ? c.first : c.gap;
-    if (itv) {
-      wr.gamma(code);
-      wr.gamma(uint64_t(len) - kMinItv);
-    } else {
-      wr.zeta3(code);
-    }
-    pa = a;
-    plen = len;
+// plan_segments (cgr_format.cpp): segments and bits after the section's header.
+__device__ __forceinline__ void plan_section(const Section &sec, uint32_t lane, uint32_t &nseg, uint64_t &bits) {
+  uint64_t s = 0, last_s = 0;
+  uint32_t closed = 0, last_cnt = 0, last_bits = 0, b = 0, cnt = 0;
+  for (;;) {
+    cnt = fit_segment(sec, s, lane, b);
+    if (s + cnt >= sec.n) break;  // the open tail
+    last_s = s;
+    last_cnt = cnt;
+    last_bits = b;
+    closed++;
+    s += cnt;
+  }
+  if (closed == 0) {
+    nseg = 1;
+    bits = gamma_size(cnt) + b;
+  } else {
+    nseg = closed;
+    const uint64_t tail = gap_bits(sec, last_s + last_cnt, sec.n, lane);
+    bits = uint64_t(closed - 1) * kSegLen + gamma_size(sec.n - last_s) + last_bits + tail;
   }
 }
 
-// One section: plan it again, writing every closed segment once the next one
-// closes, then the last (merged with the tail) at the end.
-__device__ void write_section(Writer &wr, uint64_t base, const uint32_t *nb, uint64_t deg, uint32_t node, bool itv) {
-  bool pend = false;
-  uint64_t pstart = 0;
-  uint32_t pcnt = 0, pindex = 0, closed = 0;
-  const Plan pl = plan_section(nb, deg, node, itv, [&](uint64_t start, uint32_t cnt) {
-    if (pend) write_segment(wr, base + uint64_t(pindex) * kSegLen, nb, deg, node, itv, pstart, pcnt);
-    pend = true;
-    pstart = start;
-    pcnt = cnt;
-    pindex = closed++;
-  });
-  if (pend) write_segment(wr, base + uint64_t(pindex) * kSegLen, nb, deg, node, itv, pstart, pcnt + pl.cnt);
-  else write_segment(wr, base, nb, deg, node, itv, pl.start, pl.cnt);
+// Bits of x that end right before bit `end` of the words w (MSB first).
+__device__ __forceinline__ void or_bits(uint32_t *w, uint32_t end, uint64_t x) {
+  const uint32_t k = (end - 1) >> 5, sh = 31u - ((end - 1) & 31u);
+  const uint32_t a = uint32_t(x << sh), b = uint32_t(sh ? x >> (32 - sh) : x >> 32), c = sh ? uint32_t(x >> (64 - sh)) : 0u;
+  if (a) atomicOr(w + k, a);
+  if (b) atomicOr(w + k - 1, b);
+  if (c) atomicOr(w + k - 2, c);
 }
 
-struct NoClose {
-  __device__ void operator()(uint64_t, uint32_t) const {}
-};
+// gamma(x) at bit `at` of the zeroed stream, by one thread.
+__device__ __forceinline__ uint64_t put_gamma(uint32_t *words, uint64_t nwords, uint64_t at, uint64_t x, bool &bad) {
+  const uint64_t end = at + gamma_size(x);
+  if ((end + 31) / 32 > nwords) {
+    bad = true;
+    return end;
+  }
+  const uint64_t base = at >> 5;
+  or_bits(words + base, uint32_t(end - base * 32), x + 1);
+  return end;
+}
 
-// Pass 1: per compressed position, its bit length and the numbers pass 2
-// needs (segment counts, interval section length after its header).
-__global__ void k_encode_size(const uint64_t *row, const uint32_t *clm, const uint32_t *vertices, uint64_t n_c,
-                              uint64_t *bits, uint32_t *nseg_i, uint32_t *nseg_r, uint64_t *itv_bits, uint32_t *err) {
-  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n_c; i += uint64_t(gridDim.x) * blockDim.x) {
-    const uint32_t v = vertices[i];
-    const uint32_t *nb = clm + row[v];
-    const uint64_t deg = row[v + 1] - row[v];
-    for (uint64_t k = 1; k < deg; k++)
-      if (nb[k] <= nb[k - 1]) {  // the gap codes need strictly ascending lists
-        atomicOr(err, 1u);
-        break;
+// The segment of items [s, s + cnt) at bit `at`: gamma(cnt), the first item
+// coded against the node, the rest as gaps.  buf: kSegWords zeroed shared
+// words of the warp, left zeroed.  Returns the segment's end.
+__device__ __forceinline__ uint64_t write_segment(const Section &sec, uint64_t s, uint32_t cnt, uint64_t at,
+                                                  uint32_t *buf, uint32_t *words, uint64_t nwords, uint32_t lane,
+                                                  bool &bad) {
+  const uint32_t off = uint32_t(at) & 31u;
+  uint32_t end = off + gamma_size(cnt);
+  if (lane == 0) or_bits(buf, end, uint64_t(cnt) + 1);
+  for (uint32_t j0 = 0; j0 < cnt; j0 += 32) {
+    const uint32_t j = j0 + lane;
+    uint64_t code = 0, len = 0;
+    uint32_t b = 0;
+    if (j < cnt) {
+      sec.codes(s + j, j == 0, code, len);
+      b = sec.bits(code, len);
+    }
+    const uint32_t incl = warp_incl_scan(b, lane);
+    const uint32_t e = end + incl;
+    if (b && e <= kSegWords * 32) {
+      if (sec.itv) {
+        or_bits(buf, e - gamma_size(len), code + 1);
+        or_bits(buf, e, len + 1);
+      } else {  // h zeros, a one, the 3 (h + 1) bits of code + 1
+        or_bits(buf, e, (1ull << (b / 4 * 3)) | (code + 1));
       }
-    const Plan pi = plan_section(nb, deg, v, true, NoClose{});
-    const Plan pr = plan_section(nb, deg, v, false, NoClose{});
-    nseg_i[i] = pi.nseg();
-    nseg_r[i] = pr.nseg();
-    itv_bits[i] = pi.bits();
-    bits[i] = gamma_size(pi.nseg() - 1) + pi.bits() + gamma_size(pr.nseg() - 1) + pr.bits();
+    }
+    end += __shfl_sync(kFull, incl, 31);
+  }
+  __syncwarp();
+  const uint64_t w0 = at >> 5;
+  const uint32_t nw = (end + 31) / 32;
+  if (nw > kSegWords || w0 + nw > nwords) {
+    bad = true;
+  } else if (lane < nw) {
+    // the first and last words are shared with what lies beside the segment
+    const uint32_t x = buf[lane];
+    if (lane == 0 || lane == nw - 1) {
+      if (x) atomicOr(words + w0 + lane, x);
+    } else {
+      words[w0 + lane] = x;
+    }
+  }
+  __syncwarp();
+  if (lane < kSegWords) buf[lane] = 0u;
+  __syncwarp();
+  return at - off + end;
+}
+
+__device__ __forceinline__ uint64_t write_section(const Section &sec, uint64_t base, uint32_t nseg, uint32_t *buf,
+                                                  uint32_t *words, uint64_t nwords, uint32_t lane, bool &bad) {
+  uint64_t s = 0, end = base;
+  for (uint32_t k = 0; k < nseg && !bad; k++) {
+    uint32_t b;
+    const uint32_t cnt = k + 1 < nseg ? fit_segment(sec, s, lane, b) : uint32_t(sec.n - s);
+    end = write_segment(sec, s, cnt, base + uint64_t(k) * kSegLen, buf, words, nwords, lane, bad);
+    s += cnt;
+  }
+  return end;
+}
+
+struct EncodeArgs {
+  const uint64_t *row;
+  const uint32_t *clm, *vertices;
+  uint32_t *work;           // one word per arc: the split lists
+  uint64_t n_c, n_large;
+  uint64_t *bits, *itv_bits;
+  uint32_t *nseg_i, *nseg_r, *nres, *nitv;
+  unsigned long long *ctr;  // work counter
+  uint32_t *err;
+};
+
+// Pass 1: per compressed position its split lists, its bit length and the
+// numbers pass 2 needs (item and segment counts, interval section length
+// after its header).
+__global__ void __launch_bounds__(kEncThreads) k_encode_size(EncodeArgs a) {
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  for (;;) {
+    const Claim c = claim_positions(a.ctr, a.n_large, a.n_c, lane);
+    if (c.p >= a.n_c) break;
+    for (uint64_t i = c.p; i < c.e; i++) {
+      const uint32_t v = a.vertices[i];
+      const uint32_t *nb = a.clm + a.row[v];
+      uint32_t *t = a.work + a.row[v];
+      const uint64_t deg = a.row[v + 1] - a.row[v];
+      // cons bit j: id j continues the run of id j - 1.  An id belongs to an
+      // interval when three continuations in a row touch it.
+      uint32_t cur = lane < deg ? nb[lane] : 0u, cons_before = 0;
+      uint64_t nr = 0, ns = 0, ne = 0;
+      bool bad = false;
+      const auto cons_of = [&](uint32_t x, uint32_t left, uint64_t k) {
+        const uint32_t up = __shfl_up_sync(kFull, x, 1);
+        const uint32_t prev = lane ? up : left;
+        const bool has = k < deg && k > 0;
+        bad |= has && x <= prev;  // the gap codes need strictly ascending lists
+        return __ballot_sync(kFull, has && uint64_t(prev) + 1 == uint64_t(x));
+      };
+      uint32_t cons = cons_of(cur, 0u, lane);
+      for (uint64_t k0 = 0; k0 < deg; k0 += 32) {
+        const uint64_t k = k0 + lane, kn = k + 32;
+        const uint32_t nxt = kn < deg ? nb[kn] : 0u;
+        const uint32_t cons_next = cons_of(nxt, __shfl_sync(kFull, cur, 31), kn);
+        // bit 4 + j: id k0 + j
+        const uint64_t x = (uint64_t(cons_before >> 28)) | (uint64_t(cons) << 4) | (uint64_t(cons_next & 15u) << 36);
+        const uint64_t t3 = x & (x >> 1) & (x >> 2);
+        const uint32_t in = uint32_t(((t3 >> 1) | t3 | (t3 << 1) | (t3 << 2)) >> 4);
+        const uint32_t valid = deg - k0 >= 32 ? kFull : (1u << uint32_t(deg - k0)) - 1u;
+        const uint32_t res = ~in & valid, starts = in & ~cons & valid, ends = in & ~uint32_t(x >> 5) & valid;
+        if ((res >> lane) & 1u) t[nr + __popc(res & lt)] = cur;
+        if ((starts >> lane) & 1u) t[deg - 1 - 2 * (ns + __popc(starts & lt))] = cur;
+        if ((ends >> lane) & 1u) t[deg - 2 - 2 * (ne + __popc(ends & lt))] = cur;
+        nr += __popc(res);
+        ns += __popc(starts);
+        ne += __popc(ends);
+        cons_before = cons;
+        cons = cons_next;
+        cur = nxt;
+      }
+      if (__any_sync(kFull, bad)) {
+        if (lane == 0) atomicOr(a.err, 1u);
+        continue;
+      }
+      __syncwarp();  // the lists are read by other lanes below
+      uint32_t nsi, nsr;
+      uint64_t bi, br;
+      plan_section(Section{t, deg, ns, v, true}, lane, nsi, bi);
+      plan_section(Section{t, deg, nr, v, false}, lane, nsr, br);
+      if (lane == 0) {
+        a.nres[i] = uint32_t(nr);
+        a.nitv[i] = uint32_t(ns);
+        a.nseg_i[i] = nsi;
+        a.nseg_r[i] = nsr;
+        a.itv_bits[i] = bi;
+        a.bits[i] = gamma_size(nsi - 1) + bi + gamma_size(nsr - 1) + br;
+      }
+    }
   }
 }
 
 // Pass 2: writes every compressed position at its offset.
-__global__ void k_encode_write(const uint64_t *row, const uint32_t *clm, const uint32_t *vertices, uint64_t n_c,
-                               const uint64_t *offsets, const uint32_t *nseg_i, const uint32_t *nseg_r,
-                               const uint64_t *itv_bits, uint32_t *words, uint64_t nwords, uint32_t *err) {
-  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n_c; i += uint64_t(gridDim.x) * blockDim.x) {
-    const uint32_t v = vertices[i];
-    const uint32_t *nb = clm + row[v];
-    const uint64_t deg = row[v + 1] - row[v];
-    Writer wr{words, nwords, offsets[i], 0, 0, false, false};
-    wr.gamma(nseg_i[i] - 1);
-    const uint64_t ibase = wr.pos;
-    write_section(wr, ibase, nb, deg, v, true);
-    wr.pos = ibase + itv_bits[i];
-    wr.gamma(nseg_r[i] - 1);
-    const uint64_t rbase = wr.pos;
-    write_section(wr, rbase, nb, deg, v, false);
-    wr.flush();
-    if (wr.bad || wr.pos != offsets[i + 1]) atomicOr(err, 2u);
+__global__ void __launch_bounds__(kEncThreads) k_encode_write(EncodeArgs a, const uint64_t *offsets, uint32_t *words,
+                                                              uint64_t nwords) {
+  __shared__ uint32_t sbuf[kEncWarps * kSegWords];
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t *buf = sbuf + (threadIdx.x >> 5) * kSegWords;
+  if (lane < kSegWords) buf[lane] = 0u;
+  __syncwarp();
+  for (;;) {
+    const Claim c = claim_positions(a.ctr, a.n_large, a.n_c, lane);
+    if (c.p >= a.n_c) break;
+    for (uint64_t i = c.p; i < c.e; i++) {
+      const uint32_t v = a.vertices[i];
+      const uint32_t *t = a.work + a.row[v];
+      const uint64_t deg = a.row[v + 1] - a.row[v];
+      const uint32_t nsi = a.nseg_i[i], nsr = a.nseg_r[i];
+      const uint64_t ibase = offsets[i] + gamma_size(nsi - 1), rhead = ibase + a.itv_bits[i],
+                     rbase = rhead + gamma_size(nsr - 1);
+      bool bad = false;
+      if (lane == 0) {
+        put_gamma(words, nwords, offsets[i], nsi - 1, bad);
+        put_gamma(words, nwords, rhead, nsr - 1, bad);
+      }
+      bad = __any_sync(kFull, bad);
+      const uint64_t iend = write_section(Section{t, deg, a.nitv[i], v, true}, ibase, nsi, buf, words, nwords, lane, bad);
+      const uint64_t rend = write_section(Section{t, deg, a.nres[i], v, false}, rbase, nsr, buf, words, nwords, lane, bad);
+      if (lane == 0 && (bad || iend != rhead || rend != offsets[i + 1])) atomicOr(a.err, 2u);
+    }
   }
 }
 
@@ -369,12 +440,15 @@ void cgr_encode_gpu(const CsrView &g, const CgrParams &p, int small_thresh, int 
   ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "attribute");
   if (n_c) {
     DevBuf<uint64_t> d_bits(n_c), d_itv(n_c), d_off(n_c + 1);
-    DevBuf<uint32_t> d_vert(n_c), d_nsi(n_c), d_nsr(n_c), d_err(1);
+    DevBuf<uint32_t> d_vert(n_c), d_nsi(n_c), d_nsr(n_c), d_nres(n_c), d_nitv(n_c), d_work(m), d_err(1);
+    DevBuf<unsigned long long> d_ctr(2);  // a work counter per pass
+    ck(cudaMemset(d_ctr.p, 0, 16), "clear work counters");
     ck(cudaMemcpy(d_vert.p, out.vertices.data(), n_c * 4, cudaMemcpyHostToDevice), "upload positions");
     ck(cudaMemset(d_err.p, 0, 4), "clear error");
-    const int threads = 128;
-    const int blocks = int(std::min<uint64_t>((n_c + threads - 1) / threads, uint64_t(sms) * 16));
-    k_encode_size<<<blocks, threads>>>(d_row.p, d_clm.p, d_vert.p, n_c, d_bits.p, d_nsi.p, d_nsr.p, d_itv.p, d_err.p);
+    EncodeArgs ea{d_row.p, d_clm.p, d_vert.p, d_work.p, n_c, out.n_large, d_bits.p, d_itv.p,
+                  d_nsi.p, d_nsr.p, d_nres.p, d_nitv.p, d_ctr.p, d_err.p};
+    const int blocks = int(std::min<uint64_t>((n_c + kEncWarps - 1) / kEncWarps, uint64_t(sms) * 8));
+    k_encode_size<<<blocks, kEncThreads>>>(ea);
     ck(cudaGetLastError(), "size pass");
     std::vector<uint64_t> bits(n_c);
     ck(cudaMemcpy(bits.data(), d_bits.p, n_c * 8, cudaMemcpyDeviceToHost), "read sizes");
@@ -387,8 +461,8 @@ void cgr_encode_gpu(const CsrView &g, const CgrParams &p, int small_thresh, int 
     DevBuf<uint32_t> d_words(nwords);
     ck(cudaMemset(d_words.p, 0, nwords * 4), "clear stream");
     ck(cudaMemcpy(d_off.p, out.offsets.data(), (n_c + 1) * 8, cudaMemcpyHostToDevice), "upload offsets");
-    k_encode_write<<<blocks, threads>>>(d_row.p, d_clm.p, d_vert.p, n_c, d_off.p, d_nsi.p, d_nsr.p, d_itv.p,
-                                        d_words.p, nwords, d_err.p);
+    ea.ctr = d_ctr.p + 1;
+    k_encode_write<<<blocks, kEncThreads>>>(ea, d_off.p, d_words.p, nwords);
     ck(cudaGetLastError(), "write pass");
     ck(cudaMemcpy(&err, d_err.p, 4, cudaMemcpyDeviceToHost), "read error");
     if (err) throw std::runtime_error("cgr_encode_gpu: a vertex's bits did not end at its offset");
