@@ -1257,20 +1257,27 @@ __global__ void __launch_bounds__(kThreads, 4) k_decode_two_pass(IterArgs a) {
   const uint64_t keep_pol = l2_evict_last_policy();
   busy_mark(a, 0, false);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  // Decode groups come from the iteration's work queue, kGroupClaim at a
+  // Decode groups come from the iteration's work queue, group_claim at a
   // time, each warp's next claim made one ahead so that its atomic is off the
   // critical path.  A fixed grid-stride assignment left SMs idle for 28 % of
   // the kernel at R-MAT scale 22 (ncu: 0.66 ms of SM activity in a 0.92 ms
   // launch): groups whose interval segments expand thousands of ids finished
   // late on the warps that drew them.
+  // With one group a claim (group_claim, group_base: a graph of few groups per warp)
+  // every warp's first group is its own instead (warp w of block b takes group
+  // w * gridDim.x + b, so that neighbouring groups, a hub's among them, start
+  // on different SMs): when the first two claims came from the queue with 4
+  // groups each, most warps had no work while the first ones ran 8 groups in
+  // a row (pre-pass at R-MAT scale 16 / 18 / 20: 111 / 144 / 258 us, now 51 /
+  // 82 / 168 us).
   uint32_t *gctr = a.work + kWorkCounters * (a.it_dev ? c.it : 0u) + kWqGroups;
   const auto claim = [&]() {
     uint32_t x = 0;
-    if (lane == 0) x = atomicAdd(gctr, kGroupClaim);
+    if (lane == 0) x = a.group_base + atomicAdd(gctr, a.group_claim);
     return __shfl_sync(kFull, x, 0);
   };
-  uint32_t gi = claim();
-  uint32_t ahead = claim(), cend = gi + kGroupClaim;
+  uint32_t gi = a.group_base ? warp * gridDim.x + blockIdx.x : claim();
+  uint32_t ahead = claim(), cend = gi + a.group_claim;
   uint32_t *wspan = sspan + (kStage == 2 ? warp * 2 * kSpanWords : 0);
   uint64_t *wbar = sbar + (kStage == 2 ? warp * 2 : 0);
   uint32_t phase[2] = {0u, 0u};
@@ -1304,7 +1311,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_decode_two_pass(IterArgs a) {
       gi++;
     } else {
       gi = ahead;
-      cend = ahead + kGroupClaim;
+      cend = ahead + a.group_claim;
       ahead = claim();
     }
   };

@@ -55,8 +55,13 @@ struct DecodeGroup {
 // the ids' top bits) beat 768 by 1.5 %; 1280 and 1536 shrink L1 and lose 3 %
 // and 13 % (R-MAT scale 24)
 constexpr uint32_t kDecodeWindow = 1024;
-// decode groups a warp of the pre-pass claims from its work queue at once
+// Decode groups a warp of the pre-pass claims from its work queue at once: 4
+// where every resident warp gets several such claims, else 1, so that every
+// warp gets work (a claim's atomic is off the critical path either way).
 constexpr uint32_t kGroupClaim = 4;
+inline uint32_t group_claim_for(uint32_t n_groups, int grid) {
+  return uint64_t(n_groups) >= uint64_t(grid) * kWarps * kGroupClaim * 4 ? kGroupClaim : 1u;
+}
 // lpa_tune.gather_cache 0: the pre-pass reads the labels of ids below this
 // through L1 (32 KB of labels), the others through L2 only
 constexpr uint32_t kHotIds = 8192;
@@ -124,6 +129,8 @@ struct IterArgs {
   uint32_t n_light;
   const DecodeGroup *groups;    // two-pass pre-pass work: 32 segments per group
   uint32_t n_groups;
+  uint32_t group_claim;         // groups a warp claims at once (group_claim_for)
+  uint32_t group_base;          // with one group a claim: the warps' own first groups, else 0
   const uint4 *pidx;            // per compressed position: {ibase - offset, rbase - offset, nseg_i, nseg_r}
   const BlockItem *cblock;      // count-pass block items (largest first)
   uint32_t n_cblock;

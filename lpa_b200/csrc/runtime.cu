@@ -606,6 +606,8 @@ static IterArgs iter_args(lpa_handle *h, unsigned long long *changed, uint32_t *
   a.n_light = h->n_light;
   a.groups = h->d_groups;
   a.n_groups = h->n_groups;
+  a.group_claim = group_claim_for(h->n_groups, h->grid_decode);
+  a.group_base = a.group_claim == 1 ? uint32_t(h->grid_decode) * kWarps : 0;
   a.cblock = h->d_cblock;
   a.n_cblock = h->n_cblock;
   a.cwarp = h->d_citems;
@@ -727,6 +729,8 @@ static void enqueue_streamed_iteration(lpa_handle *h, unsigned long long *change
     a.n_light = r.n_light;
     a.groups = r.groups;
     a.n_groups = r.n_groups;
+    a.group_claim = group_claim_for(r.n_groups, r.grid_decode);
+    a.group_base = a.group_claim == 1 ? uint32_t(r.grid_decode) * kWarps : 0;
     a.cblock = r.cblock;
     a.n_cblock = r.n_cblock;
     a.cwarp = r.cwarp;
