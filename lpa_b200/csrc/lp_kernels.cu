@@ -13,7 +13,7 @@
 //     parallel (one thread each), ids are staged in shared memory, labels are
 //     gathered with many loads in flight, then counted in a shared (or global)
 //     table or the sketch;
-//   * light chunks of up to 32 consecutive positions, taken by one warp: each
+//   * light items of up to 32 consecutive positions, taken by one warp: each
 //     lane decodes one vertex into the warp's staging area, the warp gathers
 //     all labels at once, then counts per vertex (one vertex per round, or
 //     several vertices per round for degrees <= 32).
@@ -949,7 +949,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_iterate(IterArgs a) {
     }
     __syncthreads();
     next = sh.item;
-    const uint32_t s = a.heavy[i].tag;
+    const uint32_t s = a.heavy[i].seg;
     const bool from_scratch = a.seg_var[s] == kVarTwoPass;
     const Seg sg = a.segs[s];
     const long long t0 = clock64();
@@ -959,28 +959,34 @@ __global__ void __launch_bounds__(kThreads, 2) k_iterate(IterArgs a) {
                 (unsigned long long)((clock64() - t0) * kWarps * a.cw_iterate));
   }
 
-  // light chunks: a warp claims 4 consecutive chunks at a time, prefetches
-  // the last 3 into L2 at once and runs them in order
-  for (;;) {
-    uint32_t i0 = 0;
-    if (lane == 0) i0 = atomicAdd(qctr + 1, 4u);
-    i0 = __shfl_sync(kFull, i0, 0);
-    if (i0 >= a.n_light) break;
-    WorkItem wi{};
-    if (lane < 4 && i0 + lane < a.n_light) wi = a.light[i0 + lane];
-    if (lane >= 1 && lane < 4 && i0 + lane < a.n_light)
-      prefetch_l2(reinterpret_cast<const void *>(wi.pf_addr), wi.pf_bytes);
-    for (uint32_t k = 0; k < 4 && i0 + k < a.n_light; k++) {
-      const uint32_t item = __shfl_sync(kFull, wi.tag, k);
-      const uint32_t s = item >> 3;
-      const Seg sg = a.segs[s];
-      const uint32_t p0 = sg.begin + (item & 7u) * 32u;
-      const long long t0 = clock64();
-      light_chunk(a, c, wstage, wslots, wepoch, s, p0, min(sg.end, p0 + 32u), a.seg_var[s], changed);
-      if (a.seg_cycles && lane == 0)
-        atomicAdd(reinterpret_cast<unsigned long long *>(a.seg_cycles + s),
-                  (unsigned long long)((clock64() - t0) * a.cw_iterate));
+  // light items, one at a time: a warp's first is its own, the others come
+  // from the queue.  It knows its next item while it runs one (claimed a round
+  // earlier, its range prefetched into L2).
+  const uint32_t own = gridDim.x * kWarps;
+  const auto claim = [&]() {
+    uint32_t x = 0;
+    if (lane == 0) x = atomicAdd(qctr + 1, 1u);
+    return own + __shfl_sync(kFull, x, 0);
+  };
+  WorkItem wi{};
+  uint32_t cur = warp * gridDim.x + blockIdx.x, ahead = a.n_light > own ? claim() : a.n_light;
+  if (cur < a.n_light) wi = a.light[cur];
+  while (cur < a.n_light) {
+    WorkItem wn{};
+    if (ahead < a.n_light) {
+      wn = a.light[ahead];
+      if (lane == 0) prefetch_l2(reinterpret_cast<const void *>(wn.pf_addr), wn.pf_bytes);
     }
+    uint32_t x = 0;  // the claim after that; not waited for until the item is done
+    if (lane == 0 && ahead < a.n_light) x = atomicAdd(qctr + 1, 1u);
+    const long long t0 = clock64();
+    light_chunk(a, c, wstage, wslots, wepoch, wi.seg, wi.p0, wi.p0 + wi.np, a.seg_var[wi.seg], changed);
+    if (a.seg_cycles && lane == 0)
+      atomicAdd(reinterpret_cast<unsigned long long *>(a.seg_cycles + wi.seg),
+                (unsigned long long)((clock64() - t0) * a.cw_iterate));
+    cur = ahead;
+    wi = wn;
+    ahead = ahead < a.n_light ? own + __shfl_sync(kFull, x, 0) : ahead;
   }
   busy_mark(a, 2, true);
   flush_changed(c.changed, changed);
@@ -1081,8 +1087,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_batch(BatchArgs b) {
       // a tiny segment: one thread per position (<= 256 positions)
       if (sg.begin + t < sg.end) changed += packed_vertex(ia, c, sg.begin + t, stage + t * kPackedMaxDeg);
     } else {
-      const uint32_t p0 = sg.begin + warp * 32u;  // light segments hold at most 8 chunks
-      if (p0 < sg.end) light_chunk(ia, c, wstage, wslots, wepoch, s, p0, min(sg.end, p0 + 32u), v, changed);
+      // light segments hold at most 256 positions: the same share for every warp
+      const uint32_t per = (sg.end - sg.begin + kWarps - 1) / kWarps, p0 = sg.begin + warp * per;
+      if (p0 < sg.end) light_chunk(ia, c, wstage, wslots, wepoch, s, p0, min(sg.end, p0 + per), v, changed);
     }
     flush_changed(c.changed, changed);
     __threadfence();

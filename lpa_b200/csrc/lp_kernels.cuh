@@ -35,11 +35,14 @@ struct Seg {
 };
 
 // A work item with the device range it will read, so a warp or block can
-// prefetch items it has claimed but not started.
+// prefetch items it has claimed but not started.  Heavy: one segment by a
+// block; light: positions [p0, p0 + np) of a segment by a warp, as many as one
+// batch of its staging area takes (32 positions, kWarpStage labels).
 struct WorkItem {
-  uint32_t tag;        // heavy: segment id; light: (segment << 3) | 32-position chunk
+  uint32_t seg;
   uint32_t pf_bytes;   // bytes of the range to prefetch
   uint64_t pf_addr;    // device address of the range (bitstream bits, small-CSR ids or scratch ids)
+  uint32_t p0, np;
 };
 
 // Work of the two-pass pre-pass: nlanes (<= 32) consecutive segments of the
@@ -125,7 +128,7 @@ struct IterArgs {
   const uint8_t *seg_var;       // variant per segment
   const WorkItem *heavy;        // block work items (one segment each), largest first
   uint32_t n_heavy;
-  const WorkItem *light;        // warp work items (32-position chunks)
+  const WorkItem *light;        // warp work items
   uint32_t n_light;
   const DecodeGroup *groups;    // two-pass pre-pass work: 32 segments per group
   uint32_t n_groups;

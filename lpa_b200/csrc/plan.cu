@@ -73,7 +73,7 @@ __device__ __forceinline__ bool warp_capable(const SegDev &si, uint32_t cms) {
 
 // The device range a work item over positions [p0, p1) will read (for its
 // L2 prefetch): the bitstream words, the scratch labels or the small-CSR ids.
-__device__ WorkItem make_item(const PlanArgs &a, uint32_t tag, uint32_t p0, uint32_t p1, bool two_pass) {
+__device__ WorkItem make_item(const PlanArgs &a, uint32_t s, uint32_t p0, uint32_t p1, bool two_pass) {
   uint64_t addr = 0, bytes = 0;
   if (p0 < a.n_c) {
     if (two_pass) {
@@ -89,7 +89,7 @@ __device__ WorkItem make_item(const PlanArgs &a, uint32_t tag, uint32_t p0, uint
     addr = reinterpret_cast<uint64_t>(a.small_nbr + b);
     bytes = (e - b) * 4;
   }
-  return WorkItem{tag, uint32_t(bytes < 0x7FFFFFFFull ? bytes : 0x7FFFFFFFull), addr};
+  return WorkItem{s, uint32_t(bytes < 0x7FFFFFFFull ? bytes : 0x7FFFFFFFull), addr, p0, p1 - p0};
 }
 
 // One segment's items.  kEmit false: counts them (and marks the positions
@@ -159,12 +159,17 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
       c[kLPacked]++;
     }
   } else {
-    const uint32_t chunks = (si.end - si.begin + 31) / 32;
-    for (uint32_t k = 0; k < chunks; k++) {
-      const uint32_t p0 = si.begin + 32 * k, p1 = min(si.end, p0 + 32);
-      if (kEmit) a.light[o[kLLight] + k] = make_item(a, (s << 3) | k, p0, p1, tp);
+    // as many positions as one batch of a warp takes: with 32 positions
+    // whatever their degrees, a warp had up to 32,000 labels in one item, and
+    // took four such items at a time
+    uint32_t p = si.begin;
+    while (p < si.end) {
+      uint32_t q = p, labels = 0;
+      while (q < si.end && q - p < 32 && (q == p || labels + a.deg[q] <= kWarpStage)) labels += a.deg[q++];
+      if (kEmit) a.light[o[kLLight] + c[kLLight]] = make_item(a, s, p, q, tp);
+      c[kLLight]++;
+      p = q;
     }
-    c[kLLight] = chunks;
   }
   if (tp && si.region == 0) {
     // decode groups: 32 consecutive 256-bit segments of the positions,
