@@ -281,7 +281,7 @@ void train(lpa_handle *h) {
   k_mlp_features<<<blocks, threads, 0, h->stream>>>(L->d_feat, h->d_segs, h->d_seg_changed_prev, it_feat, L->d_X,
                                                       ns);
   k_mlp_targets<<<blocks, threads, 0, h->stream>>>(h->d_seg_cycles, L->d_T, ns);
-  cudaMemcpyAsync(L->d_var, h->d_seg_var, ns, cudaMemcpyDeviceToDevice, h->stream);
+  cudaMemcpyAsync(L->d_var, h->variant.data(), ns, cudaMemcpyHostToDevice, h->stream);
   const uint32_t nb = std::min<uint32_t>(kBatch, ns);
   const int gb = int(std::min<uint32_t>((nb + 127) / 128, 64));
   cudaMemsetAsync(L->d_loss, 0, sizeof(float), h->stream);

@@ -103,7 +103,6 @@ struct BlockSh {
   uint64_t red[kWarps];
   uint64_t ibase, rbase, last_end;
   uint32_t nseg_i, nseg_r, item, items, bad;
-  uint32_t spill_n;  // labels a hub has written to its spill area so far
   uint32_t hepoch;  // epoch of the block's exact table
 };
 
@@ -186,28 +185,6 @@ struct CmsAddSink {
   }
 };
 
-// Passes every label on to `inner` and also writes it to spill[0..cap), one
-// reservation per 32 labels (warp-synchronous, like every sink): the sketch's
-// second pass over a decoded hub then reads the labels back instead of
-// decoding the hub again.
-template <class Sink>
-struct SpillSink {
-  Sink inner;
-  uint32_t *spill;
-  uint32_t cap;
-  uint32_t *count;  // shared
-  __device__ __forceinline__ void operator()(bool ok, uint32_t lab) const {
-    inner(ok, lab);
-    const uint32_t m = __ballot_sync(kFull, ok);
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t base = 0;
-    if (lane == 0 && m) base = atomicAdd(count, uint32_t(__popc(m)));
-    base = __shfl_sync(kFull, base, 0);
-    const uint32_t at = base + uint32_t(__popc(m & ((1u << lane) - 1u)));
-    if (ok && at < cap) spill[at] = lab;
-  }
-};
-
 // Second sketch pass: read-only, so every lane looks up its own label.
 struct CmsBestSink {
   const uint32_t *cms;
@@ -248,25 +225,6 @@ __device__ __forceinline__ void block_gather_from(uint32_t *stage, const uint32_
     for (int u = 0; u < 4; u++) {
       const uint32_t k = k0 + u * kThreads;
       if (k < total) stage[k] = v[u];
-    }
-  }
-}
-
-// Labels src[0..total) from global memory (a hub's spill area), 4 loads per
-// thread in flight, into sink; block-synchronous.
-template <class Sink>
-__device__ __forceinline__ void block_consume_global(const uint32_t *src, uint32_t total, const Sink &sink) {
-  for (uint32_t k0 = 0; k0 < total; k0 += 4 * kThreads) {
-    uint32_t v[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const uint32_t k = k0 + u * kThreads + threadIdx.x;
-      v[u] = k < total ? __ldcg(src + k) : 0u;
-    }
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const uint32_t k = k0 + u * kThreads + threadIdx.x;
-      sink(k < total, v[u]);
     }
   }
 }
@@ -516,23 +474,11 @@ __device__ void heavy_vertex(const IterArgs &a, const Ctx &c, BlockSh &sh, uint3
     for (uint32_t i = t; i < kCmsDepth * kCmsWidth; i += kThreads) cms[i] = 0u;
     __syncthreads();
     const uint32_t lb = label_base(a, node);
-    // a hub decoded here keeps its labels in the block's spill area (when it
-    // fits), so the second pass reads them back instead of decoding again
-    const bool decoded = p < g.n_c && !from_scratch;
-    uint32_t *spill = (a.hub_spill && decoded && d <= a.hub_spill_words)
-                          ? a.hub_spill + uint64_t(blockIdx.x) * a.hub_spill_words
-                          : nullptr;
-    if (t == 0) sh.spill_n = 0;
-    __syncthreads();
-    const CmsAddSink s1{cms, a.seeds, lb};
-    const bool staged = spill ? heavy_produce(a, c, sh, stage, p, node, d, from_scratch,
-                                              SpillSink<CmsAddSink>{s1, spill, d, &sh.spill_n})
-                              : heavy_produce(a, c, sh, stage, p, node, d, from_scratch, s1);
+    const bool staged = heavy_produce(a, c, sh, stage, p, node, d, from_scratch, CmsAddSink{cms, a.seeds, lb});
     __syncthreads();
     CmsBestSink s2{cms, a.seeds, lb, &best};
     if (staged) heavy_consume_staged(sh, stage, s2);
     else if ((p >= g.n_c || from_scratch) && d <= kStage) block_consume_stage(stage, d, s2);
-    else if (spill && sh.spill_n == d) block_consume_global(spill, d, s2);
     else heavy_produce(a, c, sh, stage, p, node, d, from_scratch, s2);
     __syncthreads();
     // leave no counter behind that an epoch table could read as its own slot
@@ -1041,7 +987,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_batch(BatchArgs b) {
     const uint32_t gi = uint32_t(e >> 44), it = uint32_t(e >> 32) & 0xFFFu, s = uint32_t(e);
     if (t == 0) {
       const BatchGraph &bg = b.graphs[gi];
-      ia = IterArgs{};  // every field this launch does not use is zero (null): no hub spill, no scratch
+      ia = IterArgs{};  // every field this launch does not use is zero (null): no scratch
       ia.g = bg.g;
       ia.labs0 = bg.labs0;
       ia.labs1 = bg.labs1;
@@ -2086,7 +2032,7 @@ __global__ void k_decode_positions(DecodeArgs a) {
     const uint64_t p = a.pos_list ? a.pos_list[i] : a.pos_begin + i;
     if (p >= g.n_c) continue;
     uint32_t *dst = a.out + a.arc_off[p];
-    const uint64_t d = a.arc_off[p + 1] - a.arc_off[p];
+    const uint64_t d = g.deg[p];
     uint64_t k = 0;
     const int64_t r = walk_vertex(GWords{g.words}, g.offsets[p], g.offsets[p + 1], g.vertices[p], g.n,
                                   [&](uint32_t id) {

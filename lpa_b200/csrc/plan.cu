@@ -42,7 +42,7 @@ struct PlanArgs {
   const uint32_t *deg;       // by position
   const uint32_t *vertices;  // by position
   const uint4 *pidx;         // per compressed position (two-pass plans only)
-  const uint64_t *arc_off;   // n + 1 (two-pass plans only)
+  const uint64_t *arc_off;   // n_c + 1 (two-pass plans only)
   const uint64_t *offsets;   // n_c + 1
   const uint32_t *small_off; // n - n_c + 1
   const uint32_t *words, *small_nbr, *scratch;
@@ -78,7 +78,7 @@ __device__ WorkItem make_item(const PlanArgs &a, uint32_t s, uint32_t p0, uint32
   if (p0 < a.n_c) {
     if (two_pass) {
       addr = reinterpret_cast<uint64_t>(a.scratch + a.arc_off[p0]);
-      bytes = (a.arc_off[p1] - a.arc_off[p0]) * 4;
+      for (uint32_t p = p0; p < p1; p++) bytes += uint64_t(a.deg[p]) * 4;
     } else {
       const uint64_t b = a.offsets[p0] >> 5, e = a.offsets[p1] >> 5;
       addr = reinterpret_cast<uint64_t>(a.words + b);

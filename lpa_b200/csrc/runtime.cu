@@ -223,18 +223,8 @@ static void build_segments(lpa_handle *h) {
 // few launches and one copy of the list sizes, not a host loop over n.
 static void upload_range_lists(lpa_handle *h);
 
-// The block path's sketch hubs keep their labels between the sketch's two
-// passes in a per-block spill area (at most 2 GiB in all; larger hubs decode
-// twice), allocated once a plan gives k_iterate heavy items.
-static void ensure_hub_spill(lpa_handle *h) {
-  if (h->d_hub_spill || h->n_heavy == 0 || h->max_sketch_deg == 0) return;
-  const uint64_t per_block = std::min<uint64_t>(h->max_sketch_deg, (2ull << 30) / 4 / uint64_t(std::max(1, h->grid)));
-  h->d_hub_spill = dalloc<uint32_t>(h, per_block * uint64_t(h->grid), "hub spill");
-  h->hub_spill_words = uint32_t(per_block);
-}
-
 static void upload_lists(lpa_handle *h) {
-  h2d(h, h->d_seg_var, h->variant.data(), h->variant.size(), "upload variants");
+  h2d(h, h->d_seg_var, h->run_variant.data(), h->run_variant.size(), "upload variants");
   if (h->streamed) {
     upload_range_lists(h);
     return;
@@ -298,7 +288,6 @@ static void upload_lists(lpa_handle *h) {
   h->n_groups = out.n_groups;
   h->n_cblock = out.n_cblock;
   h->n_cwarp = out.n_cwarp;
-  ensure_hub_spill(h);
   h->plan_version++;
   // the resident blocks (the warps take decode groups from a work queue),
   // fewer when there are fewer groups than warps
@@ -380,24 +369,88 @@ static void upload_range_lists(lpa_handle *h) {
     h->n_cblock += r.n_cblock;
     h->n_cwarp += r.n_cwarp;
   }
-  ensure_hub_spill(h);
   h->plan_version++;
 }
 
-static void ensure_two_pass_scratch(lpa_handle *h) {
-  if (h->d_scratch) return;
-  std::vector<uint64_t> &off = h->h_arc_off;
-  off.assign(h->n + 1, 0);
-  for (uint64_t p = 0; p < h->n; p++) off[p + 1] = off[p] + h->h_deg[p];
-  h->d_arc_off = dalloc<uint64_t>(h, h->n + 1, "arc offsets");
-  h2d(h, h->d_arc_off, off.data(), h->n + 1, "upload arc offsets");
-  // + 4: a 16-byte-aligned bulk copy may read up to 12 bytes past the last label
-  // (streamed: one range's labels at a time, after up to 3 words of alignment)
-  h->d_scratch = dalloc<uint32_t>(h, h->streamed ? h->scratch_words : off[h->n_c] + 4, "two-pass scratch");
-  // where every compressed position's segments start, for the pre-pass
+// A vertex that only a block or the two-pass kernels can take (heavy bucket)
+// in the compressed region.
+static bool is_hub(const SegInfo &s) { return s.region == 0 && s.bucket == kHeavy; }
+
+template <class T>
+static void dfree(lpa_handle *h, T *&p) {
+  if (!p) return;
+  h->allocations.erase(std::find(h->allocations.begin(), h->allocations.end(), (void *)p));
+  cudaFree(p);
+  p = nullptr;
+}
+
+// The two-pass kernels' scratch and position index, for the hubs alone (a
+// plan whose block-variant hubs run through them) or for every compressed
+// position.  The hubs' labels have an allocation of their own, so that a
+// handle that goes from one to the other holds no more than the whole: index
+// arc_off[p] of d_scratch reaches into either.
+static void ensure_two_pass_scratch(lpa_handle *h, bool full) {
+  if (h->scratch_scope >= (full ? 2 : 1)) return;
+  if (h->streamed) full = true;  // one range's labels at a time, after up to 3 words of alignment
   const uint64_t nc = std::max<uint64_t>(1, h->n_c);
-  h->d_pidx = dalloc<uint4>(h, nc, "position index");
-  h->d_cursor = dalloc<uint32_t>(h, nc, "pre-pass cursors");
+  const bool first = h->scratch_scope == 0;
+  std::vector<uint64_t> &off = h->h_arc_off;  // streamed: in position order, else the hubs' labels first
+  if (first) {
+    std::vector<uint8_t> hub(h->n_c, 0);
+    if (!h->streamed)
+      for (const SegInfo &s : h->segs)
+        if (is_hub(s)) std::fill(hub.begin() + s.begin, hub.begin() + s.end, uint8_t(1));
+    off.assign(h->n_c + 1, 0);
+    uint64_t at = 0;
+    for (int pass = 0; pass < 2; pass++) {
+      for (uint64_t p = 0; p < h->n_c; p++) {
+        if (bool(hub[p]) != (pass == 0)) continue;
+        off[p] = at;
+        at += h->h_deg[p];
+      }
+      if (pass == 0) h->hub_arcs = at;
+    }
+    off[h->n_c] = at;
+  }
+  uint64_t *d_arc_off = h->d_arc_off;
+  uint32_t *d_scratch = h->d_scratch, *d_rest = nullptr;
+  uint4 *d_pidx = h->d_pidx;
+  uint32_t *d_cursor = h->d_cursor;
+  try {
+    if (first) {
+      // + 4: a 16-byte-aligned bulk copy may read up to 12 bytes past the last label
+      d_scratch = dalloc<uint32_t>(h, h->streamed ? h->scratch_words : h->hub_arcs + 4, "two-pass scratch");
+      d_arc_off = dalloc<uint64_t>(h, h->n_c + 1, "arc offsets");
+      d_pidx = dalloc<uint4>(h, nc, "position index");
+      d_cursor = dalloc<uint32_t>(h, nc, "pre-pass cursors");
+    }
+    if (full && !h->streamed) d_rest = dalloc<uint32_t>(h, off[h->n_c] - h->hub_arcs + 4, "two-pass scratch");
+  } catch (const Fail &) {
+    if (first) {
+      dfree(h, d_scratch);
+      dfree(h, d_arc_off);
+      dfree(h, d_pidx);
+      dfree(h, d_cursor);
+    }
+    throw;
+  }
+  std::vector<uint64_t> dev = off;
+  if (d_rest) {
+    // both allocations are 256-byte aligned, so indices keep their 16-byte alignment
+    const uint64_t shift = uint64_t((reinterpret_cast<int64_t>(d_rest) - reinterpret_cast<int64_t>(d_scratch)) / 4);
+    for (uint64_t p = 0; p < h->n_c; p++)
+      if (off[p] >= h->hub_arcs) dev[p] = off[p] - h->hub_arcs + shift;
+  }
+  h->d_arc_off = d_arc_off;
+  h->d_scratch = d_scratch;
+  if (d_rest) h->d_scratch_rest = d_rest;
+  h->d_pidx = d_pidx;
+  h->d_cursor = d_cursor;
+  h->scratch_scope = full ? 2 : 1;
+  h2d(h, h->d_arc_off, dev.data(), h->n_c + 1, "upload arc offsets");
+  check(h, cudaStreamSynchronize(h->stream), "arc offsets");
+  if (!first) return;
+  // where every compressed position's segments start, for the pre-pass
   check(h, cudaMemsetAsync(h->d_cursor, 0, nc * sizeof(uint32_t), h->stream), "clear cursors");
   if (h->streamed) {
     for (const StreamRange &r : h->ranges) {
@@ -416,19 +469,43 @@ static void ensure_two_pass_scratch(lpa_handle *h) {
   }
   lpa_status st = take_device_error(h);
   if (st != LPA_OK) throw Fail{st, "position index: " + h->last_error};
-  check(h, cudaStreamSynchronize(h->stream), "arc offsets");
+}
+
+// What the kernels run for the plan h->variant: the plan, except that the hubs
+// on the block variant run through the two-pass kernels, whose pre-pass
+// spreads a hub's segments over the whole GPU.  One block decoding a hub alone
+// set the length of the iteration: R-MAT scale 18 (largest degree 25,057) took
+// 0.82 to 1.86 ms in k_iterate, 7 ms of work on one of 296 blocks.  Without
+// memory for the hubs' labels k_iterate's blocks decode them.
+static void apply_run_variants(lpa_handle *h) {
+  bool two = false, hubs = false;
+  for (size_t s = 0; s < h->segs.size(); s++) {
+    two |= h->variant[s] == LPA_VARIANT_TWO_PASS;
+    hubs |= h->variant[s] == LPA_VARIANT_BLOCK && is_hub(h->segs[s]);
+  }
+  if (two) ensure_two_pass_scratch(h, true);
+  if (hubs && h->hubs_two_pass) {
+    try {
+      ensure_two_pass_scratch(h, false);
+    } catch (const Fail &f) {
+      if (f.st != LPA_ERR_OOM) throw;
+      h->hubs_two_pass = false;
+    }
+  }
+  h->run_variant = h->variant;
+  if (hubs && h->hubs_two_pass)
+    for (size_t s = 0; s < h->segs.size(); s++)
+      if (h->variant[s] == LPA_VARIANT_BLOCK && is_hub(h->segs[s])) h->run_variant[s] = LPA_VARIANT_TWO_PASS;
 }
 
 static void apply_dispatch(lpa_handle *h, int dispatch, int force) {
   h->variant.resize(h->segs.size());
-  bool any_two = false;
   for (size_t s = 0; s < h->segs.size(); s++) {
     int v = h->fixed[s];
     if (dispatch == LPA_DISPATCH_FORCE && variant_capable(force, h->segs[s], h->opts.cms_threshold)) v = force;
     h->variant[s] = uint8_t(v);
-    any_two |= v == LPA_VARIANT_TWO_PASS;
   }
-  if (any_two) ensure_two_pass_scratch(h);
+  apply_run_variants(h);
   upload_lists(h);
 }
 
@@ -573,7 +650,6 @@ static void build_plan(lpa_handle *h) {
     const uint32_t d = h->h_deg[p];
     const bool cms = h->opts.cms_threshold != 0 && d >= h->opts.cms_threshold;
     if (!cms && d > kBlockMaxSmemDeg) big = std::max<uint64_t>(big, d);
-    if (cms) h->max_sketch_deg = std::max(h->max_sketch_deg, d);
   }
   if (big) {
     h->gtab_slots = next_pow2_host(2 * big);
@@ -634,8 +710,6 @@ static IterArgs iter_args(lpa_handle *h, unsigned long long *changed, uint32_t *
   a.gbase = h->d_gbase;
   a.n_gbase = h->d_gbase ? h->n_graphs : 0u;
   a.wend = (h->nwords + 4) & ~uint64_t(3);
-  a.hub_spill = h->d_hub_spill;
-  a.hub_spill_words = h->hub_spill_words;
   return a;
 }
 
@@ -1156,9 +1230,8 @@ lpa_status lpa_decode_csr(lpa_handle *h, uint64_t *row_out, uint32_t *clm_out) {
   if (!h || !row_out || (!clm_out && h->m)) return LPA_ERR_INVALID_ARG;
   try {
     check(h, cudaSetDevice(h->device), "cudaSetDevice");
-    ensure_two_pass_scratch(h);
-    std::vector<uint64_t> off(h->n + 1, 0);
-    for (uint64_t p = 0; p < h->n; p++) off[p + 1] = off[p] + h->h_deg[p];
+    ensure_two_pass_scratch(h, true);
+    const std::vector<uint64_t> &off = h->h_arc_off;
     std::vector<uint32_t> ids(off[h->n_c]);
     DecodeArgs a{};
     a.g = dev_graph(h);
@@ -1188,7 +1261,9 @@ lpa_status lpa_decode_csr(lpa_handle *h, uint64_t *row_out, uint32_t *clm_out) {
       a.out = h->d_scratch;
       lpa_status st = decode(0, h->n_c);
       if (st != LPA_OK) return st;
-      check(h, cudaMemcpy(ids.data(), h->d_scratch, ids.size() * 4, cudaMemcpyDeviceToHost), "read decode");
+      check(h, cudaMemcpy(ids.data(), h->d_scratch, h->hub_arcs * 4, cudaMemcpyDeviceToHost), "read decode");
+      check(h, cudaMemcpy(ids.data() + h->hub_arcs, h->d_scratch_rest, (ids.size() - h->hub_arcs) * 4,
+                          cudaMemcpyDeviceToHost), "read decode");
     }
     std::vector<uint32_t> verts(h->n);
     check(h, cudaMemcpy(verts.data(), h->d_vertices, h->n * 4, cudaMemcpyDeviceToHost), "read vertices");
@@ -1424,9 +1499,7 @@ void lpa_rt_enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
   enqueue_iteration(h, changed, work);
 }
 void lpa_rt_apply_variants(lpa_handle *h) {
-  bool any_two = false;
-  for (auto v : h->variant) any_two |= v == LPA_VARIANT_TWO_PASS;
-  if (any_two) ensure_two_pass_scratch(h);
+  apply_run_variants(h);
   upload_lists(h);
 }
 lpa_status lpa_rt_take_error(lpa_handle *h) { return take_device_error(h); }

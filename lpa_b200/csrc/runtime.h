@@ -95,6 +95,7 @@ struct lpa_handle {
   std::vector<uint32_t> h_deg;
   std::vector<lpa_rt::SegInfo> segs;
   std::vector<uint8_t> variant;  // per segment
+  std::vector<uint8_t> run_variant;          // what the kernels run for it (apply_run_variants)
   std::vector<uint8_t> fixed;    // per segment, the heuristic's choice
   lpa_dev::Seg *d_segs = nullptr;
   lpa_dev::SegDev *d_segdev = nullptr;       // the segments as the device list builder reads them
@@ -131,9 +132,10 @@ struct lpa_handle {
   uint64_t *d_arc_off = nullptr;
   uint32_t *d_scratch = nullptr;
   uint32_t *d_gtab = nullptr;
-  uint32_t *d_hub_spill = nullptr;  // per block of k_iterate: a sketch hub's labels (second pass)
-  uint32_t hub_spill_words = 0;
-  uint32_t max_sketch_deg = 0;      // largest degree at or above the sketch threshold
+  uint32_t *d_scratch_rest = nullptr;  // the labels of the positions that are no hubs
+  int scratch_scope = 0;               // scratch holds nothing, the hubs' labels, every compressed position's
+  uint64_t hub_arcs = 0;               // labels in d_scratch (resident handles)
+  bool hubs_two_pass = true;           // block-variant hubs run through the two-pass kernels
   uint32_t gtab_slots = 0;
   int gtab_blocks = 0;
   long long *d_seg_cycles = nullptr;
