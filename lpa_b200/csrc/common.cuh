@@ -450,7 +450,7 @@ __device__ __forceinline__ uint64_t warp_max_u64(uint64_t v) {
 // Open-addressing exact counter in shared (or global) memory.  Keys are
 // stored as label + 1 so that 0 marks an empty slot.  cap is a power of two
 // larger than the number of distinct labels inserted.
-__device__ __forceinline__ void table_add(uint32_t *keys, uint32_t *cnts, uint32_t cap, uint32_t label,
+__device__ __forceinline__ bool table_add(uint32_t *keys, uint32_t *cnts, uint32_t cap, uint32_t label,
                                           uint32_t c) {
   const uint32_t key = label + 1u;
   uint32_t h = slot_hash(label) & (cap - 1);
@@ -458,17 +458,18 @@ __device__ __forceinline__ void table_add(uint32_t *keys, uint32_t *cnts, uint32
     uint32_t k = keys[h];
     if (k == key) {
       atomicAdd(&cnts[h], c);
-      return;
+      return true;
     }
     if (k == 0) {
       uint32_t old = atomicCAS(&keys[h], 0u, key);
       if (old == 0u || old == key) {
         atomicAdd(&cnts[h], c);
-        return;
+        return true;
       }
     }
     h = (h + 1) & (cap - 1);
   }
+  return false;  // full
 }
 
 // Exact counter in shared memory without clearing: a slot is one 64-bit word

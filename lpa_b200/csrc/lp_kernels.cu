@@ -1657,6 +1657,48 @@ __device__ __forceinline__ void sketch_count(uint32_t *cms, const uint32_t *__re
   });
 }
 
+// One share of an exact vertex's labels (BlockItem, kCountHash) by the whole
+// block: best is this thread's best of them.  keys and counts: kCountBlockSlots
+// each, zero before and after.  A share whose labels overfill the table is
+// counted again in 4, 16, ... parts of itself, told apart by further bits of
+// the hash (a bijection of the label: 20 bits leave at most 4096 labels).
+__device__ __noinline__ uint64_t count_share(uint32_t *keys, const uint32_t *src, uint32_t d, uint32_t lg,
+                                             uint32_t share) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t *cnts = keys + kCountBlockSlots;
+  uint64_t best = 0;
+  for (uint32_t more = 0;; more += 2) {
+    best = 0;
+    bool full = false;
+    for (uint32_t part = 0; part < 1u << more && !full; part++) {
+      const uint32_t want = share << more | part, sh = 32u - lg - more;
+      const auto ins = [&](uint32_t lab, uint32_t c) { full |= !table_add(keys, cnts, kCountBlockSlots, lab, c); };
+      WarpRun run;
+      warp_stream<true, 4>(src, d, warp, kWarps, [&](bool ok, uint32_t lab) {
+        ok = ok && slot_hash(lab) >> sh == want;
+        if (run.extend(ok, lab)) return;
+        if (run.cnt && lane == 0) ins(run.lab, run.cnt);
+        run.restart(ok, lab);
+        const uint32_t c = warp_merge(ok, lab);
+        if (c) ins(lab, c);
+      });
+      if (run.cnt && lane == 0) ins(run.lab, run.cnt);
+      full = __syncthreads_or(full) != 0;
+      for (uint32_t k = threadIdx.x; k < kCountBlockSlots; k += kThreads) {
+        const uint32_t key = keys[k];
+        if (key) {
+          const uint64_t cand = pack_best(cnts[k], key - 1u);
+          best = cand > best ? cand : best;
+          keys[k] = 0u;
+          cnts[k] = 0u;
+        }
+      }
+      __syncthreads();
+    }
+    if (!full) return best;
+  }
+}
+
 // Block-wide maximum of v, returned to every thread.
 __device__ __forceinline__ uint64_t block_max_u64(uint64_t v, uint64_t *red) {
   v = warp_max_u64(v);
@@ -1737,7 +1779,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_count_two_pass(IterArgs a) {
       old = ld_label(c, it.node);  // needed at the end only
     }
     uint64_t best = 0;
-    if (it.kind == kCountSketch) {
+    if ((it.kind & 15u) == kCountSketch) {
       uint32_t *cms = reinterpret_cast<uint32_t *>(cslots);
       for (uint32_t k = t; k < kCmsDepth * kCmsWidth; k += kThreads) cms[k] = 0u;
       const uint32_t lb = label_base(a, it.node);
@@ -1746,6 +1788,11 @@ __global__ void __launch_bounds__(kThreads, 5) k_count_two_pass(IterArgs a) {
       best = block_max_u64(best, red);
       // leave no counter behind that a table could read as one of its slots
       for (uint32_t k = t; k < kCmsDepth * kCmsWidth; k += kThreads) cms[k] = 0u;
+    } else if ((it.kind & 15u) == kCountHash) {
+      uint32_t *keys = reinterpret_cast<uint32_t *>(cslots);
+      for (uint32_t k = t; k < 2 * kCountBlockSlots; k += kThreads) keys[k] = 0u;
+      __syncthreads();
+      best = block_max_u64(count_share(keys, src, d, (it.kind >> 4) & 15u, it.kind >> 8), red);
     } else {
       // blocks small enough that every warp takes one: the critical path of
       // a vertex of 512..1024 labels is one block of 64 or 128, not 256
@@ -1756,10 +1803,24 @@ __global__ void __launch_bounds__(kThreads, 5) k_count_two_pass(IterArgs a) {
       best = block_max_u64(best, red);
     }
     if (t == 0) {
-      const uint32_t nl = d ? best_label(best) : old;
-      c.lab_out[it.node] = nl;
-      changed += (nl != old);
-      if (a.seg_changed && nl != old) atomicAdd(a.seg_changed + it.seg, 1u);
+      bool last = true;
+      if ((it.kind & 15u) == kCountHash) {  // the last share to finish has the vertex's best
+        HashSlot &hs = a.hash[it.slot];
+        atomicMax(&hs.best, (unsigned long long)best);
+        __threadfence();
+        last = atomicAdd(&hs.done, 1u) + 1u == 1u << ((it.kind >> 4) & 15u);
+        if (last) {
+          __threadfence();
+          best = atomicExch(&hs.best, 0ull);
+          hs.done = 0u;
+        }
+      }
+      if (last) {
+        const uint32_t nl = d ? best_label(best) : old;
+        c.lab_out[it.node] = nl;
+        changed += (nl != old);
+        if (a.seg_changed && nl != old) atomicAdd(a.seg_changed + it.seg, 1u);
+      }
       if (a.seg_cycles)
         atomicAdd(reinterpret_cast<unsigned long long *>(a.seg_cycles + it.seg),
                   (unsigned long long)((clock64() - t0) * kWarps * a.cw_count));

@@ -81,6 +81,7 @@ enum CountKind : uint32_t {
   kCountWarp = 1,    // np <= 4 positions of degree <= kCountWarpMax: warp per vertex, 512-slot table
   kCountBlock = 2,   // one position, degree <= kCountBlockMax: block per vertex, 4096-slot table
   kCountSketch = 3,  // one position at or above the sketch threshold: block per vertex
+  kCountHash = 4,    // one position, exact, degree <= kCountHashMax: a block per share of the labels' hashes
 };
 struct CountItem {
   uint32_t p0, np, seg, kind;
@@ -89,7 +90,22 @@ struct CountItem {
 struct BlockItem {
   uint64_t ao;              // scratch index of the position's labels (arc offset)
   uint32_t p, d, node;      // position, degree, vertex id
-  uint32_t seg, kind, pad;  // plan segment (cycles), kCountBlock or kCountSketch
+  uint32_t seg, kind, slot; // plan segment (cycles), kind (below), kCountHash: the vertex's HashSlot
+};
+// kind: CountKind in the low 4 bits; kCountHash: log2 of the shares in the
+// next 4, the item's share in the rest.
+// An exact vertex above the block table is counted share by share: the blocks
+// of its items each stream all its labels (from L2) and count those whose hash
+// falls to them, at most about kCountHashLoad different ones, in 4096 slots of
+// shared memory; the last to finish holds the vertex's best.  One block with a
+// table in global memory took 92 us (526 us with every label different) for
+// the degree-25,057 hub of R-MAT scale 18.
+constexpr uint32_t kCountHashLoad = 2048;
+constexpr uint32_t kCountHashMaxLog = 12;
+constexpr uint64_t kCountHashMax = uint64_t(kCountHashLoad) << kCountHashMaxLog;
+struct HashSlot {
+  unsigned long long best;  // pack_best over the finished shares
+  uint32_t done, pad;       // finished shares
 };
 constexpr uint32_t kCountWarpSlots = 512;
 constexpr uint32_t kCountWarpMax = kCountWarpSlots - 1;  // tables fill up to load 1 (triangular probing)
@@ -137,6 +153,7 @@ struct IterArgs {
   const uint4 *pidx;            // per compressed position: {ibase - offset, rbase - offset, nseg_i, nseg_r}
   const BlockItem *cblock;      // count-pass block items (largest first)
   uint32_t n_cblock;
+  HashSlot *hash;               // of the kCountHash vertices; zero between launches
   const CountItem *cwarp;
   uint32_t n_cwarp;
   uint32_t warp_claim;          // warp items a warp of the count pass claims at once

@@ -33,7 +33,7 @@ namespace lpa_dev {
 
 namespace {
 
-enum List : int { kLHeavy = 0, kLLight, kLPacked, kLGroups, kLBlock, kLWarp, kLists };
+enum List : int { kLHeavy = 0, kLLight, kLPacked, kLGroups, kLBlock, kLWarp, kLHash, kLists };
 
 struct PlanArgs {
   const SegDev *segs;
@@ -108,14 +108,13 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
   const bool block = (v == kVarBlock || tp) && !warp_capable(si, cms);
   bool counted = tp;  // the two-pass count pass takes the segment's positions
   if (tp) {
-    // exact above the count pass's block table (a hub is alone in its segment)
-    if (si.max_deg > kCountBlockMax && (cms == 0 || si.max_deg < cms)) counted = false;
+    // exact above the count pass's reach (a hub is alone in its segment)
+    if (si.max_deg > kCountHashMax && (cms == 0 || si.max_deg < cms)) counted = false;
     // the small CSR is counted by warp and group items only
     if (si.region == 1 && ((cms != 0 && si.max_deg >= cms) || si.max_deg > a.wmax)) counted = false;
   }
   const uint32_t stride = a.nseg + 1;
-  uint32_t c[kLists] = {0, 0, 0, 0, 0, 0};
-  uint32_t o[kLists] = {0, 0, 0, 0, 0, 0};
+  uint32_t c[kLists] = {}, o[kLists] = {};
   if (kEmit)
     for (int l = 0; l < kLists; l++) o[l] = a.off[l * stride + i];
   if (counted) {
@@ -123,7 +122,21 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
     while (p < si.end) {
       const uint32_t d = a.deg[p];
       const bool sk = cms != 0 && d >= cms;
-      if (sk || d > a.wmax) {
+      if (!sk && d > kCountBlockMax) {
+        uint32_t lg = 1;
+        while ((uint64_t(kCountHashLoad) << lg) < d) lg++;
+        if (kEmit) {
+          for (uint32_t k = 0; k < 1u << lg; k++) {
+            const uint32_t at = o[kLBlock] + c[kLBlock] + k;
+            a.cblock[at] = BlockItem{a.arc_off[p], p, d, a.vertices[p], s,
+                                     uint32_t(kCountHash) | lg << 4 | k << 8, o[kLHash] + c[kLHash]};
+            a.cblock_key[at] = d;
+          }
+        }
+        c[kLBlock] += 1u << lg;
+        c[kLHash]++;
+        p++;
+      } else if (sk || d > a.wmax) {
         if (kEmit) {
           const uint32_t at = o[kLBlock] + c[kLBlock];
           a.cblock[at] = BlockItem{a.arc_off[p], p, d, a.vertices[p], s,
@@ -341,7 +354,7 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   PB_TRY(reserve(reinterpret_cast<void **>(&gmark), gmark_cap, std::max<uint64_t>(1, in.n) * 4), "group marks");
   PB_TRY(reserve(reinterpret_cast<void **>(&win), win_cap, (nwin + 1) * 4), "window counts");
   PB_TRY(reserve(reinterpret_cast<void **>(&win_off), win_off_cap, (nwin + 1) * 4), "window offsets");
-  PB_TRY(reserve(reinterpret_cast<void **>(&tot), tot_cap, 8 * 4), "plan totals");
+  PB_TRY(reserve(reinterpret_cast<void **>(&tot), tot_cap, (kLists + 1) * 4), "plan totals");
   PB_TRY(cudaMemsetAsync(cnt, 0, size_t(kLists) * stride * 4, st), "clear counts");
   PB_TRY(cudaMemsetAsync(win, 0, (nwin + 1) * 4, st), "clear windows");
   PB_TRY(cudaMemsetAsync(gmark, 0, std::max<uint64_t>(1, in.n) * 4, st), "clear marks");
@@ -396,8 +409,8 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   PB_TRY(cub::DeviceScan::ExclusiveSum(temp, t, win, win_off, nwin + 1, st), "window scan");
   k_plan_totals<<<1, 32, 0, st>>>(off, stride, win_off, nwin, tot);
   PB_TRY(cudaGetLastError(), "totals launch");
-  uint32_t h_tot[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  PB_TRY(cudaMemcpyAsync(h_tot, tot, 8 * 4, cudaMemcpyDeviceToHost, st), "read totals");
+  uint32_t h_tot[kLists + 1] = {};
+  PB_TRY(cudaMemcpyAsync(h_tot, tot, (kLists + 1) * 4, cudaMemcpyDeviceToHost, st), "read totals");
   PB_TRY(cudaStreamSynchronize(st), "plan totals");
   out.n_heavy = h_tot[kLHeavy];
   out.n_light = h_tot[kLLight];
@@ -405,6 +418,7 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   out.n_groups = h_tot[kLGroups];
   out.n_cblock = h_tot[kLBlock];
   out.n_cwarp = h_tot[kLWarp] + h_tot[kLists];
+  out.n_hash = h_tot[kLHash];
 
   // outputs (the caller's buffers grow to fit) and sort staging
   PB_TRY(out.grow(out), "work lists");

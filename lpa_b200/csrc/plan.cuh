@@ -48,12 +48,13 @@ struct PlanInputs {
 // light items; cwarp = warp items followed by group items; cblock largest
 // first.
 struct PlanOutputs {
-  uint32_t n_heavy = 0, n_light = 0, n_packed = 0, n_groups = 0, n_cblock = 0, n_cwarp = 0;
+  uint32_t n_heavy = 0, n_light = 0, n_packed = 0, n_groups = 0, n_cblock = 0, n_cwarp = 0, n_hash = 0;
   WorkItem *items = nullptr;
   PackedChunk *packed = nullptr;
   DecodeGroup *groups = nullptr;
   BlockItem *cblock = nullptr;
   CountItem *cwarp = nullptr;
+  // grow() also makes room for n_hash HashSlots, all zero
   std::function<cudaError_t(PlanOutputs &)> grow;
 };
 

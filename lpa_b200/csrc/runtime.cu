@@ -223,6 +223,23 @@ static void build_segments(lpa_handle *h) {
 // few launches and one copy of the list sizes, not a host loop over n.
 static void upload_range_lists(lpa_handle *h);
 
+template <class T>
+static void dfree(lpa_handle *h, T *&p) {
+  if (!p) return;
+  h->allocations.erase(std::find(h->allocations.begin(), h->allocations.end(), (void *)p));
+  cudaFree(p);
+  p = nullptr;
+}
+
+static void grow_hash_slots(lpa_handle *h, size_t need) {
+  if (need <= h->hash_cap) return;
+  dfree(h, h->d_hash);
+  h->hash_cap = 0;
+  h->d_hash = dalloc<HashSlot>(h, need, "hash slots");
+  h->hash_cap = need;
+  check(h, cudaMemsetAsync(h->d_hash, 0, need * sizeof(HashSlot), h->stream), "clear hash slots");
+}
+
 static void upload_lists(lpa_handle *h) {
   h2d(h, h->d_seg_var, h->run_variant.data(), h->run_variant.size(), "upload variants");
   if (h->streamed) {
@@ -271,6 +288,7 @@ static void upload_lists(lpa_handle *h) {
     regrow(h->d_citems, h->citems_cap, o.n_cwarp, "count items");
     regrow(h->d_cblock, h->cblock_cap, o.n_cblock, "count block items");
     regrow(h->d_packed, h->packed_cap, o.n_packed, "packed chunks");
+    grow_hash_slots(h, o.n_hash);
     o.items = h->d_items;
     o.groups = h->d_groups;
     o.cwarp = h->d_citems;
@@ -343,6 +361,7 @@ static void upload_range_lists(lpa_handle *h) {
       regrow(r.cwarp, r.cwarp_cap, o.n_cwarp, "range count items");
       regrow(r.cblock, r.cblock_cap, o.n_cblock, "range count block items");
       regrow(r.packed, r.packed_cap, o.n_packed, "range packed chunks");
+      grow_hash_slots(h, o.n_hash);  // ranges run one after another and leave the slots zero
       o.items = r.items;
       o.groups = r.groups;
       o.cwarp = r.cwarp;
@@ -375,14 +394,6 @@ static void upload_range_lists(lpa_handle *h) {
 // A vertex that only a block or the two-pass kernels can take (heavy bucket)
 // in the compressed region.
 static bool is_hub(const SegInfo &s) { return s.region == 0 && s.bucket == kHeavy; }
-
-template <class T>
-static void dfree(lpa_handle *h, T *&p) {
-  if (!p) return;
-  h->allocations.erase(std::find(h->allocations.begin(), h->allocations.end(), (void *)p));
-  cudaFree(p);
-  p = nullptr;
-}
 
 // The two-pass kernels' scratch and position index, for the hubs alone (a
 // plan whose block-variant hubs run through them) or for every compressed
@@ -686,6 +697,7 @@ static IterArgs iter_args(lpa_handle *h, unsigned long long *changed, uint32_t *
   a.group_base = a.group_claim == 1 ? uint32_t(h->grid_decode) * kWarps : 0;
   a.cblock = h->d_cblock;
   a.n_cblock = h->n_cblock;
+  a.hash = h->d_hash;
   a.cwarp = h->d_citems;
   a.n_cwarp = h->n_cwarp;
   a.warp_claim = h->tune.warp_claim;

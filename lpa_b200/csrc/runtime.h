@@ -116,6 +116,8 @@ struct lpa_handle {
   uint32_t cw_packed = 1;
   size_t cblock_cap = 0;
   uint32_t n_cblock = 0, n_cwarp = 0;
+  lpa_dev::HashSlot *d_hash = nullptr;       // the count pass's hubs counted in shares
+  size_t hash_cap = 0;
   size_t citems_cap = 0;
   int grid_count = 0;                        // count-pass kernel
   uint32_t cw_iterate = 1, cw_decode = 1, cw_count = 1;  // seg_cycles weights (64 / resident warps per SM)
