@@ -392,8 +392,13 @@ lpa_status lpa_batch_create(const lpa_graph_desc *graphs, size_t num_graphs, con
                                cudaMemcpyHostToDevice, b->stream));
       if (g.num_small_arcs)
         bcheck(cudaMemcpyAsync(d_snbr + on, g.small_graph, g.num_small_arcs * 4, cudaMemcpyHostToDevice, b->stream));
+      // the hub list and its length sit in the label buffers until the labels do
+      bcheck(cudaMemsetAsync(bg.labs1, 0, 4, b->stream));
       k_degree_count<<<std::max<uint64_t>(1, std::min<uint64_t>((g.num_vertices + 127) / 128, 4096)), 128, 0,
-                       b->stream>>>(bg.g, d_deg + ov, nullptr, b->d_err, 0, g.num_vertices);
+                       b->stream>>>(bg.g, d_deg + ov, nullptr, b->d_err, 0, g.num_vertices, bg.labs0, bg.labs1);
+      if (g.num_compressed)
+        k_degree_hubs<<<int(std::min<uint64_t>(g.num_compressed, uint64_t(b->num_sms))), kThreads, 0, b->stream>>>(
+            bg.g, d_deg + ov, nullptr, b->d_err, bg.labs0, bg.labs1);
       ow += g.num_words + 4;
       oo += g.num_compressed + 1;
       ov += g.num_vertices;

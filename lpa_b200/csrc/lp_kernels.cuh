@@ -284,9 +284,14 @@ __global__ void k_decode_positions(DecodeArgs a);
 // Positions [p_lo, p_hi) (compressed ones only).
 __global__ void k_pos_index(DevGraph g, uint4 *pidx, uint32_t *err, uint64_t p_lo, uint64_t p_hi);
 
-// Degrees (and interval items) of positions [p_lo, p_hi).
+// Degrees (and interval items) of positions [p_lo, p_hi), a thread each;
+// positions of more than kHubBits go to hubs[0..*n_hubs) (room for every
+// compressed position of the range) and are left to k_degree_hubs.
+constexpr uint64_t kHubBits = 4096;
 __global__ void k_degree_count(DevGraph g, uint32_t *deg_out, uint32_t *itv_out, uint32_t *err, uint64_t p_lo,
-                               uint64_t p_hi);
+                               uint64_t p_hi, uint32_t *hubs, uint32_t *n_hubs);
+__global__ void k_degree_hubs(DevGraph g, uint32_t *deg_out, uint32_t *itv_out, uint32_t *err, const uint32_t *hubs,
+                              const uint32_t *n_hubs);
 __global__ void k_init_labels(uint32_t *a, uint32_t *b, uint64_t n);
 
 }  // namespace lpa_dev

@@ -569,12 +569,22 @@ static void build_plan(lpa_handle *h) {
   h->d_deg = dalloc<uint32_t>(h, h->n, "degrees");
   uint32_t *d_itv = nullptr;
   check(h, cudaMalloc(&d_itv, std::max<uint64_t>(1, h->n) * sizeof(uint32_t)), "interval counts");
+  // the positions left to k_degree_hubs, after their number
+  uint32_t *d_hubs = nullptr;
+  cudaError_t he = cudaMalloc(&d_hubs, (h->n_c + 1) * sizeof(uint32_t));
+  if (he != cudaSuccess) cudaFree(d_itv);
+  check(h, he, "hub list");
   const int threads = 128;
   auto degree_pass = [&](const DevGraph &g, uint64_t p0, uint64_t p1) {
     if (p1 <= p0) return;
     const int blocks = int(std::min<uint64_t>((p1 - p0 + threads - 1) / threads, uint64_t(h->num_sms) * 32));
-    k_degree_count<<<std::max(blocks, 1), threads, 0, h->stream>>>(g, h->d_deg, d_itv, h->d_err, p0, p1);
+    check(h, cudaMemsetAsync(d_hubs, 0, sizeof(uint32_t), h->stream), "clear hub list");
+    k_degree_count<<<std::max(blocks, 1), threads, 0, h->stream>>>(g, h->d_deg, d_itv, h->d_err, p0, p1, d_hubs + 1,
+                                                                   d_hubs);
     check(h, cudaGetLastError(), "degree kernel launch");
+    if (p0 >= h->n_c) return;  // the small CSR has none
+    k_degree_hubs<<<h->num_sms * 8, kThreads, 0, h->stream>>>(g, h->d_deg, d_itv, h->d_err, d_hubs + 1, d_hubs);
+    check(h, cudaGetLastError(), "hub degree kernel launch");
   };
   if (h->streamed) {
     // compressed positions in chunks whose stream fits one buffer, then the small CSR
@@ -616,6 +626,7 @@ static void build_plan(lpa_handle *h) {
   std::vector<uint32_t> itv(h->n);
   check(h, cudaMemcpy(itv.data(), d_itv, h->n * sizeof(uint32_t), cudaMemcpyDeviceToHost), "read interval counts");
   cudaFree(d_itv);
+  cudaFree(d_hubs);
   h->m = 0;
   h->max_deg = 0;
   for (uint64_t p = 0; p < h->n; p++) {
