@@ -1724,7 +1724,9 @@ __device__ __forceinline__ uint64_t block_max_u64(uint64_t v, uint64_t *red) {
 // groups.  The same shared memory serves the warp tables, the block table
 // (block epochs, disjoint from the warps') and the sketch (cleared before and
 // after use).  Every position's pre-pass cursor is reset here.
-template <bool kBulk>
+// kHash: the plan has kCountHash items (the call in the item loop costs the
+// others registers: 20 us of 430 at R-MAT scale 22).
+template <bool kBulk, bool kHash>
 __global__ void __launch_bounds__(kThreads, 5) k_count_two_pass(IterArgs a) {
   extern __shared__ __align__(128) unsigned long long cslots[];
   __shared__ uint64_t red[kWarps];
@@ -1788,7 +1790,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_count_two_pass(IterArgs a) {
       best = block_max_u64(best, red);
       // leave no counter behind that a table could read as one of its slots
       for (uint32_t k = t; k < kCmsDepth * kCmsWidth; k += kThreads) cms[k] = 0u;
-    } else if ((it.kind & 15u) == kCountHash) {
+    } else if (kHash && (it.kind & 15u) == kCountHash) {
       uint32_t *keys = reinterpret_cast<uint32_t *>(cslots);
       for (uint32_t k = t; k < 2 * kCountBlockSlots; k += kThreads) keys[k] = 0u;
       __syncthreads();
@@ -1804,7 +1806,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_count_two_pass(IterArgs a) {
     }
     if (t == 0) {
       bool last = true;
-      if ((it.kind & 15u) == kCountHash) {  // the last share to finish has the vertex's best
+      if (kHash && (it.kind & 15u) == kCountHash) {  // the last share to finish has the vertex's best
         HashSlot &hs = a.hash[it.slot];
         atomicMax(&hs.best, (unsigned long long)best);
         __threadfence();
@@ -1993,8 +1995,10 @@ __global__ void __launch_bounds__(kThreads, 5) k_count_two_pass(IterArgs a) {
   flush_changed(c.changed, changed);
 }
 
-template __global__ void k_count_two_pass<false>(IterArgs a);
-template __global__ void k_count_two_pass<true>(IterArgs a);
+template __global__ void k_count_two_pass<false, false>(IterArgs a);
+template __global__ void k_count_two_pass<true, false>(IterArgs a);
+template __global__ void k_count_two_pass<false, true>(IterArgs a);
+template __global__ void k_count_two_pass<true, true>(IterArgs a);
 
 template <int G>
 static void launch_decode_form(uint32_t stage, int grid, cudaStream_t s, const IterArgs &a) {
@@ -2020,9 +2024,11 @@ void launch_decode_two_pass(uint32_t gather_cache, uint32_t stage, int grid, cud
   else launch_decode_form<0>(stage, grid, s, a);
 }
 
-void launch_count_two_pass(bool bulk, int grid, cudaStream_t s, const IterArgs &a) {
-  if (bulk) k_count_two_pass<true><<<grid, kThreads, kCountSmemBytes, s>>>(a);
-  else k_count_two_pass<false><<<grid, kThreads, kCountSmemBytes, s>>>(a);
+void launch_count_two_pass(bool bulk, bool hash, int grid, cudaStream_t s, const IterArgs &a) {
+  if (bulk && hash) k_count_two_pass<true, true><<<grid, kThreads, kCountSmemBytes, s>>>(a);
+  else if (bulk) k_count_two_pass<true, false><<<grid, kThreads, kCountSmemBytes, s>>>(a);
+  else if (hash) k_count_two_pass<false, true><<<grid, kThreads, kCountSmemBytes, s>>>(a);
+  else k_count_two_pass<false, false><<<grid, kThreads, kCountSmemBytes, s>>>(a);
 }
 
 cudaError_t occupancy_decode_two_pass(int *blocks) {
@@ -2037,12 +2043,15 @@ cudaError_t occupancy_decode_two_pass(int *blocks) {
 }
 
 cudaError_t occupancy_count_two_pass(int *blocks) {
-  int b0 = 1, b1 = 1;
-  cudaError_t e =
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, k_count_two_pass<false>, kThreads, kCountSmemBytes);
+  int b[4] = {1, 1, 1, 1};
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[0], k_count_two_pass<false, false>, kThreads, kCountSmemBytes);
   if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_count_two_pass<true>, kThreads, kCountSmemBytes);
-  *blocks = b0 < b1 ? b0 : b1;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[1], k_count_two_pass<true, false>, kThreads, kCountSmemBytes);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[2], k_count_two_pass<false, true>, kThreads, kCountSmemBytes);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[3], k_count_two_pass<true, true>, kThreads, kCountSmemBytes);
+  *blocks = min(min(b[0], b[1]), min(b[2], b[3]));
   return e;
 }
 

@@ -252,16 +252,17 @@ __global__ void k_decode_two_pass(IterArgs a);
 // V2 for tiny vertices: a lane per vertex.
 __global__ void k_packed(IterArgs a);
 // Two-pass variant, pass 2: counts the labels the pre-pass wrote.
-// kBulk: group items staged by bulk copies (lpa_tune.bulk_stage)
-template <bool kBulk>
+// kBulk: group items staged by bulk copies (lpa_tune.bulk_stage); kHash: the
+// plan has kCountHash items
+template <bool kBulk, bool kHash>
 __global__ void k_count_two_pass(IterArgs a);
 
 // The template forms of the two-pass kernels are launched and sized only in
 // the file that defines them (lp_kernels.cu):
 // k_decode_two_pass<gather_cache, stage_stream, pack> on `grid` blocks of kThreads;
 void launch_decode_two_pass(uint32_t gather_cache, uint32_t stage, int grid, cudaStream_t s, const IterArgs &a);
-// k_count_two_pass<bulk> on `grid` blocks of kThreads with kCountSmemBytes;
-void launch_count_two_pass(bool bulk, int grid, cudaStream_t s, const IterArgs &a);
+// k_count_two_pass<bulk, hash> on `grid` blocks of kThreads with kCountSmemBytes;
+void launch_count_two_pass(bool bulk, bool hash, int grid, cudaStream_t s, const IterArgs &a);
 // allows the stage_stream 2 forms their dynamic shared memory (once per device)
 cudaError_t prepare_decode_two_pass();
 // the fewest resident blocks per SM over each kernel's forms.

@@ -306,6 +306,7 @@ static void upload_lists(lpa_handle *h) {
   h->n_groups = out.n_groups;
   h->n_cblock = out.n_cblock;
   h->n_cwarp = out.n_cwarp;
+  h->n_hash = out.n_hash;
   h->plan_version++;
   // the resident blocks (the warps take decode groups from a work queue),
   // fewer when there are fewer groups than warps
@@ -326,7 +327,7 @@ static void upload_range_lists(lpa_handle *h) {
     cap = need + need / 4 + 16;
     ptr = dalloc<std::remove_reference_t<decltype(*ptr)>>(h, cap, what);
   };
-  h->n_heavy = h->n_light = h->n_packed = h->n_groups = h->n_cblock = h->n_cwarp = 0;
+  h->n_heavy = h->n_light = h->n_packed = h->n_groups = h->n_cblock = h->n_cwarp = h->n_hash = 0;
   for (size_t k = 0; k < h->ranges.size(); k++) {
     StreamRange &r = h->ranges[k];
     PlanInputs in{};
@@ -387,6 +388,7 @@ static void upload_range_lists(lpa_handle *h) {
     h->n_groups += r.n_groups;
     h->n_cblock += r.n_cblock;
     h->n_cwarp += r.n_cwarp;
+    h->n_hash += out.n_hash;
   }
   h->plan_version++;
 }
@@ -763,7 +765,7 @@ static void enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
     mark(0);
   }
   if (h->n_cblock + h->n_cwarp) {
-    launch_count_two_pass(h->tune.bulk_stage != 0, h->grid_count, h->stream, a);
+    launch_count_two_pass(h->tune.bulk_stage != 0, h->n_hash != 0, h->grid_count, h->stream, a);
     h->launches++;
     mark(1);
   }
@@ -841,7 +843,7 @@ static void enqueue_streamed_iteration(lpa_handle *h, unsigned long long *change
       h->launches++;
     }
     if (r.n_cblock + r.n_cwarp) {
-      launch_count_two_pass(h->tune.bulk_stage != 0, h->grid_count, h->stream, a);
+      launch_count_two_pass(h->tune.bulk_stage != 0, h->n_hash != 0, h->grid_count, h->stream, a);
       h->launches++;
     }
     if (r.n_packed) {

@@ -117,6 +117,7 @@ struct lpa_handle {
   size_t cblock_cap = 0;
   uint32_t n_cblock = 0, n_cwarp = 0;
   lpa_dev::HashSlot *d_hash = nullptr;       // the count pass's hubs counted in shares
+  uint32_t n_hash = 0;
   size_t hash_cap = 0;
   size_t citems_cap = 0;
   int grid_count = 0;                        // count-pass kernel
