@@ -706,7 +706,7 @@ __device__ void light_chunk(const IterArgs &a, const Ctx &c, uint32_t *stage, un
     const uint32_t incl = warp_incl_scan(sd, lane);
     const bool in_batch = pending && incl <= cap_stage;
     const uint32_t batch = __ballot_sync(kFull, in_batch);
-    const uint32_t lo = __ffs(batch) - 1, hi = 32 - __clz(batch);
+    const uint32_t hi = 32 - __clz(batch);
     const uint32_t total = __shfl_sync(kFull, incl, hi - 1);
     const uint32_t base = incl - sd;
     // 1. ids: the batch decoded by all lanes together
@@ -732,81 +732,68 @@ __device__ void light_chunk(const IterArgs &a, const Ctx &c, uint32_t *stage, un
     }
     __syncwarp();
     // 3. count
-    const uint32_t dmax = __reduce_max_sync(kFull, in_batch ? d : 0u);
-    if (dmax <= 32 && (variant == kVarPacked || dmax <= 1)) {
-      // several vertices per round: G lanes per vertex
-      const uint32_t G = next_pow2(dmax);
-      const uint32_t per = 32 / G;
-      const uint32_t gl = lane / G, k = lane % G;
-      const uint32_t gm = (G == 32) ? kFull : (((1u << G) - 1u) << (gl * G));
-      for (uint32_t v0 = lo; v0 < hi; v0 += per) {
-        const uint32_t vi = v0 + gl;
-        const bool vin = vi < hi;
-        const uint32_t srcl = vin ? vi : lo;
-        const uint32_t dv = __shfl_sync(kFull, d, srcl);
-        const uint32_t bv = __shfl_sync(kFull, base, srcl);
-        const uint32_t nodev = __shfl_sync(kFull, node, srcl);
-        const uint32_t oldv = __shfl_sync(kFull, old, srcl);
-        const bool ok = vin && k < dv;
-        const uint32_t lab = ok ? stage[bv + k] : kFull;
-        const uint32_t cnt = group_counts(ok, lab, gm, gl);
-        const uint32_t maxc = __reduce_max_sync(gm, cnt);
-        const uint32_t bestl = __reduce_min_sync(gm, (ok && cnt == maxc) ? lab : kFull);
-        if (vin && k == 0) {
-          const uint32_t nl = dv ? bestl : oldv;
-          c.lab_out[nodev] = nl;
-          my_changed += (nl != oldv);
+    // vertices of degree <= 32: a lane each; one whose labels all agree takes
+    // that label at once
+    uint32_t nl = old;
+    const bool few = in_batch && d <= 32;
+    bool mixed = false;
+    if (few && d) {
+      nl = stage[base];
+      for (uint32_t j = 1; j < d; j++) mixed |= stage[base + j] != nl;
+    }
+    if (uint32_t rest = __ballot_sync(kFull, mixed)) {
+      if (one_by_one(__popc(rest), __reduce_max_sync(kFull, mixed ? d : 0u))) {
+        for (; rest; rest &= rest - 1u) {
+          const uint32_t l = uint32_t(__ffs(rest) - 1);
+          const uint32_t x = warp_mode(stage + __shfl_sync(kFull, base, l), __shfl_sync(kFull, d, l));
+          if (lane == l) nl = x;
         }
+      } else if (mixed) {
+        nl = lane_mode(stage + base, d);
       }
-    } else {
-      // one vertex per round
-      for (uint32_t j = lo; j < hi; j++) {
-        const uint32_t dv = __shfl_sync(kFull, d, j);
-        const uint32_t bv = __shfl_sync(kFull, base, j);
-        const uint32_t nodev = __shfl_sync(kFull, node, j);
-        const uint32_t oldv = __shfl_sync(kFull, old, j);
-        uint32_t bestl;
-        if (dv <= 32) {
-          const bool ok = lane < dv;
-          const uint32_t lab = ok ? stage[bv + lane] : kFull;
-          const uint32_t cnt = group_counts(ok, lab, kFull, 0u);
-          const uint32_t maxc = __reduce_max_sync(kFull, cnt);
-          bestl = __reduce_min_sync(kFull, (ok && cnt == maxc) ? lab : kFull);
-        } else {
-          // epoch table: no clearing, running argmax from the returned counts
-          if (++epoch >= kLightEpochs) {
-            for (uint32_t i = lane; i < kWarpSlots; i += 32) slots[i] = 0ull;
-            __syncwarp();
-            epoch = 1;
-          }
-          const EpochTable et{slots, min(next_pow2(2 * dv), kWarpSlots), epoch};  // cap > dv: every label fits
-          uint64_t bp = 0;
-          const auto ins = [&](uint32_t lab, uint32_t w) {
-            const uint64_t cand = pack_best(et.insert(lab, w), lab);
-            bp = cand > bp ? cand : bp;
-          };
-          // a step of one label extends the current run (fixed plan at R-MAT
-          // scale 24: 13.48 -> 13.21 ms per iteration)
-          WarpRun run;
-          for (uint32_t k0 = 0; k0 < dv; k0 += 32) {
-            const uint32_t k = k0 + lane;
-            const bool ok = k < dv;
-            const uint32_t lab = ok ? stage[bv + k] : kFull;
-            if (run.extend(ok, lab)) continue;
-            if (run.cnt && lane == 0) ins(run.lab, run.cnt);
-            run.restart(ok, lab);
-            const uint32_t w = warp_merge(ok, lab);
-            if (w) ins(lab, w);
-          }
-          if (run.cnt && lane == 0) ins(run.lab, run.cnt);
-          bestl = best_label(warp_max_u64(bp));
-          __syncwarp();
-        }
-        if (lane == 0) {
-          const uint32_t nl = dv ? bestl : oldv;
-          c.lab_out[nodev] = nl;
-          my_changed += (nl != oldv);
-        }
+    }
+    if (few) {
+      c.lab_out[node] = nl;
+      my_changed += (nl != old);
+    }
+    // the others by the warp, one after another
+    for (uint32_t m = __ballot_sync(kFull, in_batch && d > 32); m; m &= m - 1u) {
+      const uint32_t j = __ffs(m) - 1;
+      const uint32_t dv = __shfl_sync(kFull, d, j);
+      const uint32_t bv = __shfl_sync(kFull, base, j);
+      const uint32_t nodev = __shfl_sync(kFull, node, j);
+      const uint32_t oldv = __shfl_sync(kFull, old, j);
+      // epoch table: no clearing, running argmax from the returned counts
+      if (++epoch >= kLightEpochs) {
+        for (uint32_t i = lane; i < kWarpSlots; i += 32) slots[i] = 0ull;
+        __syncwarp();
+        epoch = 1;
+      }
+      const EpochTable et{slots, min(next_pow2(2 * dv), kWarpSlots), epoch};  // cap > dv: every label fits
+      uint64_t bp = 0;
+      const auto ins = [&](uint32_t lab, uint32_t w) {
+        const uint64_t cand = pack_best(et.insert(lab, w), lab);
+        bp = cand > bp ? cand : bp;
+      };
+      // a step of one label extends the current run (fixed plan at R-MAT
+      // scale 24: 13.48 -> 13.21 ms per iteration)
+      WarpRun run;
+      for (uint32_t k0 = 0; k0 < dv; k0 += 32) {
+        const uint32_t k = k0 + lane;
+        const bool ok = k < dv;
+        const uint32_t lab = ok ? stage[bv + k] : kFull;
+        if (run.extend(ok, lab)) continue;
+        if (run.cnt && lane == 0) ins(run.lab, run.cnt);
+        run.restart(ok, lab);
+        const uint32_t w = warp_merge(ok, lab);
+        if (w) ins(lab, w);
+      }
+      if (run.cnt && lane == 0) ins(run.lab, run.cnt);
+      const uint32_t bestl = best_label(warp_max_u64(bp));
+      __syncwarp();
+      if (lane == 0) {
+        c.lab_out[nodev] = bestl;
+        my_changed += (bestl != oldv);
       }
     }
     __syncwarp();
@@ -1915,31 +1902,20 @@ __global__ void __launch_bounds__(kThreads, 5) k_count_two_pass(IterArgs a) {
           c.lab_out[node] = first;
           my_changed += (first != old);
         }
-        const uint32_t rest = __ballot_sync(kFull, mixed);
-        if (rest) {
-          // G-lane groups over the mixed vertices, 32 / G of them a round
-          const uint32_t nrest = __popc(rest);
-          const uint32_t dmax = __reduce_max_sync(kFull, mixed ? d : 0u);
-          const uint32_t G = next_pow2(dmax);
-          const uint32_t per = 32 / G;
-          const uint32_t gl = lane / G, k = lane % G;
-          const uint32_t gm = (G == 32) ? kFull : (((1u << G) - 1u) << (gl * G));
-          for (uint32_t v0 = 0; v0 < nrest; v0 += per) {
-            const bool vin = v0 + gl < nrest;
-            const uint32_t srcl = vin ? __fns(rest, 0, v0 + gl + 1) : 0u;
-            const uint32_t dv = __shfl_sync(kFull, d, srcl);
-            const uint32_t nodev = __shfl_sync(kFull, node, srcl);
-            const uint32_t oldv = __shfl_sync(kFull, old, srcl);
-            const uint32_t ev = __shfl_sync(kFull, excl, srcl);
-            const bool ok = vin && k < dv;
-            const uint32_t lab = ok ? lbl[ev + k] : kFull;
-            const uint32_t cnt = group_counts(ok, lab, gm, gl);
-            const uint32_t maxc = __reduce_max_sync(gm, cnt);
-            const uint32_t bestl = __reduce_min_sync(gm, (ok && cnt == maxc) ? lab : kFull);
-            if (vin && k == 0) {
-              c.lab_out[nodev] = bestl;
-              my_changed += (bestl != oldv);
+        if (uint32_t rest = __ballot_sync(kFull, mixed)) {
+          uint32_t nl = 0;
+          if (one_by_one(__popc(rest), __reduce_max_sync(kFull, mixed ? d : 0u))) {
+            for (; rest; rest &= rest - 1u) {
+              const uint32_t l = uint32_t(__ffs(rest) - 1);
+              const uint32_t x = warp_mode(lbl + __shfl_sync(kFull, excl, l), __shfl_sync(kFull, d, l));
+              if (lane == l) nl = x;
             }
+          } else if (mixed) {
+            nl = lane_mode(lbl + excl, d);
+          }
+          if (mixed) {
+            c.lab_out[node] = nl;
+            my_changed += (nl != old);
           }
         }
         __syncwarp();
