@@ -2070,7 +2070,54 @@ __global__ void k_pos_index(DevGraph g, uint4 *pidx, uint32_t *err, uint64_t p_l
   }
 }
 
-// Decode positions into a CSR scratch (parity hook).
+// The CSR by vertex id (lpa_decode_csr): where every vertex sits, its degree in
+// row[v] (scanned by the caller), then the lists of the ids [v0, v1) into out,
+// row[v0] first.  A vertex without a position has no neighbours.
+__global__ void k_csr_inverse(const uint32_t *vertices, uint64_t n, uint32_t *pos) {
+  for (uint64_t p = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; p < n; p += uint64_t(gridDim.x) * blockDim.x)
+    pos[vertices[p]] = uint32_t(p);
+}
+__global__ void k_csr_degrees(const uint32_t *deg, const uint32_t *pos, uint64_t n, uint64_t *row) {
+  for (uint64_t v = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; v <= n; v += uint64_t(gridDim.x) * blockDim.x)
+    row[v] = v < n && pos[v] != kFull ? deg[pos[v]] : 0u;
+}
+// A warp per 32 ids (warp_decode_batch: a lane per header, the residual
+// segments spread over the lanes); ids with more than kCsrSplit arcs among
+// them go to 8 warps, 4 ids each.  The lists keep the order of the stream,
+// intervals first.
+__global__ void __launch_bounds__(kThreads) k_decode_csr(DevGraph g, const uint32_t *pos, const uint64_t *row,
+                                                         uint64_t v0, uint64_t v1, uint32_t *out, uint32_t *err) {
+  constexpr uint32_t kCsrSplit = 4096;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t nw = (uint64_t(gridDim.x) * blockDim.x) >> 5, chunks = (v1 - v0 + 31) / 32;
+  const uint64_t r0 = row[v0];
+  for (uint64_t w = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5; w < chunks * 8; w += nw) {
+    const uint64_t v = v0 + (w >> 3) * 32 + lane;
+    const uint32_t share = uint32_t(w) & 7u;
+    uint32_t p = kFull, d = 0, base = 0;
+    if (v < v1) {
+      p = pos[v];
+      base = uint32_t(row[v] - r0);  // a chunk of ids holds fewer than 2^32 arcs
+      d = uint32_t(row[v + 1] - row[v]);
+    }
+    if (__reduce_add_sync(kFull, min(d, kCsrSplit + 1)) > kCsrSplit) {
+      if ((lane >> 2) != share) d = 0;
+    } else if (share) {
+      continue;
+    }
+    const bool cgr = d != 0 && p < g.n_c, small = d != 0 && p >= g.n_c;
+    if (__any_sync(kFull, cgr) && !warp_decode_batch(g, out, cgr, p, uint32_t(v), cgr ? d : 0u, base, lane) && lane == 0)
+      set_error(err, kErrBadStream);
+    for (uint32_t m = __ballot_sync(kFull, small); m; m &= m - 1u) {
+      const uint32_t l = uint32_t(__ffs(m) - 1);
+      const uint32_t pl = __shfl_sync(kFull, p, l), dl = __shfl_sync(kFull, d, l), bl = __shfl_sync(kFull, base, l);
+      const uint32_t *src = g.small_nbr + g.small_off[pl - g.n_c];
+      for (uint32_t k = lane; k < dl; k += 32) out[bl + k] = __ldg(src + k);
+    }
+  }
+}
+
+// Decode positions into a CSR scratch (out-of-core handles).
 __global__ void k_decode_positions(DecodeArgs a) {
   const DevGraph &g = a.g;
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < a.n_pos;

@@ -280,6 +280,11 @@ struct DecodeArgs {
 };
 __global__ void k_decode_positions(DecodeArgs a);
 
+__global__ void k_csr_inverse(const uint32_t *vertices, uint64_t n, uint32_t *pos);
+__global__ void k_csr_degrees(const uint32_t *deg, const uint32_t *pos, uint64_t n, uint64_t *row);
+__global__ void k_decode_csr(DevGraph g, const uint32_t *pos, const uint64_t *row, uint64_t v0, uint64_t v1,
+                             uint32_t *out, uint32_t *err);
+
 // Per compressed position: where its interval and residual sections'
 // segments start (relative to its bit offset) and how many each has.
 // Positions [p_lo, p_hi) (compressed ones only).

@@ -309,6 +309,10 @@ int grid_for(uint64_t work, int num_sms) {
 
 }  // namespace
 
+cudaError_t exclusive_sum(uint64_t *data, uint64_t n, void *temp, size_t &temp_bytes, cudaStream_t st) {
+  return cub::DeviceScan::ExclusiveSum(temp, temp_bytes, data, data, n, st);
+}
+
 void PlanBuilder::release() {
   for (void *p : bufs)
     if (p) cudaFree(p);

@@ -42,6 +42,9 @@ struct PlanInputs {
   int num_sms;
 };
 
+// Exclusive sum of data[0..n) in place (CUB); temp nullptr: only its size.
+cudaError_t exclusive_sum(uint64_t *data, uint64_t n, void *temp, size_t &temp_bytes, cudaStream_t st);
+
 // The lists, in the caller's device buffers.  build() sets the counts, then
 // calls grow(), which must make the buffers hold them (it may reallocate),
 // then writes the lists: items = heavy items (largest first) followed by

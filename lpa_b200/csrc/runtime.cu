@@ -891,6 +891,70 @@ static void collect_times(lpa_handle *h) {
   h->last_iter_ms = h->ev_used > 1 ? ms(0, h->ev_used - 1) : 0.0;
 }
 
+// Device memory of one call.
+template <class T>
+struct TempBuf {
+  T *p = nullptr;
+  cudaError_t alloc(uint64_t count) {
+    const cudaError_t e = cudaMalloc(&p, std::max<uint64_t>(count, 1) * sizeof(T));
+    if (e != cudaSuccess) {
+      p = nullptr;
+      cudaGetLastError();
+    }
+    return e;
+  }
+  ~TempBuf() {
+    if (p) cudaFree(p);
+  }
+};
+
+// The CSR by vertex id of a resident handle: rows and lists are put together
+// on the device, in ranges of ids that fit a buffer, and copied straight to the
+// caller's arrays (a host loop over the vertices took most of 74 ms for a
+// 1M-vertex, 26M-arc graph).
+static lpa_status decode_csr_resident(lpa_handle *h, uint64_t *row_out, uint32_t *clm_out) {
+  constexpr uint64_t kBufArcs = 1ull << 26;
+  const int blocks = h->num_sms * 8;
+  TempBuf<uint32_t> pos, out;
+  TempBuf<uint64_t> row;
+  TempBuf<uint8_t> temp;
+  size_t temp_bytes = 0;
+  check(h, pos.alloc(h->n), "decode positions");
+  check(h, row.alloc(h->n + 1), "decode rows");
+  check(h, exclusive_sum(row.p, h->n + 1, nullptr, temp_bytes, h->stream), "decode scan");
+  check(h, temp.alloc(temp_bytes), "decode scan");
+  check(h, cudaMemsetAsync(pos.p, 0xFF, h->n * sizeof(uint32_t), h->stream), "clear positions");
+  k_csr_inverse<<<blocks, 256, 0, h->stream>>>(h->d_vertices, h->n, pos.p);
+  k_csr_degrees<<<blocks, 256, 0, h->stream>>>(h->d_deg, pos.p, h->n, row.p);
+  check(h, exclusive_sum(row.p, h->n + 1, temp.p, temp_bytes, h->stream), "decode scan");
+  check(h, cudaGetLastError(), "decode rows launch");
+  check(h, cudaMemcpyAsync(row_out, row.p, (h->n + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream),
+        "read rows");
+  check(h, cudaStreamSynchronize(h->stream), "read rows");
+  // the buffer: everything at once when that fits, at least the longest list
+  uint64_t cap = std::max<uint64_t>(h->max_deg, std::min<uint64_t>(row_out[h->n], kBufArcs));
+  while (out.alloc(cap) != cudaSuccess) {
+    if (cap <= h->max_deg) throw Fail{LPA_ERR_OOM, "decode buffer"};
+    cap = std::max<uint64_t>(h->max_deg, cap / 4);
+  }
+  for (uint64_t v0 = 0; v0 < h->n;) {
+    // the ids whose lists fit the buffer, from v0 on
+    const uint64_t v1 = uint64_t(std::upper_bound(row_out + v0, row_out + h->n + 1, row_out[v0] + cap) - row_out) - 1;
+    const uint64_t arcs = row_out[v1] - row_out[v0];
+    if (arcs) {
+      const uint64_t warps = (v1 - v0 + 31) / 32 * 8;
+      const int grid = int(std::min<uint64_t>((warps + kWarps - 1) / kWarps, uint64_t(blocks) * 16));
+      k_decode_csr<<<grid, kThreads, 0, h->stream>>>(dev_graph(h), pos.p, row.p, v0, v1, out.p, h->d_err);
+      check(h, cudaGetLastError(), "decode launch");
+      check(h, cudaMemcpyAsync(clm_out + row_out[v0], out.p, arcs * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream),
+            "read decode");
+      check(h, cudaStreamSynchronize(h->stream), "read decode");
+    }
+    v0 = v1;
+  }
+  return take_device_error(h);
+}
+
 // ------------------------------------------------------------------ C ABI --
 extern "C" {
 
@@ -1255,6 +1319,7 @@ lpa_status lpa_decode_csr(lpa_handle *h, uint64_t *row_out, uint32_t *clm_out) {
   if (!h || !row_out || (!clm_out && h->m)) return LPA_ERR_INVALID_ARG;
   try {
     check(h, cudaSetDevice(h->device), "cudaSetDevice");
+    if (!h->streamed) return decode_csr_resident(h, row_out, clm_out);
     ensure_two_pass_scratch(h, true);
     const std::vector<uint64_t> &off = h->h_arc_off;
     std::vector<uint32_t> ids(off[h->n_c]);
@@ -1263,32 +1328,21 @@ lpa_status lpa_decode_csr(lpa_handle *h, uint64_t *row_out, uint32_t *clm_out) {
     a.pos_list = nullptr;
     a.arc_off = h->d_arc_off;
     a.err = h->d_err;
-    auto decode = [&](uint64_t p0, uint64_t p1) {
-      a.pos_begin = p0;
-      a.n_pos = p1 - p0;
+    // range by range through one stream buffer and the scratch
+    for (const StreamRange &r : h->ranges) {
+      if (r.p1 <= r.p0) continue;
+      a.g.words = stage_words(h, 0, r.w0, r.w1, h->stream);
+      a.out = scratch_base(h, r.a0);
+      a.pos_begin = r.p0;
+      a.n_pos = r.p1 - r.p0;
       const int blocks = int(std::max<uint64_t>(1, std::min<uint64_t>((a.n_pos + 255) / 256, uint64_t(h->num_sms) * 8)));
-      if (a.n_pos) k_decode_positions<<<blocks, 256, 0, h->stream>>>(a);
+      k_decode_positions<<<blocks, 256, 0, h->stream>>>(a);
       check(h, cudaGetLastError(), "decode launch");
-      return take_device_error(h);
-    };
-    if (h->streamed) {  // range by range through one stream buffer and the scratch
-      for (const StreamRange &r : h->ranges) {
-        if (r.p1 <= r.p0) continue;
-        a.g.words = stage_words(h, 0, r.w0, r.w1, h->stream);
-        a.out = scratch_base(h, r.a0);
-        lpa_status st = decode(r.p0, r.p1);
-        if (st != LPA_OK) return st;
-        if (r.a1 > r.a0)
-          check(h, cudaMemcpy(ids.data() + r.a0, h->d_scratch + (r.a0 & 3u), (r.a1 - r.a0) * 4, cudaMemcpyDeviceToHost),
-                "read decode");
-      }
-    } else {
-      a.out = h->d_scratch;
-      lpa_status st = decode(0, h->n_c);
+      lpa_status st = take_device_error(h);
       if (st != LPA_OK) return st;
-      check(h, cudaMemcpy(ids.data(), h->d_scratch, h->hub_arcs * 4, cudaMemcpyDeviceToHost), "read decode");
-      check(h, cudaMemcpy(ids.data() + h->hub_arcs, h->d_scratch_rest, (ids.size() - h->hub_arcs) * 4,
-                          cudaMemcpyDeviceToHost), "read decode");
+      if (r.a1 > r.a0)
+        check(h, cudaMemcpy(ids.data() + r.a0, h->d_scratch + (r.a0 & 3u), (r.a1 - r.a0) * 4, cudaMemcpyDeviceToHost),
+              "read decode");
     }
     std::vector<uint32_t> verts(h->n);
     check(h, cudaMemcpy(verts.data(), h->d_vertices, h->n * 4, cudaMemcpyDeviceToHost), "read vertices");
