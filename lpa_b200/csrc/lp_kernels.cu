@@ -1068,10 +1068,73 @@ __global__ void k_batch_init(const BatchGraph *graphs, uint32_t ngraphs) {
   }
 }
 
-// One vertex of degree <= kPackedMaxDeg by one thread: it walks the vertex's
-// whole bit range (or its small-CSR list), gathering each label as soon as
-// its id is decoded, then takes the most frequent of its labels (smallest on
-// ties) by pairwise counts.  Returns 1 when the label changed.
+// The d ids of a vertex of degree d <= kPackedRegs with the commonest layout
+// (no intervals, one residual segment, at most 128 bits, gaps below 2^24), in
+// registers: the count is known, so the headers are compared, not decoded, and
+// the codes come from a 128-bit window without refills or position arithmetic.
+// False when the vertex is not of that layout (the walk takes it).
+constexpr uint32_t kPackedRegs = 8;
+__device__ __forceinline__ bool packed_ids(const DevGraph &g, uint32_t p, uint32_t node, uint32_t d,
+                                           uint32_t (&id)[kPackedRegs]) {
+  const uint64_t o0 = g.offsets[p], len = g.offsets[p + 1] - o0;
+  if (len > 128) return false;
+  const uint32_t *w = g.words + (o0 >> 5);
+  const uint32_t s = uint32_t(o0) & 31u, bits = s + uint32_t(len);
+  // words past the vertex's last are never needed
+  const uint32_t w0 = __ldg(w), w1 = bits > 32 ? __ldg(w + 1) : 0u, w2 = bits > 64 ? __ldg(w + 2) : 0u,
+                 w3 = bits > 96 ? __ldg(w + 3) : 0u, w4 = bits > 128 ? __ldg(w + 4) : 0u;
+  uint32_t x0 = __funnelshift_l(w1, w0, s), x1 = __funnelshift_l(w2, w1, s), x2 = __funnelshift_l(w3, w2, s),
+           x3 = __funnelshift_l(w4, w3, s);
+  uint32_t used = 0;
+  const auto skip = [&](uint32_t k) {  // k <= 32
+    x0 = __funnelshift_lc(x1, x0, k);
+    x1 = __funnelshift_lc(x2, x1, k);
+    x2 = __funnelshift_lc(x3, x2, k);
+    x3 = __funnelshift_lc(0u, x3, k);
+    used += k;
+  };
+  // "11": no intervals; "1" and a 0: one residual segment, whose count follows
+  const uint32_t cl = 2u * (31u - __clz(d + 1u)) + 1u;  // gamma(d)
+  if (x0 >> 28 != 0xEu || (x0 << 3) >> (32u - cl) != d + 1u) return false;
+  skip(3u + cl);
+  uint32_t v = 0;
+  bool ok = true;
+#pragma unroll
+  for (uint32_t u = 0; u < kPackedRegs; u++) {
+    if (u < d) {
+      const uint32_t h = min(__clz(x0), 8);  // zeta_3: 4 (h + 1) bits
+      ok &= h < 8u;
+      const uint32_t x = ((x0 << (h + 1u)) >> (29u - 3u * min(h, 7u))) - 1u;
+      v = u == 0 ? zigzag_first(node, x) : v + x + 1u;
+      skip(min(4u * (h + 1u), 32u));
+    }
+    id[u] = min(v, uint32_t(g.n - 1));  // a gather never leaves the labels
+  }
+  return ok && used == uint32_t(len) && uint64_t(v) < g.n;
+}
+
+// The most frequent of lab[0..d), d >= 1, the smallest on ties: a label's
+// first occurrence counts all of them.
+__device__ __forceinline__ uint32_t packed_mode(const uint32_t (&lab)[kPackedRegs], uint32_t d) {
+  uint32_t bc = 0, bl = 0;
+#pragma unroll
+  for (uint32_t u = 0; u < kPackedRegs; u++) {
+    uint32_t c = 1;
+#pragma unroll
+    for (uint32_t y = u + 1; y < kPackedRegs; y++) c += (y < d && lab[y] == lab[u]) ? 1u : 0u;
+    if (u < d && (c > bc || (c == bc && lab[u] < bl))) {
+      bc = c;
+      bl = lab[u];
+    }
+  }
+  return bl;
+}
+
+// One vertex of degree <= kPackedMaxDeg by one thread.  Up to kPackedRegs ids
+// and labels stay in registers (road grid 1404^2, 2M vertices of degree <= 7:
+// k_packed 72 -> 47 us); else the thread walks the vertex's bit range (or its
+// small-CSR list) into its label slots, issues every label load at once and
+// counts there (lane_mode).  Returns 1 when the label changed.
 // lab: this thread's kPackedMaxDeg label slots (shared memory in k_packed,
 // where a lane's slots start kPackedMaxDeg words after the previous lane's:
 // an odd stride, so the 32 lanes' k-th slots fall in 32 different banks).
@@ -1080,42 +1143,50 @@ __device__ __forceinline__ uint32_t packed_vertex(const IterArgs &a, const Ctx &
   const uint32_t node = g.vertices[p];
   const uint32_t d = g.deg[p];
   const uint32_t old = ld_label(c, node);
-  uint32_t k = 0;
-  bool bad = d > kPackedMaxDeg;
-  if (!bad && p < g.n_c) {
-    // the walk stages the ids, then every label load is in flight at once (a
-    // load in the walk's loop held the lane at its store: road grid 1404^2,
-    // k_packed 0.096 -> 0.079 ms)
-    const int64_t r = walk_vertex_buf<true>(g.words, g.offsets[p], g.offsets[p + 1], node, g.n, [&](uint32_t id) {
-      if (k < kPackedMaxDeg) lab[k] = id;
-      k++;
-    });
-    bad = r != int64_t(d);
-    if (!bad) {
-      uint32_t lv[kPackedMaxDeg];
-#pragma unroll
-      for (uint32_t j = 0; j < kPackedMaxDeg; j++) lv[j] = j < d ? ld_label(c, lab[j]) : 0u;
-#pragma unroll
-      for (uint32_t j = 0; j < kPackedMaxDeg; j++)
-        if (j < d) lab[j] = lv[j];
-    }
-  } else if (!bad) {
-    const uint32_t *ids = g.small_nbr + g.small_off[p - g.n_c];
-    for (; k < d; k++) lab[k] = ld_label(c, ids[k]);
-  }
-  if (bad) {
-    set_error(a.err, kErrBadStream);
-    return 0;
-  }
   if (d == 0) return 0;
-  uint64_t best = 0;
-  for (uint32_t x = 0; x < d; x++) {
-    uint32_t cnt = 0;
-    for (uint32_t y = 0; y < d; y++) cnt += lab[y] == lab[x];
-    const uint64_t cand = pack_best(cnt, lab[x]);
-    best = cand > best ? cand : best;
+  const bool cgr = p < g.n_c;
+  const uint32_t *ids = cgr ? nullptr : g.small_nbr + g.small_off[p - g.n_c];
+  uint32_t nl = old;
+  bool done = false;
+  if (d <= kPackedRegs) {
+    uint32_t r[kPackedRegs];
+    done = true;
+    if (cgr) {
+      done = packed_ids(g, p, node, d, r);
+    } else {
+#pragma unroll
+      for (uint32_t u = 0; u < kPackedRegs; u++) r[u] = u < d ? __ldg(ids + u) : 0u;
+    }
+    if (done) {
+#pragma unroll
+      for (uint32_t u = 0; u < kPackedRegs; u++) r[u] = u < d ? ld_label(c, r[u]) : 0u;
+      nl = packed_mode(r, d);
+    }
   }
-  const uint32_t nl = best_label(best);
+  if (!done) {
+    uint32_t k = 0;
+    bool bad = d > kPackedMaxDeg;
+    if (!bad && cgr) {
+      const int64_t r = walk_vertex_buf<true>(g.words, g.offsets[p], g.offsets[p + 1], node, g.n, [&](uint32_t id) {
+        if (k < kPackedMaxDeg) lab[k] = id;
+        k++;
+      });
+      bad = r != int64_t(d);
+    }
+    if (bad) {
+      set_error(a.err, kErrBadStream);
+      return 0;
+    }
+    uint32_t lv[kPackedMaxDeg];
+#pragma unroll
+    for (uint32_t j = 0; j < kPackedMaxDeg; j++) lv[j] = j < d ? (cgr ? lab[j] : __ldg(ids + j)) : 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < kPackedMaxDeg; j++) lv[j] = j < d ? ld_label(c, lv[j]) : 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < kPackedMaxDeg; j++)
+      if (j < d) lab[j] = lv[j];
+    nl = lane_mode(lab, d);
+  }
   c.lab_out[node] = nl;
   return nl != old;
 }
