@@ -743,6 +743,14 @@ static IterArgs iter_args(lpa_handle *h, unsigned long long *changed, uint32_t *
 // zero.
 static void enqueue_streamed_iteration(lpa_handle *h, unsigned long long *changed, uint32_t *work);
 
+// The streams and events of the captured iteration's branches.
+static void ensure_side_streams(lpa_handle *h) {
+  if (h->ev_fork) return;
+  for (auto &s : h->side) check(h, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "side stream");
+  for (auto &e : h->ev_join) check(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "events");
+  check(h, cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming), "events");
+}
+
 static void enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32_t *work) {
   if (h->streamed) {
     enqueue_streamed_iteration(h, changed, work);
@@ -759,6 +767,21 @@ static void enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
     cudaEventRecord(h->ev[ne++], h->stream);
   };
   mark(-1);
+  // In the captured iteration the kernels of different vertices are parallel
+  // branches, so that one's blocks fill the SMs that the last blocks of another
+  // leave idle.  The two-pass kernels are one branch; k_iterate joins it when
+  // it may count what the pre-pass decoded (heavy items).
+  const bool two = h->n_groups || h->n_cblock + h->n_cwarp;
+  const bool fork = h->loop_it && int(two) + int(h->n_packed != 0) + int(h->n_heavy + h->n_light != 0) > 1;
+  cudaStream_t s_packed = h->stream, s_iter = h->stream;
+  if (fork) {
+    ensure_side_streams(h);
+    cudaEventRecord(h->ev_fork, h->stream);
+    if (h->n_packed && (two || h->n_heavy + h->n_light)) s_packed = h->side[0];
+    if (h->n_heavy + h->n_light && two && !(h->n_groups && h->n_heavy)) s_iter = h->side[1];
+    for (cudaStream_t s : {s_packed, s_iter})
+      if (s != h->stream) cudaStreamWaitEvent(s, h->ev_fork, 0);
+  }
   if (h->n_groups) {
     launch_decode_two_pass(h->tune.gather_cache, h->tune.stage_stream, h->grid_decode, h->stream, a);
     h->launches++;
@@ -770,14 +793,19 @@ static void enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
     mark(1);
   }
   if (h->n_packed) {
-    k_packed<<<h->grid_packed, kThreads, 0, h->stream>>>(a);
+    k_packed<<<h->grid_packed, kThreads, 0, s_packed>>>(a);
     h->launches++;
     mark(2);
   }
   if (h->n_heavy + h->n_light) {
-    k_iterate<<<h->grid, kThreads, kSmemBytes, h->stream>>>(a);
+    k_iterate<<<h->grid, kThreads, kSmemBytes, s_iter>>>(a);
     h->launches++;
     mark(3);
+  }
+  for (int k = 0; k < 2; k++) {
+    if ((k ? s_iter : s_packed) == h->stream) continue;
+    cudaEventRecord(h->ev_join[k], h->side[k]);
+    cudaStreamWaitEvent(h->stream, h->ev_join[k], 0);
   }
   if (h->d_gtrack) {
     lpa_rt_enqueue_track(h);
@@ -1140,6 +1168,11 @@ lpa_status lpa_destroy(lpa_handle *h) {
     if (h->ev_free[b]) cudaEventDestroy(h->ev_free[b]);
   }
   if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
+  for (auto &s : h->side)
+    if (s) cudaStreamDestroy(s);
+  for (auto &e : h->ev_join)
+    if (e) cudaEventDestroy(e);
+  if (h->ev_fork) cudaEventDestroy(h->ev_fork);
   for (auto &e : h->ev)
     if (e) cudaEventDestroy(e);
   lpa_learner_free(h);

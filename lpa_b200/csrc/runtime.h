@@ -134,6 +134,8 @@ struct lpa_handle {
   // scratch
   uint64_t *d_arc_off = nullptr;
   uint32_t *d_scratch = nullptr;
+  cudaStream_t side[2] = {nullptr, nullptr};  // branches of the captured iteration
+  cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
   uint32_t *d_gtab = nullptr;
   uint32_t *d_scratch_rest = nullptr;  // the labels of the positions that are no hubs
   int scratch_scope = 0;               // scratch holds nothing, the hubs' labels, every compressed position's
