@@ -108,40 +108,54 @@ lpa_status lpa_run_graph(lpa_handle *h, int max_iter, bool early_exit, int *iter
   cudaError_t e = cudaSetDevice(h->device);
   if (e != cudaSuccess) return fail(e, "cudaSetDevice");
   if (!h->d_loop_it) {
-    e = cudaMalloc(&h->d_loop_it, 4 * sizeof(uint32_t));
+    // the loop control, then (packed loop) its barrier
+    e = cudaMalloc(&h->d_loop_it, sizeof(lpa_dev::PackedLoop));
     if (e != cudaSuccess) return fail(e, "loop counter");
     h->allocations.push_back(h->d_loop_it);
   }
-  if (!h->graph_exec || h->graph_plan_version != h->plan_version) {
+  const bool packed = lpa_rt_packed_loop_grid(h) > 0;
+  if (!packed && (!h->graph_exec || h->graph_plan_version != h->plan_version)) {
     e = build_graph(h);
     if (e != cudaSuccess) return fail(e, "build iteration graph");
   }
+  // pinned: the control sent, the control and (short runs) the counters back
   const uint32_t start = uint32_t(h->cur);
-  uint32_t *ctl = reinterpret_cast<uint32_t *>(h->h_pinned);
-  ctl[0] = start;
-  ctl[1] = start + uint32_t(max_iter);
-  ctl[2] = early_exit ? 1u : 0u;
+  lpa_dev::PackedLoop *ctl = reinterpret_cast<lpa_dev::PackedLoop *>(h->h_pinned);
+  lpa_dev::PackedLoop *back = ctl + 1;
+  *ctl = lpa_dev::PackedLoop{start, start + uint32_t(max_iter), early_exit ? 1u : 0u, start, 0u, 0u};
   e = cudaMemsetAsync(h->d_changed, 0, size_t(max_iter + 2) * sizeof(unsigned long long), h->stream);
   if (e != cudaSuccess) return fail(e, "clear counters");
-  e = cudaMemsetAsync(h->d_work, 0, size_t(lpa_dev::kWorkCounters) * size_t(max_iter + 2) * sizeof(uint32_t), h->stream);
-  if (e != cudaSuccess) return fail(e, "clear work counters");
-  e = cudaMemcpyAsync(h->d_loop_it, ctl, 3 * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream);
+  e = cudaMemcpyAsync(h->d_loop_it, ctl, sizeof(*ctl), cudaMemcpyHostToDevice, h->stream);
   if (e != cudaSuccess) return fail(e, "loop control");
-  e = cudaGraphLaunch(static_cast<cudaGraphExec_t>(h->graph_exec), h->stream);
-  if (e != cudaSuccess) return fail(e, "graph launch");
-  uint32_t it_end = 0;
-  e = cudaMemcpyAsync(&it_end, h->d_loop_it, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream);
+  if (packed) {
+    e = lpa_rt_launch_packed_loop(h);
+    if (e != cudaSuccess) return fail(e, "packed loop launch");
+  } else {
+    e = cudaMemsetAsync(h->d_work, 0, size_t(lpa_dev::kWorkCounters) * size_t(max_iter + 2) * sizeof(uint32_t),
+                        h->stream);
+    if (e != cudaSuccess) return fail(e, "clear work counters");
+    e = cudaGraphLaunch(static_cast<cudaGraphExec_t>(h->graph_exec), h->stream);
+    if (e != cudaSuccess) return fail(e, "graph launch");
+  }
+  e = cudaMemcpyAsync(back, h->d_loop_it, sizeof(*back), cudaMemcpyDeviceToHost, h->stream);
   if (e != cudaSuccess) return fail(e, "read loop counter");
-  std::vector<unsigned long long> hist(size_t(max_iter) + 2);
-  e = cudaMemcpyAsync(hist.data(), h->d_changed, hist.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+  std::vector<unsigned long long> own;
+  unsigned long long *hist = h->h_pinned + 8;
+  if (max_iter + 2 > kPinnedSlots - 9) {  // the last slot takes the error word
+    own.resize(size_t(max_iter) + 2);
+    hist = own.data();
+  }
+  e = cudaMemcpyAsync(hist, h->d_changed, size_t(max_iter + 2) * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                       h->stream);
   if (e != cudaSuccess) return fail(e, "read counters");
   lpa_status st = lpa_rt_take_error(h);  // synchronises
   if (st != LPA_OK) return st;
+  // the graph's step kernel advances the counter itself
+  const uint32_t it_end = packed ? back->it_end : back->it;
   const uint32_t done = it_end - start;
   for (uint32_t i = 0; i < done; i++) h->history.push_back(hist[start + i]);
   h->iterations += done;
-  h->launches += uint64_t(done) * h->launches_per_graph_iteration;
+  h->launches += packed ? 1u : uint64_t(done) * h->launches_per_graph_iteration;
   if (done) h->last_changed = hist[start + done - 1];
   h->cur = int(it_end & 1u);
   if (iters_done) *iters_done = int(done);

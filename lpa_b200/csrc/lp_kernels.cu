@@ -925,6 +925,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_iterate(IterArgs a) {
   flush_changed(c.changed, changed);
 }
 
+enum LabelLoad : int { kLdShared, kLdFenced };  // packed_vertex
+template <int kLoad>
 __device__ __forceinline__ uint32_t packed_vertex(const IterArgs &a, const Ctx &c, uint32_t p, uint32_t *lab);
 
 // Many graphs, one persistent launch.  A ring queue holds (graph,
@@ -1018,7 +1020,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_batch(BatchArgs b) {
       block_segment(ia, c, sh, stage, tab, wstage, wslots, wepoch, s, sg, false, changed);
     } else if (v == kVarPackedLanes) {
       // a tiny segment: one thread per position (<= 256 positions)
-      if (sg.begin + t < sg.end) changed += packed_vertex(ia, c, sg.begin + t, stage + t * kPackedMaxDeg);
+      if (sg.begin + t < sg.end) changed += packed_vertex<kLdShared>(ia, c, sg.begin + t, stage + t * kPackedMaxDeg);
     } else {
       // light segments hold at most 256 positions: the same share for every warp
       const uint32_t per = (sg.end - sg.begin + kWarps - 1) / kWarps, p0 = sg.begin + warp * per;
@@ -1138,11 +1140,15 @@ __device__ __forceinline__ uint32_t packed_mode(const uint32_t (&lab)[kPackedReg
 // lab: this thread's kPackedMaxDeg label slots (shared memory in k_packed,
 // where a lane's slots start kPackedMaxDeg words after the previous lane's:
 // an odd stride, so the 32 lanes' k-th slots fall in 32 different banks).
+template <int kLoad>
 __device__ __forceinline__ uint32_t packed_vertex(const IterArgs &a, const Ctx &c, uint32_t p, uint32_t *lab) {
   const DevGraph &g = a.g;
+  // kLdFenced: the labels change between the caller's grid-wide barriers,
+  // whose fences make plain loads see them (ld.global.nc would not)
+  const auto load = [&](uint32_t i) { return kLoad == kLdFenced ? c.lab_in[i] : ld_label(c, i); };
   const uint32_t node = g.vertices[p];
   const uint32_t d = g.deg[p];
-  const uint32_t old = ld_label(c, node);
+  const uint32_t old = load(node);
   if (d == 0) return 0;
   const bool cgr = p < g.n_c;
   const uint32_t *ids = cgr ? nullptr : g.small_nbr + g.small_off[p - g.n_c];
@@ -1159,7 +1165,7 @@ __device__ __forceinline__ uint32_t packed_vertex(const IterArgs &a, const Ctx &
     }
     if (done) {
 #pragma unroll
-      for (uint32_t u = 0; u < kPackedRegs; u++) r[u] = u < d ? ld_label(c, r[u]) : 0u;
+      for (uint32_t u = 0; u < kPackedRegs; u++) r[u] = u < d ? load(r[u]) : 0u;
       nl = packed_mode(r, d);
     }
   }
@@ -1181,7 +1187,7 @@ __device__ __forceinline__ uint32_t packed_vertex(const IterArgs &a, const Ctx &
 #pragma unroll
     for (uint32_t j = 0; j < kPackedMaxDeg; j++) lv[j] = j < d ? (cgr ? lab[j] : __ldg(ids + j)) : 0u;
 #pragma unroll
-    for (uint32_t j = 0; j < kPackedMaxDeg; j++) lv[j] = j < d ? ld_label(c, lv[j]) : 0u;
+    for (uint32_t j = 0; j < kPackedMaxDeg; j++) lv[j] = j < d ? load(lv[j]) : 0u;
 #pragma unroll
     for (uint32_t j = 0; j < kPackedMaxDeg; j++)
       if (j < d) lab[j] = lv[j];
@@ -1206,7 +1212,7 @@ __global__ void __launch_bounds__(kThreads) k_packed(IterArgs a) {
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.n_packed; i += nw) {
     const long long t0 = clock64();
     const PackedChunk ch = a.packed[i];
-    const uint32_t mine = lane < ch.np ? packed_vertex(a, c, ch.p0 + lane, slab + threadIdx.x * kPackedMaxDeg) : 0u;
+    const uint32_t mine = lane < ch.np ? packed_vertex<kLdShared>(a, c, ch.p0 + lane, slab + threadIdx.x * kPackedMaxDeg) : 0u;
     changed += mine;
     const uint32_t sc = __reduce_add_sync(kFull, mine);
     if (lane == 0) {
@@ -1218,6 +1224,88 @@ __global__ void __launch_bounds__(kThreads) k_packed(IterArgs a) {
   }
   busy_mark(a, 3, true);
   flush_changed(c.changed, changed);
+}
+
+// Waits until every block of the launch has arrived for the k-th time (k from
+// 1).  Bounded: when the others do not arrive, the error word is set and
+// every block gives up.  The launch is cooperative, so all blocks are resident.
+__device__ __forceinline__ bool grid_barrier(PackedLoop *lp, uint32_t k, uint32_t *err) {
+  __shared__ uint32_t s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&lp->arrived, 1u);
+    const volatile uint32_t *seen = &lp->arrived, *gone = &lp->gone;
+    uint32_t tries = 0;
+    bool ok = true;
+    while (*seen < k * gridDim.x) {
+      if (*gone || ++tries > kBarrierTries) {
+        ok = false;
+        break;
+      }
+    }
+    if (!ok) {
+      set_error(err, kErrTimeout);
+      atomicExch(&lp->gone, 1u);
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0u;
+}
+
+// Every iteration of a plan that is all k_packed chunks in one launch: a
+// graph of two kernels per iteration costs about 10 us an iteration beside
+// the work (road grid 64^2),
+// a barrier of the resident blocks 2 to 3 (lpa_run, 20 iterations: 207 -> 120 us;
+// 362^2: 261 -> 195 us).
+// Iterations lp->it .. lp->stop - 1 (lp->early: until nothing changes); the
+// last block's thread leaves the next iteration's number in lp->it.
+__global__ void __launch_bounds__(kThreads) k_packed_loop(IterArgs a, PackedLoop *lp) {
+  __shared__ uint32_t slab[kThreads * kPackedMaxDeg];
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t first = lp->it, stop = lp->stop;
+  const bool early = lp->early != 0u;
+  uint32_t it = first;
+  bool ok = true;
+  while (it < stop) {
+    Ctx c;
+    c.it = it;
+    c.lab_in = (it & 1u) ? a.labs1 : a.labs0;
+    c.lab_out = (it & 1u) ? a.labs0 : a.labs1;
+    c.changed = a.changed + it;
+    c.coherent = false;
+    unsigned long long changed = 0;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.n_packed; i += nw) {
+      const PackedChunk ch = a.packed[i];
+      const uint32_t mine =
+          lane < ch.np ? packed_vertex<kLdFenced>(a, c, ch.p0 + lane, slab + threadIdx.x * kPackedMaxDeg) : 0u;
+      changed += mine;
+      if (a.seg_changed) {
+        const uint32_t sc = __reduce_add_sync(kFull, mine);
+        if (lane == 0 && sc) atomicAdd(a.seg_changed + ch.seg, sc);
+      }
+    }
+    flush_changed(c.changed, changed);
+    it++;
+    if (!grid_barrier(lp, it - first, a.err)) {
+      ok = false;
+      break;
+    }
+    if (early && *reinterpret_cast<volatile unsigned long long *>(c.changed) == 0ull) break;
+  }
+  if (ok && blockIdx.x == 0 && threadIdx.x == 0) lp->it_end = it;
+}
+
+cudaError_t occupancy_packed_loop(int *blocks) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_packed_loop, kThreads, 0);
+}
+
+cudaError_t launch_packed_loop(int grid, cudaStream_t s, IterArgs a, PackedLoop *lp) {
+  void *args[] = {&a, &lp};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_packed_loop), dim3(grid), dim3(kThreads), args, 0, s);
 }
 
 // Two-pass variant, pass 1.  Every 256-bit segment of the two-pass positions

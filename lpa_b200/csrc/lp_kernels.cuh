@@ -269,6 +269,17 @@ cudaError_t prepare_decode_two_pass();
 cudaError_t occupancy_decode_two_pass(int *blocks);
 cudaError_t occupancy_count_two_pass(int *blocks);
 
+// The iterations of a plan that is all k_packed chunks in one cooperative
+// launch: iterations [it, stop), early: until nothing changes.
+struct PackedLoop {
+  uint32_t it, stop, early;
+  uint32_t it_end;         // out: the iteration after the last
+  uint32_t arrived, gone;  // the barrier's arrivals; a block that gave up
+};
+constexpr uint32_t kBarrierTries = 1u << 24;  // polls (of an L2 round trip) before a barrier gives up
+cudaError_t occupancy_packed_loop(int *blocks);
+cudaError_t launch_packed_loop(int grid, cudaStream_t s, IterArgs a, PackedLoop *lp);
+
 struct DecodeArgs {
   DevGraph g;
   const uint32_t *pos_list;  // positions to decode (nullptr: [pos_begin, pos_begin + n_pos))

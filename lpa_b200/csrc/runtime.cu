@@ -120,9 +120,11 @@ void cms_seeds(uint64_t seed, uint32_t out[kCmsDepth]) {
 
 // Reads and clears the device error word.
 lpa_status take_device_error(lpa_handle *h) {
-  uint32_t err = 0;
-  check(h, cudaMemcpyAsync(&err, h->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream), "read error word");
+  // into pinned memory: a pageable target waits for a staging copy
+  uint32_t *back = reinterpret_cast<uint32_t *>(h->h_pinned + kPinnedSlots - 1);
+  check(h, cudaMemcpyAsync(back, h->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream), "read error word");
   check(h, cudaStreamSynchronize(h->stream), "synchronize");
+  const uint32_t err = *back;
   if (err == kErrNone) return LPA_OK;
   check(h, cudaMemsetAsync(h->d_err, 0, sizeof(uint32_t), h->stream), "clear error word");
   switch (err) {
@@ -1130,7 +1132,7 @@ lpa_status lpa_create(const lpa_graph_desc *g, const lpa_opts *o, lpa_handle **o
           "clear counters");
     h->d_err = dalloc<uint32_t>(h, 1, "error word");
     check(h, cudaMemsetAsync(h->d_err, 0, sizeof(uint32_t), h->stream), "clear error word");
-    check(h, cudaMallocHost(&h->h_pinned, sizeof(unsigned long long) * 64), "pinned readback");
+    check(h, cudaMallocHost(&h->h_pinned, sizeof(unsigned long long) * kPinnedSlots), "pinned readback");
     for (auto &e : h->ev) check(h, cudaEventCreate(&e), "events");
     h->events_ready = true;
 
@@ -1609,6 +1611,28 @@ lpa_status lpa_get_segments(lpa_handle *h, uint32_t *begin, uint32_t *end, uint8
 // Internal hooks used by the dispatch and graph-loop modules.
 void lpa_rt_enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32_t *work) {
   enqueue_iteration(h, changed, work);
+}
+// The blocks of the packed loop for the current plan, 0 when the plan has
+// other work (or a batch's tracker runs after every iteration).
+int lpa_rt_packed_loop_grid(lpa_handle *h) {
+  if (h->streamed || h->d_gtrack || !h->n_packed || h->n_groups || h->n_cblock + h->n_cwarp || h->n_heavy + h->n_light)
+    return 0;
+  if (h->occ_packed_loop < 0) {
+    int coop = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device) != cudaSuccess || !coop ||
+        occupancy_packed_loop(&h->occ_packed_loop) != cudaSuccess) {
+      cudaGetLastError();
+      h->occ_packed_loop = 0;
+    }
+  }
+  return int(std::min<uint64_t>((uint64_t(h->n_packed) + kWarps - 1) / kWarps,
+                                uint64_t(h->num_sms) * h->occ_packed_loop));
+}
+cudaError_t lpa_rt_launch_packed_loop(lpa_handle *h) {
+  IterArgs a = iter_args(h, h->d_changed, h->d_work);
+  a.ktime = nullptr;
+  a.seg_cycles = nullptr;
+  return launch_packed_loop(lpa_rt_packed_loop_grid(h), h->stream, a, reinterpret_cast<PackedLoop *>(h->d_loop_it));
 }
 void lpa_rt_apply_variants(lpa_handle *h) {
   apply_run_variants(h);

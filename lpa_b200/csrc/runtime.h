@@ -178,7 +178,8 @@ struct lpa_handle {
 
   // CUDA-graph loop: while set, kernels take their parity and counter slot from it
   const uint32_t *loop_it = nullptr;
-  uint32_t *d_loop_it = nullptr;
+  uint32_t *d_loop_it = nullptr;  // a lpa_dev::PackedLoop; the graph's step kernel uses its first three words
+  int occ_packed_loop = -1;       // resident blocks per SM of k_packed_loop (-1: not asked yet)
   void *graph_exec = nullptr;  // cudaGraphExec_t of the early-exit loop
   void *graph = nullptr;       // cudaGraph_t
   uint64_t launches_per_graph_iteration = 0;
@@ -210,4 +211,7 @@ void lpa_rt_enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
 // (2 launches).
 void lpa_rt_enqueue_track(lpa_handle *h);
 void lpa_rt_apply_variants(lpa_handle *h);
+constexpr int kPinnedSlots = 128;  // 64-bit words of lpa_handle::h_pinned
+int lpa_rt_packed_loop_grid(lpa_handle *h);
+cudaError_t lpa_rt_launch_packed_loop(lpa_handle *h);
 lpa_status lpa_rt_take_error(lpa_handle *h);
