@@ -12,7 +12,8 @@
 //      yardstick every learned plan must beat;
 //   2. kExplore iterations on round-robin plans (segment s runs its
 //      ((s + k) mod capable)-th capable variant) -- every step trains the MLP;
-//   3. the MLP's plan runs, then (when it differs) the same plan with every
+//   3. the MLP's plan (the cheapest variant, the two-pass kernels where they
+//      are close) runs, then (when it differs) the same plan with every
 //      capable segment moved to the two-pass kernels -- per-segment costs do
 //      not see a kernel's critical path or launch; the faster of the two is
 //      the learned plan.  If it is slower than the fixed plan, the handle
@@ -43,6 +44,12 @@ constexpr int kRecheck = 64;
 constexpr int kTrainSteps = 64;   // Adam steps after each measured iteration
 constexpr uint32_t kBatch = 4096;  // minibatch (sampled segments)
 constexpr float kLr = 3e-3f;
+// A segment goes to another variant than the two-pass kernels where that is
+// predicted cheaper by more than this (log2 cost / 32: 1.6 times the cost).
+// Per-segment costs do not see what running one more kernel takes: on a road
+// grid joined with R-MAT scale 18 the plain argmin left the R-MAT graph's large
+// segments, a few percent apart, on k_iterate, 268 us per iteration against 204.
+constexpr float kTwoPassMargin = 0.02f;
 
 __device__ __forceinline__ uint32_t mix32(uint32_t x) {
   x ^= x >> 16;
@@ -149,6 +156,8 @@ __global__ void k_mlp_infer(const float *__restrict__ P, const float *__restrict
       int best = -1;
       for (int o = 0; o < kOut; o++)
         if (((cap[s] >> o) & 1) && (best < 0 || y[o] < y[best])) best = o;
+      if (((cap[s] >> LPA_VARIANT_TWO_PASS) & 1) && y[LPA_VARIANT_TWO_PASS] <= y[best] + kTwoPassMargin)
+        best = LPA_VARIANT_TWO_PASS;
       var_out[s] = uint8_t(best < 0 ? LPA_VARIANT_BLOCK : best);
     }
   }

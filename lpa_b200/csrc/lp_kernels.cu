@@ -1308,6 +1308,118 @@ cudaError_t launch_packed_loop(int grid, cudaStream_t s, IterArgs a, PackedLoop 
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_packed_loop), dim3(grid), dim3(kThreads), args, 0, s);
 }
 
+// The pre-pass over the record groups: a lane per record.  Each lane decodes
+// its segment's ids into the warp's staging window (its lane in the top bits,
+// or in the owner byte beside it), then the warp gathers the window's labels
+// with 8 loads per lane in flight and stores them, consecutive ids of a segment
+// to consecutive addresses.
+template <int kGather, bool kPack>
+__device__ __forceinline__ void decode_records(const IterArgs &a, const Ctx &c, uint32_t *wst, uint8_t *wown,
+                                               uint64_t keep_pol) {
+  const DevGraph &g = a.g;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t hot = uint32_t(min(g.n, uint64_t(kHotIds)));
+  const uint32_t nmax = uint32_t(g.n - 1);
+  uint32_t *ctr = a.work + kWorkCounters * (a.it_dev ? c.it : 0u) + kWqRecs;
+  const auto claim = [&]() {
+    uint32_t x = 0;
+    if (lane == 0) x = atomicAdd(ctr, 1u);
+    return __shfl_sync(kFull, x, 0);
+  };
+  // the next claim is made before a group runs where every warp gets several,
+  // else after it, so that no warp holds a group another could run
+  const bool eager = a.n_rgroups > 4u * gridDim.x * kWarps;
+  for (uint32_t gi = claim(), x = 0; gi < a.n_rgroups; gi = eager ? __shfl_sync(kFull, x, 0) : claim()) {
+    const long long t0 = clock64();
+    const RecGroup rg = a.rgroups[gi];
+    if (eager && lane == 0) x = atomicAdd(ctr, 1u);
+    bool bad = false;
+    uint32_t cnt = 0, node = 0;
+    uint64_t index = 0;
+    BitReader r;
+    if (lane < rg.n) {
+      const uint4 rec = __ldcs(reinterpret_cast<const uint4 *>(a.recs) + rg.rec0 + lane);
+      index = uint64_t((rec.y >> 12) & 0xFFu) << 32 | rec.z;
+      cnt = (rec.y >> 20) & 0xFFu;
+      node = rec.w;
+      r.seek(g.words, uint64_t(rec.y & 0xFFFu) << 32 | rec.x);
+      if (cnt == kSegCountMax) cnt = r.gamma(bad);
+    }
+    const uint32_t incl = warp_incl_scan(cnt, lane);
+    const uint32_t excl = incl - cnt;
+    const uint32_t tot = __shfl_sync(kFull, incl, 31);
+    // window item f of lane l goes to sc[drel_l + f] (32-bit arithmetic) when
+    // every lane's items lie within 2^31 of lane 0's first
+    const uint64_t i0 = (uint64_t(__shfl_sync(kFull, uint32_t(index >> 32), 0)) << 32) |
+                        __shfl_sync(kFull, uint32_t(index), 0);
+    uint32_t *sb = i0 >= a.hub_arcs ? a.scratch_rest : a.scratch;  // a plan segment is all hub or none
+    uint32_t *sc = sb + i0;
+    const int64_t away = int64_t(index - i0);
+    const bool rel32 = __all_sync(kFull, cnt == 0u || (away > -(1ll << 30) && away < (1ll << 30))) && tot < 1u << 30;
+    const int32_t drel = int32_t(away) - int32_t(excl);
+    uint32_t done = 0, v = 0;
+    for (uint32_t w0 = 0; w0 < tot; w0 += kDecodeWindow) {
+      const uint32_t w1 = min(w0 + kDecodeWindow, tot);
+      const uint32_t lim = excl + done < w1 ? min(cnt, w1 - excl) : done;
+      uint32_t *dst = wst + (int32_t(excl) - int32_t(w0));
+      const auto put = [&](uint32_t k, uint32_t id) {
+        if constexpr (kPack) {
+          dst[k] = (id & 0x07FFFFFFu) | (lane << 27);
+        } else {
+          dst[k] = id;
+          wown[int32_t(excl) - int32_t(w0) + int32_t(k)] = uint8_t(lane);
+        }
+      };
+      if (done == 0 && lim > 0) {
+        v = zigzag_first(node, r.zeta3(bad));
+        put(0, v);
+        done = 1;
+      }
+      for (; done < lim; done++) {
+        v += r.zeta3(bad) + 1u;
+        put(done, v);
+      }
+      if (done) bad |= v > nmax;  // ids ascend: the last one is the largest
+      __syncwarp();
+      for (uint32_t f0 = w0; f0 < w1; f0 += 256) {
+        uint32_t lv[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const uint32_t f = f0 + 32u * u + lane;
+          const uint32_t id = f < w1 ? min(kPack ? wst[f - w0] & 0x07FFFFFFu : wst[f - w0], nmax) : 0u;
+          lv[u] = f >= w1 ? 0u
+                  : (kGather == 2 || (kGather == 0 && id < hot)) ? __ldg(c.lab_in + id)
+                                                                  : ld_cg_keep(c.lab_in + id, keep_pol);
+        }
+        if (rel32) {
+#pragma unroll
+          for (int u = 0; u < 8; u++) {
+            const uint32_t f = f0 + 32u * u + lane;
+            const uint32_t ol = f < w1 ? (kPack ? wst[f - w0] >> 27 : wown[f - w0]) : 0u;
+            const int32_t rel = __shfl_sync(kFull, drel, ol) + int32_t(f);
+            if (f < w1) __stcs(sc + rel, lv[u]);
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < 8; u++) {
+            const uint32_t f = f0 + 32u * u + lane;
+            const uint32_t ol = f < w1 ? (kPack ? wst[f - w0] >> 27 : wown[f - w0]) : 0u;
+            const uint64_t ob = (uint64_t(__shfl_sync(kFull, uint32_t(index >> 32), ol)) << 32) |
+                                __shfl_sync(kFull, uint32_t(index), ol);
+            const uint32_t ox = __shfl_sync(kFull, excl, ol);
+            if (f < w1) __stcs(sb + ob + (f - ox), lv[u]);
+          }
+        }
+      }
+      __syncwarp();
+    }
+    if (__any_sync(kFull, bad) && lane == 0) set_error(a.err, kErrBadStream);
+    if (a.seg_cycles && lane == 0)
+      atomicAdd(reinterpret_cast<unsigned long long *>(a.seg_cycles + rg.seg),
+                (unsigned long long)((clock64() - t0) * a.cw_decode));
+  }
+}
+
 // Two-pass variant, pass 1.  Every 256-bit segment of the two-pass positions
 // is decoded by one lane, which writes the labels of its ids (not the ids) to
 // the scratch, so pass 2 only counts.  A warp takes one decode group (32
@@ -1451,6 +1563,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_decode_two_pass(IterArgs a) {
     const uint32_t pk = gd.p0 + lane;
     uint4 ix = make_uint4(0u, 0u, 0u, 0u);
     if (pk < g.n_c) ix = a.pidx[pk];
+    if (a.rgroups) ix.w = 0u;  // the residual segments have records
     uint32_t ns = ix.z + ix.w;
     if (lane == 0) ns = ns > gd.j0 ? ns - gd.j0 : 0u;
     const uint32_t incl = warp_incl_scan(ns, lane);
@@ -1644,7 +1757,15 @@ __global__ void __launch_bounds__(kThreads, 4) k_decode_two_pass(IterArgs a) {
             const uint32_t lo_l = __shfl_sync(kFull, lo, l), len_l = __shfl_sync(kFull, len, l);
             const uint64_t d_l = (uint64_t(__shfl_sync(kFull, uint32_t(dst >> 32), l)) << 32) |
                                  __shfl_sync(kFull, uint32_t(dst), l);
-            for (uint32_t k0 = 0; k0 < len_l; k0 += 128) {
+            uint32_t k1 = 0;
+            for (; k1 + 512 <= len_l; k1 += 512) {  // a long interval: 16 loads in flight
+              uint32_t lv[16];
+#pragma unroll
+              for (int u = 0; u < 16; u++) lv[u] = ld_label(c, lo_l + k1 + 32u * u + lane);
+#pragma unroll
+              for (int u = 0; u < 16; u++) __stcs(a.scratch + d_l + k1 + 32u * u + lane, lv[u]);
+            }
+            for (uint32_t k0 = k1; k0 < len_l; k0 += 128) {
               uint32_t lv[4];
 #pragma unroll
               for (int u = 0; u < 4; u++) {
@@ -1694,6 +1815,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_decode_two_pass(IterArgs a) {
       atomicAdd(reinterpret_cast<unsigned long long *>(a.seg_cycles + gd.seg),
                 (unsigned long long)((clock64() - t0) * a.cw_decode));
   }
+  if (a.rgroups)
+    decode_records<kGather, kPack>(a, c, stage + warp * kDecodeWindow, owner + (kPack ? 0u : warp * kDecodeWindow),
+                                   keep_pol);
   busy_mark(a, 0, true);
 }
 
@@ -2226,6 +2350,61 @@ __global__ void k_pos_index(DevGraph g, uint4 *pidx, uint32_t *err, uint64_t p_l
     } else {
       pidx[p] = make_uint4(uint32_t(ibase - o0), uint32_t(rbase - o0), nsi, nsr);
     }
+  }
+}
+
+__global__ void k_seg_numbers(const uint4 *pidx, const Seg *segs, const uint8_t *use, uint32_t nseg, uint64_t *nsr) {
+  for (uint32_t s = blockIdx.x; s < nseg; s += gridDim.x) {
+    if (!use[s]) continue;
+    for (uint32_t p = segs[s].begin + threadIdx.x; p < segs[s].end; p += blockDim.x) nsr[p] = pidx[p].w;
+  }
+}
+
+// A warp per position, a lane per segment.
+__global__ void k_seg_counts(DevGraph g, const uint4 *pidx, const uint64_t *roff, uint64_t *cnt, uint32_t *err) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t nw = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+  for (uint64_t p = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5; p < g.n_c; p += nw) {
+    const uint64_t r0 = roff[p];
+    const uint32_t ns = uint32_t(roff[p + 1] - r0);
+    for (uint32_t j = lane; j < ns; j += 32) {
+      bool bad = false;
+      BitReader r;
+      r.seek(g.words, g.offsets[p] + pidx[p].y + uint64_t(kSegBits) * j);
+      cnt[r0 + j] = r.gamma(bad);
+      if (bad) set_error(err, kErrBadStream);
+    }
+  }
+}
+
+__global__ void k_seg_records(DevGraph g, const uint4 *pidx, const uint64_t *roff, const uint64_t *csum,
+                              const uint64_t *index, SegRec *recs) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t nw = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+  for (uint64_t p = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5; p < g.n_c; p += nw) {
+    const uint64_t r0 = roff[p], r1 = roff[p + 1];
+    if (r0 == r1) continue;
+    // the intervals' labels first, then the residuals' in stream order
+    const uint64_t at = index[p] + g.deg[p] - (csum[r1] - csum[r0]) - csum[r0];
+    for (uint64_t i = r0 + lane; i < r1; i += 32) {
+      bool bad = false;
+      BitReader r;
+      uint64_t q = g.offsets[p] + pidx[p].y + uint64_t(kSegBits) * (i - r0);
+      r.seek(g.words, q);
+      uint32_t c = r.gamma(bad);
+      if (c < kSegCountMax) q = r.pos();
+      else c = kSegCountMax;
+      const uint64_t o = at + csum[i];
+      recs[i] = SegRec{uint32_t(q), uint32_t(q >> 32) | uint32_t(o >> 32) << 12 | c << 20, uint32_t(o), g.vertices[p]};
+    }
+  }
+}
+
+__global__ void k_seg_ranges(const Seg *segs, uint32_t nseg, const uint64_t *roff, uint32_t *seg_rec) {
+  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x) {
+    const uint64_t r0 = roff[segs[s].begin], r1 = roff[segs[s].end];
+    seg_rec[2 * s] = uint32_t(r0);
+    seg_rec[2 * s + 1] = uint32_t(r1 - r0);
   }
 }
 

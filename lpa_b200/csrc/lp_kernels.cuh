@@ -58,6 +58,29 @@ struct DecodeGroup {
 // the ids' top bits) beat 768 by 1.5 %; 1280 and 1536 shrink L1 and lose 3 %
 // and 13 % (R-MAT scale 24)
 constexpr uint32_t kDecodeWindow = 1024;
+// One residual segment of a resident handle, ready to decode (two-pass plans):
+//   x         low 32 bits of q, the bit after the segment's count
+//   y         q's next 12 bits | index's bits 32..39 << 12 | count << 20
+//   z         low 32 bits of the scratch index of its first label
+//   w         the vertex
+// A count of kSegCountMax or more is stored as kSegCountMax with q at the count
+// itself.  A group's setup without them (finding positions, reserving output,
+// reading counts) was a quarter of the pre-pass's instructions: 588 -> 550 us
+// at R-MAT scale 22, 82 -> 56 us at 18.  Records stay in stream order: sorted by
+// count in windows of 64, 128 or 256, so that the lanes of a group finish
+// together (lane use 66 -> 90 %), the pre-pass took 574, 583 and 588 us, because
+// 32 neighbouring segments share 8 lines and 32 others do not; copying every
+// lane's words to shared memory a group ahead took 852 us.  The index is into
+// the hubs' scratch below IterArgs::hub_arcs, from there into the rest.
+struct SegRec {
+  uint32_t x, y, z, w;
+};
+constexpr uint32_t kSegCountMax = 255;
+constexpr uint64_t kSegMaxBit = 1ull << 44, kSegMaxIndex = 1ull << 40;
+struct RecGroup {
+  uint32_t rec0, n, seg;  // records [rec0, rec0 + n), n <= 32, of one plan segment
+};
+
 // Decode groups a warp of the pre-pass claims from its work queue at once: 4
 // where every resident warp gets several such claims, else 1, so that every
 // warp gets work (a claim's atomic is off the critical path either way).
@@ -129,8 +152,8 @@ constexpr int kBusyKernels = 4;  // kernels of an iteration with a busy span (It
 
 // Work-queue counters of one iteration (IterArgs::work + kWorkCounters *
 // slot): k_iterate's heavy items and light chunks, the count pass's block and
-// warp items, the pre-pass's decode groups; the rest unused.
-enum WorkCounter : int { kWqHeavy = 0, kWqLight, kWqBlock, kWqWarp, kWqGroups, kWorkCounters = 8 };
+// warp items, the pre-pass's decode and record groups; the rest unused.
+enum WorkCounter : int { kWqHeavy = 0, kWqLight, kWqBlock, kWqWarp, kWqGroups, kWqRecs, kWorkCounters = 8 };
 
 struct IterArgs {
   DevGraph g;
@@ -150,6 +173,11 @@ struct IterArgs {
   uint32_t n_groups;
   uint32_t group_claim;         // groups a warp claims at once (group_claim_for)
   uint32_t group_base;          // with one group a claim: the warps' own first groups, else 0
+  const SegRec *recs;           // the residual segments of record groups
+  const RecGroup *rgroups;      // nullptr: the decode groups cover the residual segments too
+  uint32_t n_rgroups;
+  uint32_t *scratch_rest;       // base of scratch indices from hub_arcs on, for recs
+  uint64_t hub_arcs;
   const uint4 *pidx;            // per compressed position: {ibase - offset, rbase - offset, nseg_i, nseg_r}
   const BlockItem *cblock;      // count-pass block items (largest first)
   uint32_t n_cblock;
@@ -300,6 +328,17 @@ __global__ void k_decode_csr(DevGraph g, const uint32_t *pos, const uint64_t *ro
 // segments start (relative to its bit offset) and how many each has.
 // Positions [p_lo, p_hi) (compressed ones only).
 __global__ void k_pos_index(DevGraph g, uint4 *pidx, uint32_t *err, uint64_t p_lo, uint64_t p_hi);
+
+// The segment records (SegRec) of the positions p with nsr[p] != 0 (the
+// numbers of their residual segments; roff: their exclusive sum, n_c + 1):
+// k_seg_counts writes every segment's count to cnt[roff[p] + j],
+// k_seg_records the records, given the counts' exclusive sum csum and every
+// position's scratch index, k_seg_ranges every plan segment's records.
+__global__ void k_seg_numbers(const uint4 *pidx, const Seg *segs, const uint8_t *use, uint32_t nseg, uint64_t *nsr);
+__global__ void k_seg_counts(DevGraph g, const uint4 *pidx, const uint64_t *roff, uint64_t *cnt, uint32_t *err);
+__global__ void k_seg_records(DevGraph g, const uint4 *pidx, const uint64_t *roff, const uint64_t *csum,
+                              const uint64_t *index, SegRec *recs);
+__global__ void k_seg_ranges(const Seg *segs, uint32_t nseg, const uint64_t *roff, uint32_t *seg_rec);
 
 // Degrees (and interval items) of positions [p_lo, p_hi), a thread each;
 // positions of more than kHubBits go to hubs[0..*n_hubs) (room for every

@@ -33,7 +33,7 @@ namespace lpa_dev {
 
 namespace {
 
-enum List : int { kLHeavy = 0, kLLight, kLPacked, kLGroups, kLBlock, kLWarp, kLHash, kLists };
+enum List : int { kLHeavy = 0, kLLight, kLPacked, kLGroups, kLBlock, kLWarp, kLHash, kLRecs, kLists };
 
 struct PlanArgs {
   const SegDev *segs;
@@ -43,6 +43,7 @@ struct PlanArgs {
   const uint32_t *vertices;  // by position
   const uint4 *pidx;         // per compressed position (two-pass plans only)
   const uint64_t *arc_off;   // n_c + 1 (two-pass plans only)
+  const uint32_t *seg_rec;   // per segment {first record, number}, nullptr: no records
   const uint64_t *offsets;   // n_c + 1
   const uint32_t *small_off; // n - n_c + 1
   const uint32_t *words, *small_nbr, *scratch;
@@ -61,6 +62,7 @@ struct PlanArgs {
   WorkItem *light;
   PackedChunk *packed;
   DecodeGroup *groups;
+  RecGroup *rgroups;
   BlockItem *cblock;         // unsorted, with keys
   uint32_t *cblock_key;
   CountItem *cwarp;          // warp items, then group items from n_warp on
@@ -199,7 +201,7 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
       uint32_t positions = 0, lp = p, lj = j;
       while (p < si.end && gd.nlanes < 32 && positions < 32) {
         const uint4 ix = a.pidx[p];
-        const uint32_t ns = ix.z + ix.w;
+        const uint32_t ns = ix.z + (a.seg_rec ? 0u : ix.w);  // residual segments with records: below
         const uint32_t take = min(ns - j, 32u - gd.nlanes);
         gd.nlanes += take;
         positions++;
@@ -226,6 +228,13 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
         c[kLGroups]++;
       }
     }
+  }
+  if (tp && si.region == 0 && a.seg_rec) {
+    const uint32_t r0 = a.seg_rec[2 * s], nr = a.seg_rec[2 * s + 1];
+    c[kLRecs] = (nr + 31) / 32;
+    if (kEmit)
+      for (uint32_t k = 0; k < c[kLRecs]; k++)
+        a.rgroups[o[kLRecs] + k] = RecGroup{r0 + 32 * k, min(32u, nr - 32 * k), s};
   }
   if (!kEmit)
     for (int l = 0; l < kLists; l++) a.cnt[l * stride + i] = c[l];
@@ -376,6 +385,7 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   a.vertices = in.vertices;
   a.pidx = in.pidx;
   a.arc_off = in.arc_off;
+  a.seg_rec = in.seg_rec;
   a.offsets = in.offsets;
   a.small_off = in.small_off;
   a.words = in.words;
@@ -423,6 +433,7 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   out.n_cblock = h_tot[kLBlock];
   out.n_cwarp = h_tot[kLWarp] + h_tot[kLists];
   out.n_hash = h_tot[kLHash];
+  out.n_rgroups = h_tot[kLRecs];
 
   // outputs (the caller's buffers grow to fit) and sort staging
   PB_TRY(out.grow(out), "work lists");
@@ -439,6 +450,7 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   a.light = out.items + out.n_heavy;
   a.packed = out.packed;
   a.groups = out.groups;
+  a.rgroups = out.rgroups;
   a.cwarp = out.cwarp;
   a.n_warp = h_tot[kLWarp];
   if (S) k_plan_emit<<<grid_for(S, in.num_sms), 256, 0, st>>>(a);

@@ -31,6 +31,7 @@ struct PlanInputs {
   const uint32_t *vertices;  // vertex id by position
   const uint4 *pidx;         // position index (two-pass plans), else nullptr
   const uint64_t *arc_off;   // scratch offsets (two-pass plans), else nullptr
+  const uint32_t *seg_rec;   // {first, number} of every segment's records (k_seg_ranges), nullptr: no records
   const uint64_t *offsets;   // bit offsets, n_c + 1
   const uint32_t *small_off; // small CSR offsets, n - n_c + 1
   const uint32_t *words, *small_nbr, *scratch;
@@ -51,10 +52,12 @@ cudaError_t exclusive_sum(uint64_t *data, uint64_t n, void *temp, size_t &temp_b
 // light items; cwarp = warp items followed by group items; cblock largest
 // first.
 struct PlanOutputs {
-  uint32_t n_heavy = 0, n_light = 0, n_packed = 0, n_groups = 0, n_cblock = 0, n_cwarp = 0, n_hash = 0;
+  uint32_t n_heavy = 0, n_light = 0, n_packed = 0, n_groups = 0, n_cblock = 0, n_cwarp = 0, n_hash = 0,
+           n_rgroups = 0;
   WorkItem *items = nullptr;
   PackedChunk *packed = nullptr;
   DecodeGroup *groups = nullptr;
+  RecGroup *rgroups = nullptr;
   BlockItem *cblock = nullptr;
   CountItem *cwarp = nullptr;
   // grow() also makes room for n_hash HashSlots, all zero

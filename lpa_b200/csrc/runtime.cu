@@ -261,6 +261,7 @@ static void upload_lists(lpa_handle *h) {
   in.vertices = h->d_vertices;
   in.pidx = h->d_pidx;
   in.arc_off = h->d_arc_off;
+  in.seg_rec = h->d_seg_rec;
   in.offsets = h->d_offsets;
   in.small_off = h->d_small_off;
   in.words = h->d_words;
@@ -287,12 +288,14 @@ static void upload_lists(lpa_handle *h) {
   out.grow = [&](PlanOutputs &o) -> cudaError_t {
     regrow(h->d_items, h->items_cap, size_t(o.n_heavy) + o.n_light, "work items");
     regrow(h->d_groups, h->groups_cap, o.n_groups, "decode groups");
+    regrow(h->d_rgroups, h->rgroups_cap, o.n_rgroups, "record groups");
     regrow(h->d_citems, h->citems_cap, o.n_cwarp, "count items");
     regrow(h->d_cblock, h->cblock_cap, o.n_cblock, "count block items");
     regrow(h->d_packed, h->packed_cap, o.n_packed, "packed chunks");
     grow_hash_slots(h, o.n_hash);
     o.items = h->d_items;
     o.groups = h->d_groups;
+    o.rgroups = h->d_rgroups;
     o.cwarp = h->d_citems;
     o.cblock = h->d_cblock;
     o.packed = h->d_packed;
@@ -309,11 +312,13 @@ static void upload_lists(lpa_handle *h) {
   h->n_cblock = out.n_cblock;
   h->n_cwarp = out.n_cwarp;
   h->n_hash = out.n_hash;
+  h->n_rgroups = out.n_rgroups;
   h->plan_version++;
   // the resident blocks (the warps take decode groups from a work queue),
   // fewer when there are fewer groups than warps
   h->grid_decode = int(std::max<uint64_t>(
-      1, std::min<uint64_t>((uint64_t(h->n_groups) + kWarps - 1) / kWarps, uint64_t(h->num_sms) * h->occ_decode)));
+      1, std::min<uint64_t>((uint64_t(h->n_groups) + h->n_rgroups + kWarps - 1) / kWarps,
+                            uint64_t(h->num_sms) * h->occ_decode)));
 }
 
 // The work lists of every range of a streamed handle, each built by the
@@ -399,6 +404,25 @@ static void upload_range_lists(lpa_handle *h) {
 // in the compressed region.
 static bool is_hub(const SegInfo &s) { return s.region == 0 && s.bucket == kHeavy; }
 
+// Device memory of one call.
+template <class T>
+struct TempBuf {
+  T *p = nullptr;
+  cudaError_t alloc(uint64_t count) {
+    const cudaError_t e = cudaMalloc(&p, std::max<uint64_t>(count, 1) * sizeof(T));
+    if (e != cudaSuccess) {
+      p = nullptr;
+      cudaGetLastError();
+    }
+    return e;
+  }
+  ~TempBuf() {
+    if (p) cudaFree(p);
+  }
+};
+
+static void build_records(lpa_handle *h, bool full);
+
 // The two-pass kernels' scratch and position index, for the hubs alone (a
 // plan whose block-variant hubs run through them) or for every compressed
 // position.  The hubs' labels have an allocation of their own, so that a
@@ -464,7 +488,10 @@ static void ensure_two_pass_scratch(lpa_handle *h, bool full) {
   h->scratch_scope = full ? 2 : 1;
   h2d(h, h->d_arc_off, dev.data(), h->n_c + 1, "upload arc offsets");
   check(h, cudaStreamSynchronize(h->stream), "arc offsets");
-  if (!first) return;
+  if (!first) {
+    build_records(h, full);
+    return;
+  }
   // where every compressed position's segments start, for the pre-pass
   check(h, cudaMemsetAsync(h->d_cursor, 0, nc * sizeof(uint32_t), h->stream), "clear cursors");
   if (h->streamed) {
@@ -484,6 +511,62 @@ static void ensure_two_pass_scratch(lpa_handle *h, bool full) {
   }
   lpa_status st = take_device_error(h);
   if (st != LPA_OK) throw Fail{st, "position index: " + h->last_error};
+  build_records(h, full);
+}
+
+// The residual segments' records for the positions in the scratch's scope
+// (SegRec).  Without memory for them, or beyond a record's fields, the decode
+// groups cover the residual segments.
+static void build_records(lpa_handle *h, bool full) {
+  dfree(h, h->d_recs);
+  dfree(h, h->d_seg_rec);
+  const uint32_t nseg = uint32_t(h->segs.size());
+  if (h->streamed || h->n_c == 0 || h->total_bits + 1024 >= kSegMaxBit || h->h_arc_off[h->n_c] >= kSegMaxIndex) return;
+  std::vector<uint8_t> use(nseg);
+  for (uint32_t s = 0; s < nseg; s++) use[s] = h->segs[s].region == 0 && (full || is_hub(h->segs[s]));
+  TempBuf<uint8_t> d_use, temp;
+  TempBuf<uint64_t> roff, csum, index;
+  size_t t1 = 0, t2 = 0;
+  const int blocks = h->num_sms * 16;
+  const auto room = [&](cudaError_t e) { return e == cudaSuccess; };  // TempBuf clears the error
+  if (!room(d_use.alloc(nseg)) || !room(roff.alloc(h->n_c + 1)) || !room(index.alloc(h->n_c + 1))) return;
+  check(h, exclusive_sum(roff.p, h->n_c + 1, nullptr, t1, h->stream), "record scan");
+  if (!room(temp.alloc(t1))) return;
+  h2d(h, d_use.p, use.data(), nseg, "upload record scope");
+  h2d(h, index.p, h->h_arc_off.data(), h->n_c + 1, "upload record indices");
+  check(h, cudaMemsetAsync(roff.p, 0, (h->n_c + 1) * sizeof(uint64_t), h->stream), "clear segment numbers");
+  k_seg_numbers<<<blocks, 128, 0, h->stream>>>(h->d_pidx, h->d_segs, d_use.p, nseg, roff.p);
+  check(h, exclusive_sum(roff.p, h->n_c + 1, temp.p, t1, h->stream), "record scan");
+  uint64_t total = 0;
+  check(h, cudaMemcpyAsync(&total, roff.p + h->n_c, sizeof(total), cudaMemcpyDeviceToHost, h->stream), "record total");
+  check(h, cudaStreamSynchronize(h->stream), "record total");
+  if (total + 32 >= 0xFFFFFFFFull || !room(csum.alloc(total + 1))) return;
+  check(h, exclusive_sum(csum.p, total + 1, nullptr, t2, h->stream), "record scan");
+  TempBuf<uint8_t> temp2;
+  if (!room(temp2.alloc(t2))) return;
+  SegRec *recs = nullptr;
+  uint32_t *seg_rec = nullptr;
+  try {
+    recs = dalloc<SegRec>(h, total, "segment records");
+    seg_rec = dalloc<uint32_t>(h, 2 * size_t(nseg), "segment records");
+  } catch (const Fail &) {
+    dfree(h, recs);
+    return;
+  }
+  check(h, cudaMemsetAsync(csum.p + total, 0, sizeof(uint64_t), h->stream), "clear last count");
+  k_seg_counts<<<blocks, 256, 0, h->stream>>>(dev_graph(h), h->d_pidx, roff.p, csum.p, h->d_err);
+  check(h, exclusive_sum(csum.p, total + 1, temp2.p, t2, h->stream), "record scan");
+  k_seg_records<<<blocks, 256, 0, h->stream>>>(dev_graph(h), h->d_pidx, roff.p, csum.p, index.p, recs);
+  uint32_t region0 = 0;  // the compressed region's segments come first
+  while (region0 < nseg && h->segs[region0].region == 0) region0++;
+  if (region0)
+    k_seg_ranges<<<int(std::min<uint32_t>((region0 + 255) / 256, uint32_t(blocks))), 256, 0, h->stream>>>(
+        h->d_segs, region0, roff.p, seg_rec);
+  check(h, cudaGetLastError(), "record launches");
+  lpa_status st = take_device_error(h);
+  if (st != LPA_OK) throw Fail{st, "segment records: " + h->last_error};
+  h->d_recs = recs;
+  h->d_seg_rec = seg_rec;
 }
 
 // What the kernels run for the plan h->variant: the plan, except that the hubs
@@ -708,6 +791,11 @@ static IterArgs iter_args(lpa_handle *h, unsigned long long *changed, uint32_t *
   a.n_light = h->n_light;
   a.groups = h->d_groups;
   a.n_groups = h->n_groups;
+  a.recs = h->d_recs;
+  a.rgroups = h->d_seg_rec ? h->d_rgroups : nullptr;
+  a.n_rgroups = h->n_rgroups;
+  a.scratch_rest = h->d_scratch_rest - h->hub_arcs;
+  a.hub_arcs = h->hub_arcs;
   a.group_claim = group_claim_for(h->n_groups, h->grid_decode);
   a.group_base = a.group_claim == 1 ? uint32_t(h->grid_decode) * kWarps : 0;
   a.cblock = h->d_cblock;
@@ -773,18 +861,18 @@ static void enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
   // branches, so that one's blocks fill the SMs that the last blocks of another
   // leave idle.  The two-pass kernels are one branch; k_iterate joins it when
   // it may count what the pre-pass decoded (heavy items).
-  const bool two = h->n_groups || h->n_cblock + h->n_cwarp;
+  const bool decode = h->n_groups + h->n_rgroups != 0, two = decode || h->n_cblock + h->n_cwarp;
   const bool fork = h->loop_it && int(two) + int(h->n_packed != 0) + int(h->n_heavy + h->n_light != 0) > 1;
   cudaStream_t s_packed = h->stream, s_iter = h->stream;
   if (fork) {
     ensure_side_streams(h);
     cudaEventRecord(h->ev_fork, h->stream);
     if (h->n_packed && (two || h->n_heavy + h->n_light)) s_packed = h->side[0];
-    if (h->n_heavy + h->n_light && two && !(h->n_groups && h->n_heavy)) s_iter = h->side[1];
+    if (h->n_heavy + h->n_light && two && !(decode && h->n_heavy)) s_iter = h->side[1];
     for (cudaStream_t s : {s_packed, s_iter})
       if (s != h->stream) cudaStreamWaitEvent(s, h->ev_fork, 0);
   }
-  if (h->n_groups) {
+  if (decode) {
     launch_decode_two_pass(h->tune.gather_cache, h->tune.stage_stream, h->grid_decode, h->stream, a);
     h->launches++;
     mark(0);
@@ -920,23 +1008,6 @@ static void collect_times(lpa_handle *h) {
   h->iterate_ms = k_ms[3];
   h->last_iter_ms = h->ev_used > 1 ? ms(0, h->ev_used - 1) : 0.0;
 }
-
-// Device memory of one call.
-template <class T>
-struct TempBuf {
-  T *p = nullptr;
-  cudaError_t alloc(uint64_t count) {
-    const cudaError_t e = cudaMalloc(&p, std::max<uint64_t>(count, 1) * sizeof(T));
-    if (e != cudaSuccess) {
-      p = nullptr;
-      cudaGetLastError();
-    }
-    return e;
-  }
-  ~TempBuf() {
-    if (p) cudaFree(p);
-  }
-};
 
 // The CSR by vertex id of a resident handle: rows and lists are put together
 // on the device, in ranges of ids that fit a buffer, and copied straight to the
@@ -1615,7 +1686,7 @@ void lpa_rt_enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
 // The blocks of the packed loop for the current plan, 0 when the plan has
 // other work (or a batch's tracker runs after every iteration).
 int lpa_rt_packed_loop_grid(lpa_handle *h) {
-  if (h->streamed || h->d_gtrack || !h->n_packed || h->n_groups || h->n_cblock + h->n_cwarp || h->n_heavy + h->n_light)
+  if (h->streamed || h->d_gtrack || !h->n_packed || h->n_groups + h->n_rgroups || h->n_cblock + h->n_cwarp || h->n_heavy + h->n_light)
     return 0;
   if (h->occ_packed_loop < 0) {
     int coop = 0;

@@ -139,6 +139,11 @@ struct lpa_handle {
   uint32_t *d_gtab = nullptr;
   uint32_t *d_scratch_rest = nullptr;  // the labels of the positions that are no hubs
   int scratch_scope = 0;               // scratch holds nothing, the hubs' labels, every compressed position's
+  lpa_dev::SegRec *d_recs = nullptr;   // the residual segments of the scope (resident handles)
+  uint32_t *d_seg_rec = nullptr;       // per plan segment {first, number} of them; nullptr: no records
+  lpa_dev::RecGroup *d_rgroups = nullptr;
+  uint32_t n_rgroups = 0;
+  size_t rgroups_cap = 0;
   uint64_t hub_arcs = 0;               // labels in d_scratch (resident handles)
   bool hubs_two_pass = true;           // block-variant hubs run through the two-pass kernels
   uint32_t gtab_slots = 0;
