@@ -68,10 +68,9 @@ struct CgrGraph {
 void cgr_encode(const CsrView &g, const CgrParams &p, int small_thresh, int large_thresh,
                 CgrGraph &out, int threads = 0);
 
-// The same encoding on a GPU (byte-identical output): the per-vertex bit
-// sizing and writing run one thread per compressed vertex on `device`; the
-// position order, offsets prefix sum and small CSR stay on the host.  Only
-// the reference parameters (3, 4, 256, 256).  Throws std::invalid_argument on
+// The same encoding on a GPU (byte-identical output), position order, prefix
+// sums and small CSR included; the bit sizing and writing run one warp per
+// compressed vertex.  Only the reference parameters (3, 4, 256, 256).  Throws std::invalid_argument on
 // unsupported input and std::runtime_error on a CUDA failure.
 void cgr_encode_gpu(const CsrView &g, const CgrParams &p, int small_thresh, int large_thresh, CgrGraph &out,
                     int device = 0);

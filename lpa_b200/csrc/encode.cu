@@ -1,9 +1,10 @@
 // GPU-side CGR encoder, byte-identical to lpa::cgr_encode (cgr_format.cpp),
 // which restates the reference's CgrCompressor (src/compressor.cpp:306-515).
 //
-// The host keeps the cheap O(n) parts (position order, prefix sum of the bit
-// lengths, small CSR); the device does the per-vertex work, one warp per
-// compressed position:
+// Everything runs on the device: the position order (a stable
+// partition by degree class), the prefix sums of the bit lengths and of the small lists (host
+// loops over the vertices took 10 ms at R-MAT scale 20) and the per-vertex
+// work, one warp per compressed position:
 //   pass 1  splits the neighbour list, 32 ids a step, into residuals and
 //           intervals (maximal runs of >= 4 consecutive ids), kept in a work
 //           array in the vertex's own range (residuals from its front,
@@ -27,10 +28,13 @@
 // >= 4, 256-bit segments for both sections) are supported.
 #include <cuda_runtime.h>
 
+#include <cub/device/device_scan.cuh>
+
 #include <algorithm>
 #include <cstdint>
 #include <stdexcept>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "lpa/cgr_format.h"
@@ -357,6 +361,36 @@ __global__ void __launch_bounds__(kEncThreads) k_encode_write(EncodeArgs a, cons
   }
 }
 
+// Position order.  k_class: a vertex's class as a one in the high (degree >=
+// large) or low (>= small) half of x, 0 at n; after x's exclusive sum, whose
+// halves count both classes before a vertex, k_place puts every vertex at its
+// position: large by id, mid by id, small by id.
+__global__ void k_class(const uint64_t *row, uint64_t n, uint64_t large, uint64_t small, uint64_t *x) {
+  for (uint64_t v = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; v <= n; v += uint64_t(gridDim.x) * blockDim.x) {
+    const uint64_t d = v < n ? row[v + 1] - row[v] : 0u;
+    x[v] = v == n ? 0u : d >= large ? 1ull << 32 : d >= small ? 1u : 0u;
+  }
+}
+__global__ void k_place(const uint64_t *row, uint64_t n, uint64_t large, uint64_t small, const uint64_t *x,
+                        uint32_t *vertices) {
+  const uint64_t nl = x[n] >> 32, nm = x[n] & 0xFFFFFFFFull;
+  for (uint64_t v = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; v < n; v += uint64_t(gridDim.x) * blockDim.x) {
+    const uint64_t d = row[v + 1] - row[v], il = x[v] >> 32, im = x[v] & 0xFFFFFFFFull;
+    vertices[d >= large ? il : d >= small ? nl + im : nl + nm + (v - il - im)] = uint32_t(v);
+  }
+}
+
+// Degrees of ns vertices (and a 0 after them), for the scan to list offsets.
+__global__ void k_small_degrees(const uint64_t *row, const uint32_t *vertices_small, uint64_t ns, uint64_t *deg) {
+  for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k <= ns; k += uint64_t(gridDim.x) * blockDim.x)
+    deg[k] = k < ns ? row[vertices_small[k] + 1] - row[vertices_small[k]] : 0u;
+}
+
+__global__ void k_narrow(const uint64_t *in, uint64_t n, uint32_t *out) {
+  for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k < n; k += uint64_t(gridDim.x) * blockDim.x)
+    out[k] = uint32_t(in[k]);
+}
+
 // The small CSR: one warp copies each small vertex's list (lists are
 // contiguous in both arrays, positions n_c.. in order).
 __global__ void k_gather_small(const uint64_t *row, const uint32_t *clm, const uint32_t *vertices_small,
@@ -389,6 +423,30 @@ struct DevBuf {
   DevBuf &operator=(const DevBuf &) = delete;
 };
 
+// v.resize(n) of an empty vector, its pages touched by several threads first:
+// a fresh page costs more than copying into it (45 MB of stream: 16 ms by one
+// thread).
+template <class T>
+void grow(std::vector<T> &v, size_t n) {
+  v.reserve(n);
+  char *p = reinterpret_cast<char *>(v.data());
+  const size_t bytes = n * sizeof(T), page = 4096;
+  const size_t nt = std::min<size_t>({16, std::max(1u, std::thread::hardware_concurrency()), bytes >> 21});
+  if (nt > 1) {
+    std::vector<std::thread> pool;
+    try {
+      for (size_t t = 0; t < nt; t++)
+        pool.emplace_back([=]() {
+          for (size_t i = bytes * t / nt; i < bytes * (t + 1) / nt; i += page)
+            *reinterpret_cast<volatile char *>(p + i) = 0;
+        });
+    } catch (...) {  // no more threads: resize touches what is left
+    }
+    for (auto &th : pool) th.join();
+  }
+  v.resize(n);
+}
+
 }  // namespace
 
 namespace lpa {
@@ -403,98 +461,100 @@ void cgr_encode_gpu(const CsrView &g, const CgrParams &p, int small_thresh, int 
   if (g.n > 0xFFFFFFFFull) throw std::invalid_argument("cgr_encode_gpu: more than 2^32 vertices");
   ck(cudaSetDevice(device), "cudaSetDevice");
   const uint64_t n = g.n, m = n ? g.row[n] : 0;
-  auto deg = [&](uint64_t v) { return g.row[v + 1] - g.row[v]; };
-
-  // position order: large by id, mid by id, small by id (as the host encoder)
   out = CgrGraph();
   out.n = n;
   out.small_thresh = small_thresh;
   out.large_thresh = large_thresh;
-  out.vertices.resize(n);
-  uint64_t nl = 0, nm = 0;
-  for (uint64_t v = 0; v < n; v++) {
-    const uint64_t d = deg(v);
-    if (d >= uint64_t(large_thresh)) nl++;
-    else if (d >= uint64_t(small_thresh)) nm++;
-  }
-  out.n_large = nl;
-  out.n_c = nl + nm;
-  {
-    uint64_t il = 0, im = nl, is = nl + nm;
-    for (uint64_t v = 0; v < n; v++) {
-      const uint64_t d = deg(v);
-      if (d >= uint64_t(large_thresh)) out.vertices[il++] = uint32_t(v);
-      else if (d >= uint64_t(small_thresh)) out.vertices[im++] = uint32_t(v);
-      else out.vertices[is++] = uint32_t(v);
-    }
-  }
-  const uint64_t n_c = out.n_c;
-  out.offsets.assign(n_c + 1, 0);
+  int sms = 148;
+  ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "attribute");
+  const int wide = sms * 8;
 
   // the CSR on the device, once, for both the encoder and the small CSR
   DevBuf<uint64_t> d_row(n + 1);
   DevBuf<uint32_t> d_clm(m);
   ck(cudaMemcpy(d_row.p, g.row, (n + 1) * 8, cudaMemcpyHostToDevice), "upload row");
   if (m) ck(cudaMemcpy(d_clm.p, g.clm, m * 4, cudaMemcpyHostToDevice), "upload clm");
-  int sms = 148;
-  ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "attribute");
-  if (n_c) {
-    DevBuf<uint64_t> d_bits(n_c), d_itv(n_c), d_off(n_c + 1);
-    DevBuf<uint32_t> d_vert(n_c), d_nsi(n_c), d_nsr(n_c), d_nres(n_c), d_nitv(n_c), d_work(m), d_err(1);
-    DevBuf<unsigned long long> d_ctr(2);  // a work counter per pass
-    ck(cudaMemset(d_ctr.p, 0, 16), "clear work counters");
-    ck(cudaMemcpy(d_vert.p, out.vertices.data(), n_c * 4, cudaMemcpyHostToDevice), "upload positions");
-    ck(cudaMemset(d_err.p, 0, 4), "clear error");
-    EncodeArgs ea{d_row.p, d_clm.p, d_vert.p, d_work.p, n_c, out.n_large, d_bits.p, d_itv.p,
-                  d_nsi.p, d_nsr.p, d_nres.p, d_nitv.p, d_ctr.p, d_err.p};
-    const int blocks = int(std::min<uint64_t>((n_c + kEncWarps - 1) / kEncWarps, uint64_t(sms) * 8));
-    k_encode_size<<<blocks, kEncThreads>>>(ea);
-    ck(cudaGetLastError(), "size pass");
-    std::vector<uint64_t> bits(n_c);
-    ck(cudaMemcpy(bits.data(), d_bits.p, n_c * 8, cudaMemcpyDeviceToHost), "read sizes");
-    uint32_t err = 0;
-    ck(cudaMemcpy(&err, d_err.p, 4, cudaMemcpyDeviceToHost), "read error");
-    if (err) throw std::invalid_argument("cgr_encode_gpu: neighbour lists must be strictly ascending");
-    for (uint64_t i = 0; i < n_c; i++) out.offsets[i + 1] = out.offsets[i] + bits[i];
-    out.total_bits = out.offsets[n_c];
-    const uint64_t nwords = (out.total_bits + 31) / 32 + 4;  // 4 zero words of tail, as the host encoder
-    DevBuf<uint32_t> d_words(nwords);
-    ck(cudaMemset(d_words.p, 0, nwords * 4), "clear stream");
-    ck(cudaMemcpy(d_off.p, out.offsets.data(), (n_c + 1) * 8, cudaMemcpyHostToDevice), "upload offsets");
-    ea.ctr = d_ctr.p + 1;
-    k_encode_write<<<blocks, kEncThreads>>>(ea, d_off.p, d_words.p, nwords);
-    ck(cudaGetLastError(), "write pass");
-    ck(cudaMemcpy(&err, d_err.p, 4, cudaMemcpyDeviceToHost), "read error");
-    if (err) throw std::runtime_error("cgr_encode_gpu: a vertex's bits did not end at its offset");
-    out.words.resize(nwords);
-    ck(cudaMemcpy(out.words.data(), d_words.p, nwords * 4, cudaMemcpyDeviceToHost), "read stream");
-  } else {
-    out.total_bits = 0;
-    out.words.assign(4, 0u);
-  }
 
-  // small CSR (src/compressor.cpp:267-282): offsets on the host, the gather
-  // of the lists on the device
-  if (n > n_c) {
-    const uint64_t ns = n - n_c;
-    out.small_offset.resize(ns + 1);
-    out.small_offset[0] = 0;
-    uint64_t acc = 0;
-    for (uint64_t i = n_c; i < n; i++) {
-      acc += deg(out.vertices[i]);
-      if (acc > 0xFFFFFFFFull) throw std::invalid_argument("cgr_encode_gpu: small CSR exceeds 2^32 arcs");
-      out.small_offset[i - n_c + 1] = uint32_t(acc);
-    }
-    out.small_graph.resize(acc);
-    if (acc) {
-      DevBuf<uint32_t> d_vs(ns), d_so(ns + 1), d_sg(acc);
-      ck(cudaMemcpy(d_vs.p, out.vertices.data() + n_c, ns * 4, cudaMemcpyHostToDevice), "upload small positions");
-      ck(cudaMemcpy(d_so.p, out.small_offset.data(), (ns + 1) * 4, cudaMemcpyHostToDevice), "upload small offsets");
-      k_gather_small<<<sms * 8, 256>>>(d_row.p, d_clm.p, d_vs.p, d_so.p, ns, d_sg.p);
-      ck(cudaGetLastError(), "small CSR gather");
-      ck(cudaMemcpy(out.small_graph.data(), d_sg.p, acc * 4, cudaMemcpyDeviceToHost), "read small CSR");
-    }
+  // position order: large by id, mid by id, small by id (as the host encoder)
+  auto scan = [&](uint64_t *data, uint64_t count) {  // exclusive, in place
+    size_t bytes = 0;
+    ck(cub::DeviceScan::ExclusiveSum(nullptr, bytes, data, data, count), "scan");
+    DevBuf<char> temp(bytes);
+    ck(cub::DeviceScan::ExclusiveSum(temp.p, bytes, data, data, count), "scan");
+  };
+  DevBuf<uint32_t> d_vert(n);
+  uint64_t num = 0;
+  {
+    DevBuf<uint64_t> d_class(n + 1);
+    k_class<<<wide, 256>>>(d_row.p, n, uint64_t(large_thresh), uint64_t(small_thresh), d_class.p);
+    ck(cudaGetLastError(), "position order");
+    scan(d_class.p, n + 1);
+    k_place<<<wide, 256>>>(d_row.p, n, uint64_t(large_thresh), uint64_t(small_thresh), d_class.p, d_vert.p);
+    ck(cudaGetLastError(), "position order");
+    ck(cudaMemcpy(&num, d_class.p + n, 8, cudaMemcpyDeviceToHost), "class sizes");
   }
+  out.n_large = num >> 32;
+  const uint64_t n_c = out.n_c = out.n_large + (num & 0xFFFFFFFFull), ns = n - n_c;
+  const uint32_t *d_small = d_vert.p + n_c;
+
+  // d_bits: the bit lengths, then their sums, the offsets
+  DevBuf<uint64_t> d_bits(n_c + 1), d_itv(n_c);
+  DevBuf<uint32_t> d_nsi(n_c), d_nsr(n_c), d_nres(n_c), d_nitv(n_c), d_work(n_c ? m : 0), d_err(1);
+  DevBuf<unsigned long long> d_ctr(2);  // a work counter per pass
+  ck(cudaMemset(d_ctr.p, 0, 16), "clear work counters");
+  ck(cudaMemset(d_err.p, 0, 4), "clear error");
+  EncodeArgs ea{d_row.p, d_clm.p, d_vert.p, d_work.p, n_c, out.n_large, d_bits.p, d_itv.p,
+                d_nsi.p, d_nsr.p, d_nres.p, d_nitv.p, d_ctr.p, d_err.p};
+  const int blocks = int(std::max<uint64_t>(1, std::min<uint64_t>((n_c + kEncWarps - 1) / kEncWarps, uint64_t(wide))));
+  if (n_c) k_encode_size<<<blocks, kEncThreads>>>(ea);
+  ck(cudaGetLastError(), "size pass");
+  grow(out.vertices, n);
+  if (n) ck(cudaMemcpy(out.vertices.data(), d_vert.p, n * 4, cudaMemcpyDeviceToHost), "read positions");
+  uint32_t err = 0;
+  ck(cudaMemcpy(&err, d_err.p, 4, cudaMemcpyDeviceToHost), "read error");
+  if (err) throw std::invalid_argument("cgr_encode_gpu: neighbour lists must be strictly ascending");
+  ck(cudaMemset(d_bits.p + n_c, 0, 8), "clear last size");
+  scan(d_bits.p, n_c + 1);
+  ck(cudaMemcpy(&out.total_bits, d_bits.p + n_c, 8, cudaMemcpyDeviceToHost), "read total");
+  // 4 zero words of tail, as the host encoder
+  const uint64_t nwords = (out.total_bits + 31) / 32 + 4;
+  DevBuf<uint32_t> d_words(nwords);
+  ck(cudaMemset(d_words.p, 0, nwords * 4), "clear stream");
+  ea.ctr = d_ctr.p + 1;
+  if (n_c) k_encode_write<<<blocks, kEncThreads>>>(ea, d_bits.p, d_words.p, nwords);
+  ck(cudaGetLastError(), "write pass");
+
+  // small CSR (src/compressor.cpp:267-282)
+  DevBuf<uint64_t> d_so64(ns + 1);
+  DevBuf<uint32_t> d_so(ns + 1);
+  uint64_t acc = 0;
+  if (ns) {
+    k_small_degrees<<<wide, 256>>>(d_row.p, d_small, ns, d_so64.p);
+    ck(cudaGetLastError(), "small offsets");
+    scan(d_so64.p, ns + 1);
+    k_narrow<<<wide, 256>>>(d_so64.p, ns + 1, d_so.p);
+    ck(cudaGetLastError(), "small offsets");
+    // the host's pages while the device writes
+    grow(out.words, nwords);
+    grow(out.small_offset, ns + 1);
+    ck(cudaMemcpy(&acc, d_so64.p + ns, 8, cudaMemcpyDeviceToHost), "read small total");
+    if (acc > 0xFFFFFFFFull) throw std::invalid_argument("cgr_encode_gpu: small CSR exceeds 2^32 arcs");
+  } else {
+    grow(out.words, nwords);
+  }
+  DevBuf<uint32_t> d_sg(acc);
+  if (acc) {
+    k_gather_small<<<wide, 256>>>(d_row.p, d_clm.p, d_small, d_so.p, ns, d_sg.p);
+    ck(cudaGetLastError(), "small CSR gather");
+    grow(out.small_graph, acc);
+  }
+  out.offsets.resize(n_c + 1);
+  ck(cudaMemcpy(out.offsets.data(), d_bits.p, (n_c + 1) * 8, cudaMemcpyDeviceToHost), "read offsets");
+  ck(cudaMemcpy(&err, d_err.p, 4, cudaMemcpyDeviceToHost), "read error");
+  if (err) throw std::runtime_error("cgr_encode_gpu: a vertex's bits did not end at its offset");
+  ck(cudaMemcpy(out.words.data(), d_words.p, nwords * 4, cudaMemcpyDeviceToHost), "read stream");
+  if (ns) ck(cudaMemcpy(out.small_offset.data(), d_so.p, (ns + 1) * 4, cudaMemcpyDeviceToHost), "read small offsets");
+  if (acc) ck(cudaMemcpy(out.small_graph.data(), d_sg.p, acc * 4, cudaMemcpyDeviceToHost), "read small CSR");
 }
 
 }  // namespace lpa
