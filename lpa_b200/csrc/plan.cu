@@ -94,6 +94,11 @@ __device__ WorkItem make_item(const PlanArgs &a, uint32_t s, uint32_t p0, uint32
   return WorkItem{s, uint32_t(bytes < 0x7FFFFFFFull ? bytes : 0x7FFFFFFFull), addr, p0, p1 - p0};
 }
 
+// A segment's offset in list l, from the sums over all lists one after another.
+__device__ __forceinline__ uint32_t list_off(const uint32_t *off, uint32_t l, uint32_t stride, uint32_t i) {
+  return off[size_t(l) * stride + i] - off[size_t(l) * stride];
+}
+
 // One segment's items.  kEmit false: counts them (and marks the positions
 // its group items will take); true: writes them at the scanned offsets.
 template <bool kEmit>
@@ -118,7 +123,7 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
   const uint32_t stride = a.nseg + 1;
   uint32_t c[kLists] = {}, o[kLists] = {};
   if (kEmit)
-    for (int l = 0; l < kLists; l++) o[l] = a.off[l * stride + i];
+    for (int l = 0; l < kLists; l++) o[l] = list_off(a.off, l, stride, i);
   if (counted) {
     uint32_t p = si.begin;
     while (p < si.end) {
@@ -237,7 +242,7 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
         a.rgroups[o[kLRecs] + k] = RecGroup{r0 + 32 * k, min(32u, nr - 32 * k), s};
   }
   if (!kEmit)
-    for (int l = 0; l < kLists; l++) a.cnt[l * stride + i] = c[l];
+    for (int l = 0; l < kLists; l++) a.cnt[size_t(l) * stride + i] = c[l];
 }
 
 __global__ void k_plan_count(PlanArgs a) {
@@ -299,7 +304,7 @@ __global__ void k_window_emit(PlanArgs a, uint64_t nwin) {
 // The list sizes: offset[nseg] of every list, then the group items.
 __global__ void k_plan_totals(const uint32_t *off, uint32_t stride, const uint32_t *win_off, uint64_t nwin,
                               uint32_t *tot) {
-  if (threadIdx.x < kLists) tot[threadIdx.x] = off[threadIdx.x * stride + stride - 1];
+  if (threadIdx.x < kLists) tot[threadIdx.x] = list_off(off, threadIdx.x, stride, stride - 1);
   if (threadIdx.x == kLists) tot[kLists] = win_off[nwin];
 }
 
@@ -362,12 +367,30 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   const uint64_t G = std::max<uint32_t>(1, in.group_positions);
   const uint64_t win0 = (in.c_end - in.c_begin + G - 1) / G, win1 = (in.s_end - in.s_begin + G - 1) / G;
   const uint64_t nwin = win0 + win1;
-  PB_TRY(reserve(reinterpret_cast<void **>(&cnt), cnt_cap, size_t(kLists) * stride * 4), "plan counts");
-  PB_TRY(reserve(reinterpret_cast<void **>(&off), off_cap, size_t(kLists) * stride * 4), "plan offsets");
-  PB_TRY(reserve(reinterpret_cast<void **>(&gmark), gmark_cap, std::max<uint64_t>(1, in.n) * 4), "group marks");
-  PB_TRY(reserve(reinterpret_cast<void **>(&win), win_cap, (nwin + 1) * 4), "window counts");
-  PB_TRY(reserve(reinterpret_cast<void **>(&win_off), win_off_cap, (nwin + 1) * 4), "window offsets");
-  PB_TRY(reserve(reinterpret_cast<void **>(&tot), tot_cap, (kLists + 1) * 4), "plan totals");
+  // one allocation for what the counting needs, one for the sorting
+  size_t need = 0, t = 0;
+  PB_TRY(cub::DeviceScan::ExclusiveSum(nullptr, t, cnt, off, size_t(kLists) * stride, st), "scan size");
+  need = std::max(need, t);
+  PB_TRY(cub::DeviceScan::ExclusiveSum(nullptr, t, win, win_off, nwin + 1, st), "scan size");
+  need = std::max(need, t);
+  const size_t scan_bytes = need;
+  const auto pad = [](size_t x) { return (x + 255) & ~size_t(255); };
+  const size_t per_list = pad(size_t(kLists) * stride * 4), marks = pad(std::max<uint64_t>(1, in.n) * 4),
+               windows = pad((nwin + 1) * 4), totals = pad((kLists + 1) * 4);
+  PB_TRY(reserve(&count_ws, count_ws_cap, 2 * per_list + marks + 2 * windows + totals + scan_bytes), "plan counts");
+  char *ws = static_cast<char *>(count_ws);
+  const auto take = [&ws](size_t bytes) {
+    char *p = ws;
+    ws += bytes;
+    return p;
+  };
+  cnt = reinterpret_cast<uint32_t *>(take(per_list));
+  off = reinterpret_cast<uint32_t *>(take(per_list));
+  gmark = reinterpret_cast<uint32_t *>(take(marks));
+  win = reinterpret_cast<uint32_t *>(take(windows));
+  win_off = reinterpret_cast<uint32_t *>(take(windows));
+  tot = reinterpret_cast<uint32_t *>(take(totals));
+  void *temp = take(scan_bytes);
   PB_TRY(cudaMemsetAsync(cnt, 0, size_t(kLists) * stride * 4, st), "clear counts");
   PB_TRY(cudaMemsetAsync(win, 0, (nwin + 1) * 4, st), "clear windows");
   PB_TRY(cudaMemsetAsync(gmark, 0, std::max<uint64_t>(1, in.n) * 4, st), "clear marks");
@@ -407,19 +430,11 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   PB_TRY(cudaGetLastError(), "plan count launch");
   if (nwin) k_window_count<<<grid_for(nwin, in.num_sms), 256, 0, st>>>(a, nwin);
   PB_TRY(cudaGetLastError(), "window count launch");
-  // exclusive scans (one extra element each: its offset is the total)
-  size_t need = 0, t = 0;
-  PB_TRY(cub::DeviceScan::ExclusiveSum(nullptr, t, cnt, off, stride, st), "scan size");
-  need = std::max(need, t);
-  PB_TRY(cub::DeviceScan::ExclusiveSum(nullptr, t, win, win_off, nwin + 1, st), "scan size");
-  need = std::max(need, t);
-  PB_TRY(reserve(&temp, temp_cap, need), "scan temp");
-  for (int l = 0; l < kLists; l++) {
-    t = temp_cap;
-    PB_TRY(cub::DeviceScan::ExclusiveSum(temp, t, cnt + size_t(l) * stride, off + size_t(l) * stride, stride, st),
-           "scan");
-  }
-  t = temp_cap;
+  // exclusive scans (one extra element each: its offset is the total): every
+  // list's at once, a list's offsets then from its first (list_off)
+  t = scan_bytes;
+  PB_TRY(cub::DeviceScan::ExclusiveSum(temp, t, cnt, off, size_t(kLists) * stride, st), "scan");
+  t = scan_bytes;
   PB_TRY(cub::DeviceScan::ExclusiveSum(temp, t, win, win_off, nwin + 1, st), "window scan");
   k_plan_totals<<<1, 32, 0, st>>>(off, stride, win_off, nwin, tot);
   PB_TRY(cudaGetLastError(), "totals launch");
@@ -438,11 +453,22 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   // outputs (the caller's buffers grow to fit) and sort staging
   PB_TRY(out.grow(out), "work lists");
   const uint32_t nsort = std::max(out.n_heavy, out.n_cblock);
-  PB_TRY(reserve(reinterpret_cast<void **>(&heavy_tmp), heavy_tmp_cap, size_t(out.n_heavy + 1) * sizeof(WorkItem)),
-         "heavy staging");
-  PB_TRY(reserve(reinterpret_cast<void **>(&cblock_tmp), cblock_tmp_cap,
-                 size_t(out.n_cblock + 1) * sizeof(BlockItem)), "block staging");
-  PB_TRY(reserve(reinterpret_cast<void **>(&keys), keys_cap, size_t(nsort + 1) * 4 * 4), "sort keys");
+  size_t sort_bytes = 0;
+  for (const uint32_t count : {out.n_heavy, out.n_cblock}) {
+    if (count == 0) continue;
+    PB_TRY(cub::DeviceRadixSort::SortPairsDescending(nullptr, t, keys, keys, keys, keys, count, 0, 32, st), "sort size");
+    sort_bytes = std::max(sort_bytes, t);
+  }
+  const size_t heavy_bytes = pad(size_t(out.n_heavy + 1) * sizeof(WorkItem)),
+               cblock_bytes = pad(size_t(out.n_cblock + 1) * sizeof(BlockItem)),
+               key_bytes = pad(size_t(nsort + 1) * 3 * 4), idx_bytes = pad(size_t(nsort + 1) * 2 * 4);
+  PB_TRY(reserve(&sort_ws, sort_ws_cap, heavy_bytes + cblock_bytes + key_bytes + idx_bytes + sort_bytes), "sort staging");
+  ws = static_cast<char *>(sort_ws);
+  heavy_tmp = reinterpret_cast<WorkItem *>(take(heavy_bytes));
+  cblock_tmp = reinterpret_cast<BlockItem *>(take(cblock_bytes));
+  keys = reinterpret_cast<uint32_t *>(take(key_bytes));
+  uint32_t *idx_in = reinterpret_cast<uint32_t *>(take(idx_bytes)), *idx_out = idx_in + (nsort + 1);
+  void *sort_temp = take(sort_bytes);
   a.heavy = heavy_tmp;
   a.heavy_key = keys;
   a.cblock = cblock_tmp;
@@ -461,20 +487,11 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   // largest first, ties in segment order (a stable radix sort of the keys
   // with the item indices)
   uint32_t *kout = keys + 2 * (nsort + 1);
-  uint32_t *idx_in = nullptr, *idx_out = nullptr;
-  PB_TRY(reserve(reinterpret_cast<void **>(&idx), idx_cap, size_t(nsort + 1) * 2 * 4), "sort indices");
-  idx_in = idx;
-  idx_out = idx + (nsort + 1);
   auto sort_gather = [&](const uint32_t *k_in, uint32_t count, auto *src, auto *dst) -> cudaError_t {
     if (count == 0) return cudaSuccess;
     k_iota<<<grid_for(count, in.num_sms), 256, 0, st>>>(idx_in, count);
-    size_t sb = 0;
-    cudaError_t e = cub::DeviceRadixSort::SortPairsDescending(nullptr, sb, k_in, kout, idx_in, idx_out, count, 0, 32, st);
-    if (e != cudaSuccess) return e;
-    e = reserve(&temp, temp_cap, sb);
-    if (e != cudaSuccess) return e;
-    sb = temp_cap;
-    e = cub::DeviceRadixSort::SortPairsDescending(temp, sb, k_in, kout, idx_in, idx_out, count, 0, 32, st);
+    size_t sb = sort_bytes;  // of the larger list
+    const cudaError_t e = cub::DeviceRadixSort::SortPairsDescending(sort_temp, sb, k_in, kout, idx_in, idx_out, count, 0, 32, st);
     if (e != cudaSuccess) return e;
     k_gather<<<grid_for(count, in.num_sms), 256, 0, st>>>(src, idx_out, dst, count);
     return cudaGetLastError();

@@ -76,12 +76,11 @@ class PlanBuilder {
   cudaError_t reserve(void **ptr, size_t &cap, size_t bytes);
   std::vector<void *> bufs;
   uint32_t *cnt = nullptr, *off = nullptr, *gmark = nullptr, *win = nullptr, *win_off = nullptr, *tot = nullptr;
-  uint32_t *keys = nullptr, *idx = nullptr;
+  uint32_t *keys = nullptr;
   WorkItem *heavy_tmp = nullptr;
   BlockItem *cblock_tmp = nullptr;
-  void *temp = nullptr;
-  size_t cnt_cap = 0, off_cap = 0, gmark_cap = 0, win_cap = 0, win_off_cap = 0, tot_cap = 0, keys_cap = 0,
-         idx_cap = 0, heavy_tmp_cap = 0, cblock_tmp_cap = 0, temp_cap = 0;
+  void *count_ws = nullptr, *sort_ws = nullptr;  // the arrays above lie in these
+  size_t count_ws_cap = 0, sort_ws_cap = 0;
 };
 
 }  // namespace lpa_dev

@@ -41,18 +41,50 @@ void check(lpa_handle *h, cudaError_t e, const char *where) {
   (void)h;
 }
 
+// Device memory of the handle.  Small arrays are pieces of shared blocks
+// (256-byte aligned): a handle has about 40 arrays, and an allocation and its
+// release cost 0.05 to 0.1 ms each whatever their size.
+constexpr uint64_t kSlabBytes = 4ull << 20, kSlabPiece = 1ull << 20;
+
 template <class T>
 T *dalloc(lpa_handle *h, uint64_t count, const char *what) {
   void *p = nullptr;
-  const uint64_t bytes = std::max<uint64_t>(count, 1) * sizeof(T);
-  cudaError_t e = cudaMalloc(&p, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    throw Fail{LPA_ERR_OOM, std::string("cudaMalloc ") + what + " (" + std::to_string(bytes) + " bytes)"};
+  const uint64_t bytes = std::max<uint64_t>(count, 1) * sizeof(T), padded = (bytes + 255) & ~uint64_t(255);
+  if (padded <= kSlabPiece && h->slab_left < padded) {
+    if (cudaMalloc(&p, kSlabBytes) == cudaSuccess) {
+      h->slabs.push_back(p);
+      h->slab = static_cast<char *>(p);
+      h->slab_left = kSlabBytes;
+    } else {
+      cudaGetLastError();  // no room for a block: an allocation of its own
+    }
   }
-  h->allocations.push_back(p);
+  if (padded <= kSlabPiece && h->slab_left >= padded) {
+    p = h->slab;
+    h->slab += padded;
+    h->slab_left -= padded;
+  } else {
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      throw Fail{LPA_ERR_OOM, std::string("cudaMalloc ") + what + " (" + std::to_string(bytes) + " bytes)"};
+    }
+    h->allocations.push_back(p);
+  }
   h->device_bytes += bytes;
   return static_cast<T *>(p);
+}
+
+// Gives an array back; a piece of a shared block stays with its block until
+// the handle goes.
+template <class T>
+void dfree(lpa_handle *h, T *&p) {
+  const auto it = std::find(h->allocations.begin(), h->allocations.end(), (void *)p);
+  if (it != h->allocations.end()) {
+    h->allocations.erase(it);
+    cudaFree(p);
+  }
+  p = nullptr;
 }
 
 template <class T>
@@ -225,12 +257,16 @@ static void build_segments(lpa_handle *h) {
 // few launches and one copy of the list sizes, not a host loop over n.
 static void upload_range_lists(lpa_handle *h);
 
-template <class T>
-static void dfree(lpa_handle *h, T *&p) {
-  if (!p) return;
-  h->allocations.erase(std::find(h->allocations.begin(), h->allocations.end(), (void *)p));
-  cudaFree(p);
-  p = nullptr;
+// Global exact-count tables, once a plan gives k_iterate heavy items: for its
+// exact vertices above the shared table, one table per block, at most 2 GiB.
+static void ensure_gtab(lpa_handle *h) {
+  if (h->d_gtab || h->n_heavy == 0 || h->max_exact_deg == 0) return;
+  h->gtab_slots = next_pow2_host(2 * uint64_t(h->max_exact_deg));
+  const uint64_t per_block = uint64_t(h->gtab_slots) * 2 * sizeof(uint32_t);
+  h->gtab_blocks = int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(h->grid), (2ull << 30) / per_block)));
+  h->d_gtab = dalloc<uint32_t>(h, uint64_t(h->gtab_blocks) * 2 * h->gtab_slots, "global count tables");
+  h->grid = std::min(h->grid, h->gtab_blocks);
+  check(h, cudaMemsetAsync(h->d_gtab, 0, uint64_t(h->gtab_blocks) * per_block, h->stream), "clear tables");
 }
 
 static void grow_hash_slots(lpa_handle *h, size_t need) {
@@ -276,11 +312,7 @@ static void upload_lists(lpa_handle *h) {
   in.num_sms = h->num_sms;
   auto regrow = [&](auto *&ptr, size_t &cap, size_t need, const char *what) {
     if (need <= cap && ptr) return;
-    if (ptr) {
-      auto it = std::find(h->allocations.begin(), h->allocations.end(), (void *)ptr);
-      if (it != h->allocations.end()) h->allocations.erase(it);
-      cudaFree(ptr);
-    }
+    dfree(h, ptr);
     cap = need + need / 4 + 16;
     ptr = dalloc<std::remove_reference_t<decltype(*ptr)>>(h, cap, what);
   };
@@ -313,6 +345,7 @@ static void upload_lists(lpa_handle *h) {
   h->n_cwarp = out.n_cwarp;
   h->n_hash = out.n_hash;
   h->n_rgroups = out.n_rgroups;
+  ensure_gtab(h);
   h->plan_version++;
   // the resident blocks (the warps take decode groups from a work queue),
   // fewer when there are fewer groups than warps
@@ -326,11 +359,7 @@ static void upload_lists(lpa_handle *h) {
 static void upload_range_lists(lpa_handle *h) {
   auto regrow = [&](auto *&ptr, size_t &cap, size_t need, const char *what) {
     if (need <= cap && ptr) return;
-    if (ptr) {
-      auto it = std::find(h->allocations.begin(), h->allocations.end(), (void *)ptr);
-      if (it != h->allocations.end()) h->allocations.erase(it);
-      cudaFree(ptr);
-    }
+    dfree(h, ptr);
     cap = need + need / 4 + 16;
     ptr = dalloc<std::remove_reference_t<decltype(*ptr)>>(h, cap, what);
   };
@@ -397,6 +426,7 @@ static void upload_range_lists(lpa_handle *h) {
     h->n_cwarp += r.n_cwarp;
     h->n_hash += out.n_hash;
   }
+  ensure_gtab(h);
   h->plan_version++;
 }
 
@@ -524,26 +554,35 @@ static void build_records(lpa_handle *h, bool full) {
   if (h->streamed || h->n_c == 0 || h->total_bits + 1024 >= kSegMaxBit || h->h_arc_off[h->n_c] >= kSegMaxIndex) return;
   std::vector<uint8_t> use(nseg);
   for (uint32_t s = 0; s < nseg; s++) use[s] = h->segs[s].region == 0 && (full || is_hub(h->segs[s]));
-  TempBuf<uint8_t> d_use, temp;
-  TempBuf<uint64_t> roff, csum, index;
+  // working memory, two allocations: {position sums, indices, scope, scan}, {count sums, scan}
+  struct Piece { uint64_t *p = nullptr; } roff, csum, index;
+  TempBuf<uint64_t> w1, w2;
   size_t t1 = 0, t2 = 0;
   const int blocks = h->num_sms * 16;
   const auto room = [&](cudaError_t e) { return e == cudaSuccess; };  // TempBuf clears the error
-  if (!room(d_use.alloc(nseg)) || !room(roff.alloc(h->n_c + 1)) || !room(index.alloc(h->n_c + 1))) return;
-  check(h, exclusive_sum(roff.p, h->n_c + 1, nullptr, t1, h->stream), "record scan");
-  if (!room(temp.alloc(t1))) return;
-  h2d(h, d_use.p, use.data(), nseg, "upload record scope");
+  check(h, exclusive_sum(nullptr, h->n_c + 1, nullptr, t1, h->stream), "record scan");
+  const uint64_t words = h->n_c + 1, use_words = nseg / 8 + 1;
+  if (!room(w1.alloc(2 * words + use_words + 32 + (t1 + 7) / 8 + 32))) return;
+  roff.p = w1.p;
+  index.p = w1.p + words;
+  uint8_t *d_use = reinterpret_cast<uint8_t *>(w1.p + 2 * words);
+  const auto aligned = [](uint64_t *p) {
+    return reinterpret_cast<void *>((reinterpret_cast<uintptr_t>(p) + 255) & ~uintptr_t(255));
+  };
+  void *scan1 = aligned(w1.p + 2 * words + use_words);
+  h2d(h, d_use, use.data(), nseg, "upload record scope");
   h2d(h, index.p, h->h_arc_off.data(), h->n_c + 1, "upload record indices");
   check(h, cudaMemsetAsync(roff.p, 0, (h->n_c + 1) * sizeof(uint64_t), h->stream), "clear segment numbers");
-  k_seg_numbers<<<blocks, 128, 0, h->stream>>>(h->d_pidx, h->d_segs, d_use.p, nseg, roff.p);
-  check(h, exclusive_sum(roff.p, h->n_c + 1, temp.p, t1, h->stream), "record scan");
+  k_seg_numbers<<<blocks, 128, 0, h->stream>>>(h->d_pidx, h->d_segs, d_use, nseg, roff.p);
+  check(h, exclusive_sum(roff.p, h->n_c + 1, scan1, t1, h->stream), "record scan");
   uint64_t total = 0;
   check(h, cudaMemcpyAsync(&total, roff.p + h->n_c, sizeof(total), cudaMemcpyDeviceToHost, h->stream), "record total");
   check(h, cudaStreamSynchronize(h->stream), "record total");
-  if (total + 32 >= 0xFFFFFFFFull || !room(csum.alloc(total + 1))) return;
-  check(h, exclusive_sum(csum.p, total + 1, nullptr, t2, h->stream), "record scan");
-  TempBuf<uint8_t> temp2;
-  if (!room(temp2.alloc(t2))) return;
+  if (total + 32 >= 0xFFFFFFFFull) return;
+  check(h, exclusive_sum(nullptr, total + 1, nullptr, t2, h->stream), "record scan");
+  if (!room(w2.alloc(total + 1 + 32 + (t2 + 7) / 8 + 32))) return;
+  csum.p = w2.p;
+  void *scan2 = aligned(w2.p + total + 1);
   SegRec *recs = nullptr;
   uint32_t *seg_rec = nullptr;
   try {
@@ -555,7 +594,7 @@ static void build_records(lpa_handle *h, bool full) {
   }
   check(h, cudaMemsetAsync(csum.p + total, 0, sizeof(uint64_t), h->stream), "clear last count");
   k_seg_counts<<<blocks, 256, 0, h->stream>>>(dev_graph(h), h->d_pidx, roff.p, csum.p, h->d_err);
-  check(h, exclusive_sum(csum.p, total + 1, temp2.p, t2, h->stream), "record scan");
+  check(h, exclusive_sum(csum.p, total + 1, scan2, t2, h->stream), "record scan");
   k_seg_records<<<blocks, 256, 0, h->stream>>>(dev_graph(h), h->d_pidx, roff.p, csum.p, index.p, recs);
   uint32_t region0 = 0;  // the compressed region's segments come first
   while (region0 < nseg && h->segs[region0].region == 0) region0++;
@@ -753,21 +792,10 @@ static void build_plan(lpa_handle *h) {
   check(h, cudaMemsetAsync(h->d_seg_cycles, 0, std::max<size_t>(1, h->segs.size()) * sizeof(long long), h->stream),
         "clear cycles");
 
-  // global exact-count tables for exact vertices above the shared table
-  uint64_t big = 0;
   for (uint64_t p = 0; p < h->n; p++) {
     const uint32_t d = h->h_deg[p];
-    const bool cms = h->opts.cms_threshold != 0 && d >= h->opts.cms_threshold;
-    if (!cms && d > kBlockMaxSmemDeg) big = std::max<uint64_t>(big, d);
-  }
-  if (big) {
-    h->gtab_slots = next_pow2_host(2 * big);
-    const uint64_t per_block = uint64_t(h->gtab_slots) * 2 * sizeof(uint32_t);
-    // one table per block of the persistent kernel; at most 2 GiB of tables
-    h->gtab_blocks = int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(h->grid), (2ull << 30) / per_block)));
-    h->grid = std::min(h->grid, h->gtab_blocks);
-    h->d_gtab = dalloc<uint32_t>(h, uint64_t(h->gtab_blocks) * 2 * h->gtab_slots, "global count tables");
-    check(h, cudaMemsetAsync(h->d_gtab, 0, uint64_t(h->gtab_blocks) * per_block, h->stream), "clear tables");
+    if (!(h->opts.cms_threshold != 0 && d >= h->opts.cms_threshold) && d > kBlockMaxSmemDeg)
+      h->max_exact_deg = std::max(h->max_exact_deg, d);
   }
   apply_dispatch(h, h->opts.dispatch == LPA_DISPATCH_FORCE ? LPA_DISPATCH_FORCE : LPA_DISPATCH_FIXED,
                  h->opts.force_variant);
@@ -1232,7 +1260,9 @@ lpa_status lpa_destroy(lpa_handle *h) {
   lpa_rt_destroy_graph(h);
   h->plan_builder.release();
   for (void *p : h->allocations) cudaFree(p);
+  for (void *p : h->slabs) cudaFree(p);
   h->allocations.clear();
+  h->slabs.clear();
   if (h->h_pinned) cudaFreeHost(h->h_pinned);
   if (h->copy_stream) cudaStreamSynchronize(h->copy_stream);
   if (h->h_wpinned) cudaFreeHost(h->h_wpinned);
