@@ -7,7 +7,7 @@
 // seeded cm_hash rows (include/cms.cuh:96-132) and take the argmax of the
 // sketch estimate over their neighbour labels, smallest label on ties.
 //
-// k_iterate is a persistent kernel fed by two device work queues:
+// k_iterate and k_light are persistent kernels, each fed by a device work queue:
 //   * heavy items (block variant, and two-pass segments above the warp
 //     limit), taken by a whole block, largest first: 256-bit segments decode in
 //     parallel (one thread each), ids are staged in shared memory, labels are
@@ -676,6 +676,8 @@ __device__ bool warp_decode_batch(const DevGraph &g, uint32_t *stage, bool activ
 }
 
 // Up to 32 consecutive positions [p0, p1) by one warp.
+// kSlots: the slots of the warp's table.
+template <uint32_t kSlots>
 __device__ void light_chunk(const IterArgs &a, const Ctx &c, uint32_t *stage, unsigned long long *slots,
                             uint32_t &epoch, uint32_t seg, uint32_t p0, uint32_t p1, int variant,
                             unsigned long long &changed) {
@@ -763,32 +765,45 @@ __device__ void light_chunk(const IterArgs &a, const Ctx &c, uint32_t *stage, un
       const uint32_t bv = __shfl_sync(kFull, base, j);
       const uint32_t nodev = __shfl_sync(kFull, node, j);
       const uint32_t oldv = __shfl_sync(kFull, old, j);
-      // epoch table: no clearing, running argmax from the returned counts
-      if (++epoch >= kLightEpochs) {
-        for (uint32_t i = lane; i < kWarpSlots; i += 32) slots[i] = 0ull;
-        __syncwarp();
-        epoch = 1;
-      }
-      const EpochTable et{slots, min(next_pow2(2 * dv), kWarpSlots), epoch};  // cap > dv: every label fits
+      // epoch table: no clearing, running argmax from the returned counts.  A
+      // vertex with more labels than slots is counted in 2, 4, ... parts told
+      // apart by the top bits of the slot hash.
       uint64_t bp = 0;
-      const auto ins = [&](uint32_t lab, uint32_t w) {
-        const uint64_t cand = pack_best(et.insert(lab, w), lab);
-        bp = cand > bp ? cand : bp;
-      };
-      // a step of one label extends the current run (fixed plan at R-MAT
-      // scale 24: 13.48 -> 13.21 ms per iteration)
-      WarpRun run;
-      for (uint32_t k0 = 0; k0 < dv; k0 += 32) {
-        const uint32_t k = k0 + lane;
-        const bool ok = k < dv;
-        const uint32_t lab = ok ? stage[bv + k] : kFull;
-        if (run.extend(ok, lab)) continue;
-        if (run.cnt && lane == 0) ins(run.lab, run.cnt);
-        run.restart(ok, lab);
-        const uint32_t w = warp_merge(ok, lab);
-        if (w) ins(lab, w);
+      for (uint32_t lg = dv <= kSlots ? 0u : dv <= 2 * kSlots - kSlots / 4 ? 1u : 2u;; lg += 2) {
+        bool full = false;
+        bp = 0;
+        for (uint32_t part = 0; part < 1u << lg && !full; part++) {
+          if (++epoch >= kLightEpochs) {
+            for (uint32_t i = lane; i < kSlots; i += 32) slots[i] = 0ull;
+            __syncwarp();
+            epoch = 1;
+          }
+          const EpochTable et{slots, min(next_pow2(2 * dv), kSlots), epoch};
+          const auto ins = [&](uint32_t lab, uint32_t w) {
+            const uint32_t n = et.insert(lab, w);
+            full |= n == 0u;
+            const uint64_t cand = pack_best(n, lab);
+            bp = cand > bp ? cand : bp;
+          };
+          // a step of one label extends the current run (fixed plan at R-MAT
+          // scale 24: 13.48 -> 13.21 ms per iteration)
+          WarpRun run;
+          for (uint32_t k0 = 0; k0 < dv; k0 += 32) {
+            const uint32_t k = k0 + lane;
+            bool ok = k < dv;
+            const uint32_t lab = ok ? stage[bv + k] : kFull;
+            if (lg) ok = ok && slot_hash(lab) >> (32u - lg) == part;
+            if (run.extend(ok, lab)) continue;
+            if (run.cnt && lane == 0) ins(run.lab, run.cnt);
+            run.restart(ok, lab);
+            const uint32_t w = warp_merge(ok, lab);
+            if (w) ins(lab, w);
+          }
+          if (run.cnt && lane == 0) ins(run.lab, run.cnt);
+          full = __any_sync(kFull, full);
+        }
+        if (!full) break;
       }
-      if (run.cnt && lane == 0) ins(run.lab, run.cnt);
       const uint32_t bestl = best_label(warp_max_u64(bp));
       __syncwarp();
       if (lane == 0) {
@@ -825,7 +840,7 @@ __device__ void block_segment(const IterArgs &a, const Ctx &c, BlockSh &sh, uint
   }
   if (__syncthreads_and(fits)) {
     const int v = from_scratch ? kVarTwoPass : kVarWarp;
-    for (uint32_t p = sg.begin + warp; p < sg.end; p += kWarps) light_chunk(a, c, wstage, wslots, wepoch, s, p, p + 1, v, changed);
+    for (uint32_t p = sg.begin + warp; p < sg.end; p += kWarps) light_chunk<kWarpSlots>(a, c, wstage, wslots, wepoch, s, p, p + 1, v, changed);
     __syncthreads();  // the block's shared memory is free for the next item
     return;
   }
@@ -848,7 +863,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_iterate(IterArgs a) {
   __shared__ BlockSh sh;
   uint32_t *stage = smem;         // kStage words
   uint32_t *tab = smem + kStage;  // kTableSlots keys + kTableSlots counts (or the sketch)
-  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  const uint32_t t = threadIdx.x, warp = t >> 5;
   for (uint32_t i = t; i < 2 * kTableSlots; i += kThreads) tab[i] = 0u;
   if (t == 0) sh.hepoch = kHeavyEpochFirst;
   __syncthreads();
@@ -892,13 +907,34 @@ __global__ void __launch_bounds__(kThreads, 2) k_iterate(IterArgs a) {
                 (unsigned long long)((clock64() - t0) * kWarps * a.cw_iterate));
   }
 
+  busy_mark(a, 2, true);
+  flush_changed(c.changed, changed);
+}
+
+// The light items of the warp, packed and block variants, a warp each.  A
+// kernel of its own, apart from the heavy items' registers and 12 KB of
+// shared memory per warp: 8 KB here (1024 staged labels, 512 table slots) and
+// three blocks per SM instead of two (light items of the fixed plan: R-MAT scale
+// 20 264 -> 208 us, 22 1135 -> 891 us, 4M-vertex copy model 950 -> 624 us).
+__global__ void __launch_bounds__(kThreads, 3) k_light(IterArgs a) {
+  extern __shared__ __align__(16) unsigned long long lsmem[];
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  unsigned long long *wslots = lsmem + warp * kLightSlots;
+  uint32_t *wstage = reinterpret_cast<uint32_t *>(lsmem + kWarps * kLightSlots) + warp * kWarpStage;
+  for (uint32_t i = lane; i < kLightSlots; i += 32) wslots[i] = 0ull;
+  __syncwarp();
+  const Ctx c = resolve(a);
+  busy_mark(a, 2, false);
+  unsigned long long changed = 0;
+  uint32_t *qctr = a.work + kWorkCounters * (a.it_dev ? c.it : 0u) + kWqLight;
+  uint32_t wepoch = 0;
   // light items, one at a time: a warp's first is its own, the others come
   // from the queue.  It knows its next item while it runs one (claimed a round
   // earlier, its range prefetched into L2).
   const uint32_t own = gridDim.x * kWarps;
   const auto claim = [&]() {
     uint32_t x = 0;
-    if (lane == 0) x = atomicAdd(qctr + 1, 1u);
+    if (lane == 0) x = atomicAdd(qctr, 1u);
     return own + __shfl_sync(kFull, x, 0);
   };
   WorkItem wi{};
@@ -911,18 +947,24 @@ __global__ void __launch_bounds__(kThreads, 2) k_iterate(IterArgs a) {
       if (lane == 0) prefetch_l2(reinterpret_cast<const void *>(wn.pf_addr), wn.pf_bytes);
     }
     uint32_t x = 0;  // the claim after that; not waited for until the item is done
-    if (lane == 0 && ahead < a.n_light) x = atomicAdd(qctr + 1, 1u);
+    if (lane == 0 && ahead < a.n_light) x = atomicAdd(qctr, 1u);
     const long long t0 = clock64();
-    light_chunk(a, c, wstage, wslots, wepoch, wi.seg, wi.p0, wi.p0 + wi.np, a.seg_var[wi.seg], changed);
+    light_chunk<kLightSlots>(a, c, wstage, wslots, wepoch, wi.seg, wi.p0, wi.p0 + wi.np, a.seg_var[wi.seg], changed);
     if (a.seg_cycles && lane == 0)
       atomicAdd(reinterpret_cast<unsigned long long *>(a.seg_cycles + wi.seg),
-                (unsigned long long)((clock64() - t0) * a.cw_iterate));
+                (unsigned long long)((clock64() - t0) * a.cw_light));
     cur = ahead;
     wi = wn;
     ahead = ahead < a.n_light ? own + __shfl_sync(kFull, x, 0) : ahead;
   }
   busy_mark(a, 2, true);
   flush_changed(c.changed, changed);
+}
+
+cudaError_t prepare_light(int *blocks) {
+  cudaError_t e = cudaFuncSetAttribute(k_light, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kLightSmemBytes));
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_light, kThreads, kLightSmemBytes);
+  return e;
 }
 
 enum LabelLoad : int { kLdShared, kLdFenced };  // packed_vertex
@@ -1024,7 +1066,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_batch(BatchArgs b) {
     } else {
       // light segments hold at most 256 positions: the same share for every warp
       const uint32_t per = (sg.end - sg.begin + kWarps - 1) / kWarps, p0 = sg.begin + warp * per;
-      if (p0 < sg.end) light_chunk(ia, c, wstage, wslots, wepoch, s, p0, min(sg.end, p0 + per), v, changed);
+      if (p0 < sg.end) light_chunk<kWarpSlots>(ia, c, wstage, wslots, wepoch, s, p0, min(sg.end, p0 + per), v, changed);
     }
     flush_changed(c.changed, changed);
     __threadfence();

@@ -27,6 +27,9 @@ constexpr uint32_t kV1MaxDeg = kWarpSlots - 1;         // 1023: a warp's table h
 constexpr uint32_t kV2MaxDeg = 32;
 constexpr uint32_t kBlockMaxSmemDeg = kTableSlots / 2; // exact degrees counted in shared memory (<= 4095)
 
+constexpr uint32_t kLightSlots = 512;                  // 64-bit slots per warp of k_light
+constexpr size_t kLightSmemBytes = size_t(kWarps) * (kLightSlots * 8 + kWarpStage * 4);
+
 // dynamic shared memory of the iteration kernel
 constexpr size_t kSmemBytes = size_t(kStage) * 4 + size_t(kTableSlots) * 8;
 
@@ -190,13 +193,13 @@ struct IterArgs {
   uint32_t cw_packed;           // cost weight of a k_packed warp-cycle (as cw_iterate)
   uint32_t *cursor;             // per compressed position: labels written by the pre-pass (pass 2 resets)
   long long *seg_cycles;        // per-segment device cycles (nullptr: off)
-  // weights of one warp-cycle of k_iterate / k_decode_two_pass /
+  // weights of one warp-cycle of k_iterate / k_light / k_decode_two_pass /
   // k_count_two_pass in seg_cycles: 960 / (the kernel's resident warps per
   // SM), so a booked unit is the same share of an SM whichever kernel spent it
-  uint32_t cw_iterate, cw_decode, cw_count;
+  uint32_t cw_iterate, cw_light, cw_decode, cw_count;
   // nullptr, or the busy span of each kernel of the iteration on the GPU's
   // clock (ns): ktime[k] = earliest warp start, ktime[kBusyKernels + k] =
-  // latest warp end, k = 0 k_decode_two_pass, 1 k_count_two_pass, 2 k_iterate,
+  // latest warp end, k = 0 k_decode_two_pass, 1 k_count_two_pass, 2 k_iterate and k_light,
   // 3 k_packed
   unsigned long long *ktime;
   uint32_t *seg_changed;        // per-segment changed counts (nullptr: off)
@@ -272,6 +275,9 @@ __global__ void k_batch(BatchArgs b);
 __global__ void k_batch_init(const BatchGraph *graphs, uint32_t ngraphs);
 
 __global__ void k_iterate(IterArgs a);
+__global__ void k_light(IterArgs a);
+// allows k_light its shared memory; its resident blocks per SM
+cudaError_t prepare_light(int *blocks);
 // kGather: the cache path of the residual label reads (lpa_tune.gather_cache);
 // kStage: the stream staging (lpa_tune.stage_stream); kPack: staged ids carry
 // their lane (n <= 2^27, unstaged forms)

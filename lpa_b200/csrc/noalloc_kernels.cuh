@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_na_count(NoAllocArgs a) {
       p0 = uint32_t(g.n_c + (ch - cchunks) * 32);
       p1 = uint32_t(g.n < uint64_t(p0) + 32ull ? g.n : uint64_t(p0) + 32ull);
     }
-    light_chunk(ia, c, wstage, wslots, wepoch, 0, p0, p1, kVarTwoPass, changed);
+    light_chunk<kWarpSlots>(ia, c, wstage, wslots, wepoch, 0, p0, p1, kVarTwoPass, changed);
   }
   flush_changed(c.changed, changed);
 }

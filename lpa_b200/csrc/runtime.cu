@@ -839,6 +839,7 @@ static IterArgs iter_args(lpa_handle *h, unsigned long long *changed, uint32_t *
   a.cursor = h->d_cursor;
   a.seg_cycles = (h->opts.record_timings >= 2 || h->collect_cycles) ? h->d_seg_cycles : nullptr;
   a.cw_iterate = h->cw_iterate;
+  a.cw_light = h->cw_light;
   a.cw_decode = h->cw_decode;
   a.cw_count = h->cw_count;
   a.ktime = (h->collect_cycles || h->measure_busy || h->learner_spans) ? h->d_ktime : nullptr;
@@ -887,17 +888,17 @@ static void enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
   mark(-1);
   // In the captured iteration the kernels of different vertices are parallel
   // branches, so that one's blocks fill the SMs that the last blocks of another
-  // leave idle.  The two-pass kernels are one branch; k_iterate joins it when
-  // it may count what the pre-pass decoded (heavy items).
+  // leave idle.  The two-pass kernels are one branch, with k_iterate, which may
+  // count what the pre-pass decoded.
   const bool decode = h->n_groups + h->n_rgroups != 0, two = decode || h->n_cblock + h->n_cwarp;
-  const bool fork = h->loop_it && int(two) + int(h->n_packed != 0) + int(h->n_heavy + h->n_light != 0) > 1;
-  cudaStream_t s_packed = h->stream, s_iter = h->stream;
+  const bool fork = h->loop_it && int(two) + int(h->n_packed != 0) + int(h->n_light != 0) > 1;
+  cudaStream_t s_packed = h->stream, s_light = h->stream;
   if (fork) {
     ensure_side_streams(h);
     cudaEventRecord(h->ev_fork, h->stream);
-    if (h->n_packed && (two || h->n_heavy + h->n_light)) s_packed = h->side[0];
-    if (h->n_heavy + h->n_light && two && !(decode && h->n_heavy)) s_iter = h->side[1];
-    for (cudaStream_t s : {s_packed, s_iter})
+    if (h->n_packed) s_packed = h->side[0];
+    if (h->n_light && two) s_light = h->side[1];
+    for (cudaStream_t s : {s_packed, s_light})
       if (s != h->stream) cudaStreamWaitEvent(s, h->ev_fork, 0);
   }
   if (decode) {
@@ -915,13 +916,17 @@ static void enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
     h->launches++;
     mark(2);
   }
-  if (h->n_heavy + h->n_light) {
-    k_iterate<<<h->grid, kThreads, kSmemBytes, s_iter>>>(a);
+  if (h->n_light) {
+    k_light<<<h->grid_light, kThreads, kLightSmemBytes, s_light>>>(a);
     h->launches++;
-    mark(3);
   }
+  if (h->n_heavy) {
+    k_iterate<<<h->grid, kThreads, kSmemBytes, h->stream>>>(a);
+    h->launches++;
+  }
+  if (h->n_heavy + h->n_light) mark(3);
   for (int k = 0; k < 2; k++) {
-    if ((k ? s_iter : s_packed) == h->stream) continue;
+    if ((k ? s_light : s_packed) == h->stream) continue;
     cudaEventRecord(h->ev_join[k], h->side[k]);
     cudaStreamWaitEvent(h->stream, h->ev_join[k], 0);
   }
@@ -996,7 +1001,11 @@ static void enqueue_streamed_iteration(lpa_handle *h, unsigned long long *change
       k_packed<<<h->grid_packed, kThreads, 0, h->stream>>>(a);
       h->launches++;
     }
-    if (r.n_heavy + r.n_light) {
+    if (r.n_light) {
+      k_light<<<h->grid_light, kThreads, kLightSmemBytes, h->stream>>>(a);
+      h->launches++;
+    }
+    if (r.n_heavy) {
       k_iterate<<<h->grid, kThreads, kSmemBytes, h->stream>>>(a);
       h->launches++;
     }
@@ -1175,6 +1184,10 @@ lpa_status lpa_create(const lpa_graph_desc *g, const lpa_opts *o, lpa_handle **o
     // 960 is divisible by every resident warp count these kernels reach (16..64 in steps of 8)
     const auto weight = [](int blocks) { return uint32_t(std::max(1, 960 / (std::max(1, blocks) * kWarps))); };
     h->cw_iterate = weight(h->occ);
+    int occ_light = 1;
+    check(h, prepare_light(&occ_light), "light kernel");
+    h->grid_light = h->num_sms * std::max(1, occ_light);
+    h->cw_light = weight(occ_light);
     h->cw_count = weight(occ_count);
     h->cw_decode = weight(occ_decode);
     int occ_packed = 1;

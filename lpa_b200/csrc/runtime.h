@@ -121,9 +121,10 @@ struct lpa_handle {
   size_t hash_cap = 0;
   size_t citems_cap = 0;
   int grid_count = 0;                        // count-pass kernel
-  uint32_t cw_iterate = 1, cw_decode = 1, cw_count = 1;  // seg_cycles weights (64 / resident warps per SM)
+  uint32_t cw_iterate = 1, cw_light = 1, cw_decode = 1, cw_count = 1;  // seg_cycles weights (64 / resident warps per SM)
   std::vector<uint64_t> h_arc_off;
-  int grid = 0;          // persistent iteration kernel
+  int grid = 0;          // k_iterate
+  int grid_light = 0;    // k_light
   int grid_decode = 0;   // two-pass decode kernel
   int occ = 1;
   int occ_decode = 1;    // resident blocks per SM of the two-pass decode kernel
