@@ -26,6 +26,11 @@
 
 using namespace lpa_dev;
 
+// Queue items of one block: a graph's iteration lasts as long as its longest
+// item, so segments are shorter than a plan's (256 mid or 64 large positions,
+// 16384 arcs): one warp batch of mid positions, two large ones a warp.
+constexpr lpa_rt::SegLimits kQueueSegs = {{256, 64, 16, 1}, 4096};
+
 struct lpa_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -421,7 +426,7 @@ lpa_status lpa_batch_create(const lpa_graph_desc *graphs, size_t num_graphs, con
     uint64_t big = 0;
     ov = 0;
     for (size_t gi = 0; gi < num_graphs; gi++) {
-      auto segs = lpa_rt::make_segments(deg.data() + ov, b->n[gi], b->n_c[gi], b->opts.cms_threshold);
+      auto segs = lpa_rt::make_segments(deg.data() + ov, b->n[gi], b->n_c[gi], b->opts.cms_threshold, kQueueSegs);
       seg_off[gi + 1] = seg_off[gi] + segs.size();
       for (auto &sg : segs) {
         all_segs.push_back(Seg{sg.begin, sg.end});

@@ -23,11 +23,6 @@ namespace {
 
 constexpr int kMaxRunSlots = 1 << 16;
 
-// Segment cutting limits per bucket: positions (light segments hold at most
-// 8 warp chunks of 32) and arcs.
-constexpr uint32_t kSegPositions[kNumBuckets] = {256, 256, 64, 1};
-constexpr uint64_t kSegArcs = 16384;
-
 struct Fail {
   lpa_status st;
   std::string msg;
@@ -210,7 +205,8 @@ int fixed_variant(const SegInfo &s) {
 }  // namespace lpa_rt
 
 // ------------------------------------------------------------------ plan ---
-std::vector<SegInfo> lpa_rt::make_segments(const uint32_t *deg, uint64_t n, uint64_t n_c, uint32_t cms) {
+std::vector<SegInfo> lpa_rt::make_segments(const uint32_t *deg, uint64_t n, uint64_t n_c, uint32_t cms,
+                                          const SegLimits &lim) {
   std::vector<SegInfo> segs;
   auto bucket_of = [&](uint32_t d) -> uint8_t {
     if ((cms != 0 && d >= cms) || d > kV1MaxDeg) return kHeavy;
@@ -233,8 +229,8 @@ std::vector<SegInfo> lpa_rt::make_segments(const uint32_t *deg, uint64_t n, uint
       continue;
     }
     const uint8_t b = bucket_of(d);
-    if (open && (cur.bucket != b || cur.region != region || cur.end - cur.begin >= kSegPositions[b] ||
-                 cur.arcs + d > kSegArcs)) {
+    if (open && (cur.bucket != b || cur.region != region || cur.end - cur.begin >= lim.positions[b] ||
+                 cur.arcs + d > lim.arcs)) {
       close();
     }
     if (!open) {

@@ -41,8 +41,15 @@ inline uint32_t next_pow2_host(uint64_t x) {
 
 bool variant_capable(int variant, const SegInfo &s, uint32_t cms_thr);
 int fixed_variant(const SegInfo &s);
+// Segment cutting limits: positions per bucket, and arcs.
+struct SegLimits {
+  uint32_t positions[kNumBuckets];
+  uint64_t arcs;
+};
+constexpr SegLimits kPlanSegs = {{256, 256, 64, 1}, 16384};
 // Segments of a graph from its degrees by position (runs of one bucket).
-std::vector<SegInfo> make_segments(const uint32_t *deg, uint64_t n, uint64_t n_c, uint32_t cms_thr);
+std::vector<SegInfo> make_segments(const uint32_t *deg, uint64_t n, uint64_t n_c, uint32_t cms_thr,
+                                   const SegLimits &lim = kPlanSegs);
 
 }  // namespace lpa_rt
 
