@@ -33,6 +33,7 @@ void destroy_graph(lpa_handle *h) {
 
 cudaError_t build_graph(lpa_handle *h) {
   destroy_graph(h);
+  lpa_rt_prepare_branches(h);
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaGraphCreate(&g, 0);
   if (e != cudaSuccess) return e;
@@ -113,11 +114,7 @@ lpa_status lpa_run_graph(lpa_handle *h, int max_iter, bool early_exit, int *iter
     if (e != cudaSuccess) return fail(e, "loop counter");
     h->allocations.push_back(h->d_loop_it);
   }
-  const bool packed = lpa_rt_packed_loop_grid(h) > 0;
-  if (!packed && (!h->graph_exec || h->graph_plan_version != h->plan_version)) {
-    e = build_graph(h);
-    if (e != cudaSuccess) return fail(e, "build iteration graph");
-  }
+  bool packed = lpa_rt_packed_loop_grid(h) > 0;
   // pinned: the control sent, the control and (short runs) the counters back
   const uint32_t start = uint32_t(h->cur);
   lpa_dev::PackedLoop *ctl = reinterpret_cast<lpa_dev::PackedLoop *>(h->h_pinned);
@@ -129,8 +126,14 @@ lpa_status lpa_run_graph(lpa_handle *h, int max_iter, bool early_exit, int *iter
   if (e != cudaSuccess) return fail(e, "loop control");
   if (packed) {
     e = lpa_rt_launch_packed_loop(h);
-    if (e != cudaSuccess) return fail(e, "packed loop launch");
-  } else {
+    if (e != cudaSuccess && h->occ_packed_loop != 0) return fail(e, "packed loop launch");
+    packed = e == cudaSuccess;
+  }
+  if (!packed) {
+    if (!h->graph_exec || h->graph_plan_version != h->plan_version) {
+      e = build_graph(h);
+      if (e != cudaSuccess) return fail(e, "build iteration graph");
+    }
     e = cudaMemsetAsync(h->d_work, 0, size_t(lpa_dev::kWorkCounters) * size_t(max_iter + 2) * sizeof(uint32_t),
                         h->stream);
     if (e != cudaSuccess) return fail(e, "clear work counters");

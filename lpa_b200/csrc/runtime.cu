@@ -858,14 +858,6 @@ static IterArgs iter_args(lpa_handle *h, unsigned long long *changed, uint32_t *
 // zero.
 static void enqueue_streamed_iteration(lpa_handle *h, unsigned long long *changed, uint32_t *work);
 
-// The streams and events of the captured iteration's branches.
-static void ensure_side_streams(lpa_handle *h) {
-  if (h->ev_fork) return;
-  for (auto &s : h->side) check(h, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "side stream");
-  for (auto &e : h->ev_join) check(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "events");
-  check(h, cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming), "events");
-}
-
 static void enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32_t *work) {
   if (h->streamed) {
     enqueue_streamed_iteration(h, changed, work);
@@ -887,10 +879,9 @@ static void enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
   // leave idle.  The two-pass kernels are one branch, with k_iterate, which may
   // count what the pre-pass decoded.
   const bool decode = h->n_groups + h->n_rgroups != 0, two = decode || h->n_cblock + h->n_cwarp;
-  const bool fork = h->loop_it && int(two) + int(h->n_packed != 0) + int(h->n_light != 0) > 1;
+  const bool fork = h->loop_it && h->branches && int(two) + int(h->n_packed != 0) + int(h->n_light != 0) > 1;
   cudaStream_t s_packed = h->stream, s_light = h->stream;
   if (fork) {
-    ensure_side_streams(h);
     cudaEventRecord(h->ev_fork, h->stream);
     if (h->n_packed) s_packed = h->side[0];
     if (h->n_light && two) s_light = h->side[1];
@@ -1722,6 +1713,19 @@ lpa_status lpa_get_segments(lpa_handle *h, uint32_t *begin, uint32_t *end, uint8
 void lpa_rt_enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32_t *work) {
   enqueue_iteration(h, changed, work);
 }
+// The streams and events of the captured iteration's branches, made before a
+// capture begins; without them its kernels follow one another.
+void lpa_rt_prepare_branches(lpa_handle *h) {
+  if (h->branches) return;
+  bool ok = true;
+  for (auto &s : h->side)
+    if (!s) ok &= cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaEvent_t *e : {&h->ev_fork, &h->ev_join[0], &h->ev_join[1]})
+    if (!*e) ok &= cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  h->branches = ok;
+}
+
 // The blocks of the packed loop for the current plan, 0 when the plan has
 // other work (or a batch's tracker runs after every iteration).
 int lpa_rt_packed_loop_grid(lpa_handle *h) {
@@ -1742,7 +1746,13 @@ cudaError_t lpa_rt_launch_packed_loop(lpa_handle *h) {
   IterArgs a = iter_args(h, h->d_changed, h->d_work);
   a.ktime = nullptr;
   a.seg_cycles = nullptr;
-  return launch_packed_loop(lpa_rt_packed_loop_grid(h), h->stream, a, reinterpret_cast<PackedLoop *>(h->d_loop_it));
+  const cudaError_t e =
+      launch_packed_loop(lpa_rt_packed_loop_grid(h), h->stream, a, reinterpret_cast<PackedLoop *>(h->d_loop_it));
+  if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs for this process than the device has
+    cudaGetLastError();
+    h->occ_packed_loop = 0;
+  }
+  return e;
 }
 void lpa_rt_apply_variants(lpa_handle *h) {
   apply_run_variants(h);

@@ -144,6 +144,7 @@ struct lpa_handle {
   uint32_t *d_scratch = nullptr;
   cudaStream_t side[2] = {nullptr, nullptr};  // branches of the captured iteration
   cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
+  bool branches = false;  // they exist
   uint32_t *d_gtab = nullptr;
   uint32_t *d_scratch_rest = nullptr;  // the labels of the positions that are no hubs
   int scratch_scope = 0;               // scratch holds nothing, the hubs' labels, every compressed position's
@@ -228,6 +229,7 @@ void lpa_rt_enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
 void lpa_rt_enqueue_track(lpa_handle *h);
 void lpa_rt_apply_variants(lpa_handle *h);
 constexpr int kPinnedSlots = 128;  // 64-bit words of lpa_handle::h_pinned
+void lpa_rt_prepare_branches(lpa_handle *h);
 int lpa_rt_packed_loop_grid(lpa_handle *h);
 cudaError_t lpa_rt_launch_packed_loop(lpa_handle *h);
 lpa_status lpa_rt_take_error(lpa_handle *h);
