@@ -470,22 +470,35 @@ void cgr_encode_gpu(const CsrView &g, const CgrParams &p, int small_thresh, int 
   const int wide = sms * 8;
 
   // the CSR on the device, once, for both the encoder and the small CSR
-  DevBuf<uint64_t> d_row(n + 1);
-  DevBuf<uint32_t> d_clm(m);
+  // few allocations: what n and m size, what n_c sizes, the stream, the small CSR
+  size_t total = 0;
+  const auto piece = [&total](size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) & ~size_t(255);
+    return at;
+  };
+  size_t scan_bytes = 0;  // of the longest scan, over n + 1
+  ck(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, static_cast<uint64_t *>(nullptr), static_cast<uint64_t *>(nullptr),
+                                   n + 1), "scan");
+  const size_t o_row = piece((n + 1) * 8), o_clm = piece(m * 4), o_class = piece((n + 1) * 8), o_vert = piece(n * 4),
+               o_scan = piece(scan_bytes);
+  DevBuf<char> mem_n(total);
+  struct { uint64_t *p; } d_row{reinterpret_cast<uint64_t *>(mem_n.p + o_row)},
+      d_class{reinterpret_cast<uint64_t *>(mem_n.p + o_class)};
+  struct { uint32_t *p; } d_clm{reinterpret_cast<uint32_t *>(mem_n.p + o_clm)},
+      d_vert{reinterpret_cast<uint32_t *>(mem_n.p + o_vert)};
   ck(cudaMemcpy(d_row.p, g.row, (n + 1) * 8, cudaMemcpyHostToDevice), "upload row");
   if (m) ck(cudaMemcpy(d_clm.p, g.clm, m * 4, cudaMemcpyHostToDevice), "upload clm");
 
   // position order: large by id, mid by id, small by id (as the host encoder)
-  auto scan = [&](uint64_t *data, uint64_t count) {  // exclusive, in place
+  auto scan = [&](uint64_t *data, uint64_t count) {  // exclusive, in place; count <= n + 1
     size_t bytes = 0;
     ck(cub::DeviceScan::ExclusiveSum(nullptr, bytes, data, data, count), "scan");
-    DevBuf<char> temp(bytes);
-    ck(cub::DeviceScan::ExclusiveSum(temp.p, bytes, data, data, count), "scan");
+    if (bytes > scan_bytes) throw std::runtime_error("cgr_encode_gpu: scan memory");
+    ck(cub::DeviceScan::ExclusiveSum(mem_n.p + o_scan, bytes, data, data, count), "scan");
   };
-  DevBuf<uint32_t> d_vert(n);
   uint64_t num = 0;
   {
-    DevBuf<uint64_t> d_class(n + 1);
     k_class<<<wide, 256>>>(d_row.p, n, uint64_t(large_thresh), uint64_t(small_thresh), d_class.p);
     ck(cudaGetLastError(), "position order");
     scan(d_class.p, n + 1);
@@ -498,9 +511,18 @@ void cgr_encode_gpu(const CsrView &g, const CgrParams &p, int small_thresh, int 
   const uint32_t *d_small = d_vert.p + n_c;
 
   // d_bits: the bit lengths, then their sums, the offsets
-  DevBuf<uint64_t> d_bits(n_c + 1), d_itv(n_c);
-  DevBuf<uint32_t> d_nsi(n_c), d_nsr(n_c), d_nres(n_c), d_nitv(n_c), d_work(n_c ? m : 0), d_err(1);
-  DevBuf<unsigned long long> d_ctr(2);  // a work counter per pass
+  total = 0;
+  const size_t o_ctr = piece(2 * 8 + 4), o_bits = piece((n_c + 1) * 8), o_itv = piece(n_c * 8), o_nsi = piece(n_c * 4),
+               o_nsr = piece(n_c * 4), o_nres = piece(n_c * 4), o_nitv = piece(n_c * 4), o_work = piece(n_c ? m * 4 : 0),
+               o_so64 = piece((ns + 1) * 8), o_so = piece((ns + 1) * 4);
+  DevBuf<char> mem_c(total);
+  struct { uint64_t *p; } d_bits{reinterpret_cast<uint64_t *>(mem_c.p + o_bits)},
+      d_itv{reinterpret_cast<uint64_t *>(mem_c.p + o_itv)}, d_so64{reinterpret_cast<uint64_t *>(mem_c.p + o_so64)};
+  struct { uint32_t *p; } d_nsi{reinterpret_cast<uint32_t *>(mem_c.p + o_nsi)},
+      d_nsr{reinterpret_cast<uint32_t *>(mem_c.p + o_nsr)}, d_nres{reinterpret_cast<uint32_t *>(mem_c.p + o_nres)},
+      d_nitv{reinterpret_cast<uint32_t *>(mem_c.p + o_nitv)}, d_work{reinterpret_cast<uint32_t *>(mem_c.p + o_work)},
+      d_so{reinterpret_cast<uint32_t *>(mem_c.p + o_so)}, d_err{reinterpret_cast<uint32_t *>(mem_c.p + o_ctr + 16)};
+  struct { unsigned long long *p; } d_ctr{reinterpret_cast<unsigned long long *>(mem_c.p + o_ctr)};  // one per pass
   ck(cudaMemset(d_ctr.p, 0, 16), "clear work counters");
   ck(cudaMemset(d_err.p, 0, 4), "clear error");
   EncodeArgs ea{d_row.p, d_clm.p, d_vert.p, d_work.p, n_c, out.n_large, d_bits.p, d_itv.p,
@@ -525,8 +547,6 @@ void cgr_encode_gpu(const CsrView &g, const CgrParams &p, int small_thresh, int 
   ck(cudaGetLastError(), "write pass");
 
   // small CSR (src/compressor.cpp:267-282)
-  DevBuf<uint64_t> d_so64(ns + 1);
-  DevBuf<uint32_t> d_so(ns + 1);
   uint64_t acc = 0;
   if (ns) {
     k_small_degrees<<<wide, 256>>>(d_row.p, d_small, ns, d_so64.p);

@@ -39,7 +39,7 @@ void check(lpa_handle *h, cudaError_t e, const char *where) {
 // Device memory of the handle.  Small arrays are pieces of shared blocks
 // (256-byte aligned): a handle has about 40 arrays, and an allocation and its
 // release cost 0.05 to 0.1 ms each whatever their size.
-constexpr uint64_t kSlabBytes = 4ull << 20, kSlabPiece = 1ull << 20;
+constexpr uint64_t kSlabBytes = 4ull << 20, kSlabPiece = 2ull << 20;
 
 template <class T>
 T *dalloc(lpa_handle *h, uint64_t count, const char *what) {
@@ -1038,30 +1038,39 @@ static void collect_times(lpa_handle *h) {
 // caller's arrays (a host loop over the vertices took most of 74 ms for a
 // 1M-vertex, 26M-arc graph).
 static lpa_status decode_csr_resident(lpa_handle *h, uint64_t *row_out, uint32_t *clm_out) {
-  constexpr uint64_t kBufArcs = 1ull << 26;
+  constexpr uint64_t kBufArcs = 1ull << 26, kCsrKeep = 8ull << 20;
   const int blocks = h->num_sms * 8;
-  TempBuf<uint32_t> pos, out;
-  TempBuf<uint64_t> row;
-  TempBuf<uint8_t> temp;
+  // rows, positions, scan memory, then the lists: one allocation, which small
+  // graphs keep (an allocation takes longer than their decode)
   size_t temp_bytes = 0;
-  check(h, pos.alloc(h->n), "decode positions");
-  check(h, row.alloc(h->n + 1), "decode rows");
-  check(h, exclusive_sum(row.p, h->n + 1, nullptr, temp_bytes, h->stream), "decode scan");
-  check(h, temp.alloc(temp_bytes), "decode scan");
+  check(h, exclusive_sum(nullptr, h->n + 1, nullptr, temp_bytes, h->stream), "decode scan");
+  const auto pad = [](uint64_t x) { return (x + 255) & ~uint64_t(255); };
+  const uint64_t row_bytes = pad((h->n + 1) * sizeof(uint64_t)), pos_bytes = pad(h->n * sizeof(uint32_t)),
+                 fixed = row_bytes + pos_bytes + pad(temp_bytes);
+  // the lists' buffer: everything at once when that fits, at least the longest list
+  uint64_t cap = std::max<uint64_t>(h->max_deg, std::min<uint64_t>(h->m, kBufArcs));
+  TempBuf<char> mem;
+  char *base = h->d_csr_ws;
+  if (!base && fixed + cap * 4 <= kCsrKeep) {
+    base = h->d_csr_ws = dalloc<char>(h, fixed + cap * 4, "decode");
+  } else if (!base) {
+    while (mem.alloc(fixed + cap * 4) != cudaSuccess) {
+      if (cap <= h->max_deg) throw Fail{LPA_ERR_OOM, "decode buffer"};
+      cap = std::max<uint64_t>(h->max_deg, cap / 4);
+    }
+    base = mem.p;
+  }
+  struct { uint64_t *p; } row{reinterpret_cast<uint64_t *>(base)};
+  struct { uint32_t *p; } pos{reinterpret_cast<uint32_t *>(base + row_bytes)}, out{reinterpret_cast<uint32_t *>(base + fixed)};
+  void *temp = base + row_bytes + pos_bytes;
   check(h, cudaMemsetAsync(pos.p, 0xFF, h->n * sizeof(uint32_t), h->stream), "clear positions");
   k_csr_inverse<<<blocks, 256, 0, h->stream>>>(h->d_vertices, h->n, pos.p);
   k_csr_degrees<<<blocks, 256, 0, h->stream>>>(h->d_deg, pos.p, h->n, row.p);
-  check(h, exclusive_sum(row.p, h->n + 1, temp.p, temp_bytes, h->stream), "decode scan");
+  check(h, exclusive_sum(row.p, h->n + 1, temp, temp_bytes, h->stream), "decode scan");
   check(h, cudaGetLastError(), "decode rows launch");
   check(h, cudaMemcpyAsync(row_out, row.p, (h->n + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream),
         "read rows");
   check(h, cudaStreamSynchronize(h->stream), "read rows");
-  // the buffer: everything at once when that fits, at least the longest list
-  uint64_t cap = std::max<uint64_t>(h->max_deg, std::min<uint64_t>(row_out[h->n], kBufArcs));
-  while (out.alloc(cap) != cudaSuccess) {
-    if (cap <= h->max_deg) throw Fail{LPA_ERR_OOM, "decode buffer"};
-    cap = std::max<uint64_t>(h->max_deg, cap / 4);
-  }
   for (uint64_t v0 = 0; v0 < h->n;) {
     // the ids whose lists fit the buffer, from v0 on
     const uint64_t v1 = uint64_t(std::upper_bound(row_out + v0, row_out + h->n + 1, row_out[v0] + cap) - row_out) - 1;

@@ -174,6 +174,7 @@ struct lpa_handle {
   int ev_used = 0;
   bool events_ready = false;
   uint64_t device_bytes = 0;
+  char *d_csr_ws = nullptr;     // lpa_decode_csr's memory, kept by small handles
   std::vector<void *> allocations, slabs;
   char *slab = nullptr;         // the rest of the last shared block
   uint64_t slab_left = 0;
