@@ -8,15 +8,17 @@
 // sketch estimate over their neighbour labels, smallest label on ties.
 //
 // k_iterate and k_light are persistent kernels, each fed by a device work queue:
-//   * heavy items (block variant, and two-pass segments above the warp
-//     limit), taken by a whole block, largest first: 256-bit segments decode in
-//     parallel (one thread each), ids are staged in shared memory, labels are
-//     gathered with many loads in flight, then counted in a shared (or global)
-//     table or the sketch;
-//   * light items of up to 32 consecutive positions, taken by one warp: each
-//     lane decodes one vertex into the warp's staging area, the warp gathers
-//     all labels at once, then counts per vertex (one vertex per round, or
-//     several vertices per round for degrees <= 32).
+//   * heavy items (hubs the two-pass kernels do not take), one per block,
+//     largest first: 256-bit segments decode in parallel (one thread each), ids
+//     are staged in shared memory, labels are gathered with many loads in
+//     flight, then counted in a shared (or global) table or the sketch;
+//   * light items of up to 32 consecutive positions, one per warp: the lanes
+//     decode the batch's segments into the warp's staging area, the warp
+//     gathers all labels at once, then counts, a lane per vertex of degree
+//     <= 32, the others one after another.
+// The two-pass kernels (k_decode_two_pass, k_count_two_pass) write every
+// neighbour label to a scratch and count from there; k_packed and
+// k_packed_loop take the tiny vertices, a lane each.
 // Every loop is bounded by the bits it consumes; malformed input sets the
 // error word instead of trapping.
 #include <type_traits>

@@ -154,7 +154,7 @@ constexpr uint32_t kPackedMaxDeg = 15;  // the tiny bucket (degree < 16)
 constexpr int kBusyKernels = 4;  // kernels of an iteration with a busy span (IterArgs::ktime)
 
 // Work-queue counters of one iteration (IterArgs::work + kWorkCounters *
-// slot): k_iterate's heavy items and light chunks, the count pass's block and
+// slot): k_iterate's heavy items, k_light's items, the count pass's block and
 // warp items, the pre-pass's decode and record groups; the rest unused.
 enum WorkCounter : int { kWqHeavy = 0, kWqLight, kWqBlock, kWqWarp, kWqGroups, kWqRecs, kWorkCounters = 8 };
 

@@ -108,7 +108,7 @@ struct lpa_handle {
   lpa_dev::SegDev *d_segdev = nullptr;       // the segments as the device list builder reads them
   lpa_dev::PlanBuilder plan_builder;         // its working memory
   uint8_t *d_seg_var = nullptr;
-  lpa_dev::WorkItem *d_items = nullptr;  // heavy items | light chunk items
+  lpa_dev::WorkItem *d_items = nullptr;  // heavy items | light items
   lpa_dev::DecodeGroup *d_groups = nullptr;  // two-pass pre-pass work (32 segments each)
   uint32_t n_heavy = 0, n_light = 0, n_groups = 0;
   size_t items_cap = 0, groups_cap = 0;
