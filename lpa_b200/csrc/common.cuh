@@ -448,10 +448,16 @@ __device__ __forceinline__ uint64_t warp_max_u64(uint64_t v) {
 }
 
 // Open-addressing exact counter in shared (or global) memory.  Keys are
-// stored as label + 1 so that 0 marks an empty slot.  cap is a power of two
-// larger than the number of distinct labels inserted.
-__device__ __forceinline__ bool table_add(uint32_t *keys, uint32_t *cnts, uint32_t cap, uint32_t label,
+// stored as label + 1 so that 0 marks an empty slot; the one label without a
+// key, kTopLabel, is counted in *top.  cap is a power of two larger than the
+// number of distinct labels inserted.
+constexpr uint32_t kTopLabel = 0xFFFFFFFFu;
+__device__ __forceinline__ bool table_add(uint32_t *keys, uint32_t *cnts, uint32_t cap, uint32_t *top, uint32_t label,
                                           uint32_t c) {
+  if (label == kTopLabel) {
+    atomicAdd(top, c);
+    return true;
+  }
   const uint32_t key = label + 1u;
   uint32_t h = slot_hash(label) & (cap - 1);
   for (uint32_t probe = 0; probe < cap; probe++) {

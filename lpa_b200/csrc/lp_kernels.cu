@@ -106,6 +106,7 @@ struct BlockSh {
   uint64_t ibase, rbase, last_end;
   uint32_t nseg_i, nseg_r, item, items, bad;
   uint32_t hepoch;  // epoch of the block's exact table
+  uint32_t top;     // the global table's count of kTopLabel
 };
 
 // Block-wide exclusive scan of v into sh.pref; returns the total.
@@ -152,10 +153,10 @@ struct WarpRun {
 // The exact tables fold lanes holding the same label first (warp_merge), so a
 // step whose lanes share a label touches the table once.
 struct ExactSink {  // global table (key/count arrays, cleared after use)
-  uint32_t *keys, *cnts, cap;
+  uint32_t *keys, *cnts, cap, *top;
   __device__ __forceinline__ void operator()(bool ok, uint32_t lab) const {
     const uint32_t w = warp_merge(ok, lab);
-    if (w) table_add(keys, cnts, cap, lab, w);
+    if (w) table_add(keys, cnts, cap, top, lab, w);
   }
 };
 
@@ -508,8 +509,11 @@ __device__ void heavy_vertex(const IterArgs &a, const Ctx &c, BlockSh &sh, uint3
     }
     uint32_t *keys = a.gtab + uint64_t(blockIdx.x) * 2 * a.gtab_slots;
     uint32_t *cnts = keys + a.gtab_slots;
-    heavy_produce(a, c, sh, stage, p, node, d, from_scratch, ExactSink{keys, cnts, cap});
+    if (t == 0) sh.top = 0;
     __syncthreads();
+    heavy_produce(a, c, sh, stage, p, node, d, from_scratch, ExactSink{keys, cnts, cap, &sh.top});
+    __syncthreads();
+    if (t == 0 && sh.top) best = pack_best(sh.top, kTopLabel);
     for (uint32_t i = t; i < cap; i += kThreads) {
       const uint32_t kk = keys[i];
       if (kk) {
@@ -1978,6 +1982,7 @@ __device__ __forceinline__ void sketch_count(uint32_t *cms, const uint32_t *__re
 // the hash (a bijection of the label: 20 bits leave at most 4096 labels).
 __device__ __noinline__ uint64_t count_share(uint32_t *keys, const uint32_t *src, uint32_t d, uint32_t lg,
                                              uint32_t share) {
+  __shared__ uint32_t top;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint32_t *cnts = keys + kCountBlockSlots;
   uint64_t best = 0;
@@ -1986,7 +1991,9 @@ __device__ __noinline__ uint64_t count_share(uint32_t *keys, const uint32_t *src
     bool full = false;
     for (uint32_t part = 0; part < 1u << more && !full; part++) {
       const uint32_t want = share << more | part, sh = 32u - lg - more;
-      const auto ins = [&](uint32_t lab, uint32_t c) { full |= !table_add(keys, cnts, kCountBlockSlots, lab, c); };
+      if (threadIdx.x == 0) top = 0;
+      __syncthreads();
+      const auto ins = [&](uint32_t lab, uint32_t c) { full |= !table_add(keys, cnts, kCountBlockSlots, &top, lab, c); };
       WarpRun run;
       warp_stream<true, 4>(src, d, warp, kWarps, [&](bool ok, uint32_t lab) {
         ok = ok && slot_hash(lab) >> sh == want;
@@ -2006,6 +2013,10 @@ __device__ __noinline__ uint64_t count_share(uint32_t *keys, const uint32_t *src
           keys[k] = 0u;
           cnts[k] = 0u;
         }
+      }
+      if (threadIdx.x == 0 && top) {
+        const uint64_t cand = pack_best(top, kTopLabel);
+        best = cand > best ? cand : best;
       }
       __syncthreads();
     }
