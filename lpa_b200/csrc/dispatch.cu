@@ -262,11 +262,8 @@ bool learner_setup(lpa_handle *h) {
   return L->ok;
 }
 
-void set_plan(lpa_handle *h, const std::vector<uint8_t> &plan) {
-  if (plan != h->variant) {
-    h->variant = plan;
-    lpa_rt_apply_variants(h);
-  }
+bool set_plan(lpa_handle *h, const std::vector<uint8_t> &plan) {
+  return plan == h->variant || lpa_rt_install_plan(h, plan);
 }
 
 void explore_plan(lpa_handle *h, int k, std::vector<uint8_t> &plan) {
@@ -371,7 +368,13 @@ void lpa_learner_before_iteration(lpa_handle *h) {
     default:
       plan = (L->since_check >= kRecheck) ? L->learned : h->fixed;
   }
-  set_plan(h, plan);
+  if (!set_plan(h, plan)) {  // no memory for the plan: the heuristic stays
+    lpa_learner_free(h);
+    h->opts.dispatch = LPA_DISPATCH_FIXED;
+    set_plan(h, h->fixed);
+    lpa_rt_ensure_lists(h);
+    return;
+  }
   // per-segment cycles only while the model trains on them (every item's
   // booking is an atomic); the iteration is timed by its kernels' busy spans
   // until the plan is chosen, then only on the iteration before a recheck

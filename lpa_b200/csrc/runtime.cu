@@ -36,6 +36,11 @@ void check(lpa_handle *h, cudaError_t e, const char *where) {
   (void)h;
 }
 
+// What the calling thread's next allocations are refused by name
+// (lpa_test_refuse), empty: nothing.
+thread_local std::string refused_name;
+bool refused(const char *what) { return !refused_name.empty() && refused_name == what; }
+
 // Device memory of the handle.  Small arrays are pieces of shared blocks
 // (256-byte aligned): a handle has about 40 arrays, and an allocation and its
 // release cost 0.05 to 0.1 ms each whatever their size.
@@ -45,6 +50,7 @@ template <class T>
 T *dalloc(lpa_handle *h, uint64_t count, const char *what) {
   void *p = nullptr;
   const uint64_t bytes = std::max<uint64_t>(count, 1) * sizeof(T), padded = (bytes + 255) & ~uint64_t(255);
+  if (refused(what)) throw Fail{LPA_ERR_OOM, std::string(what) + " refused"};
   if (padded <= kSlabPiece && h->slab_left < padded) {
     if (cudaMalloc(&p, kSlabBytes) == cudaSuccess) {
       h->slabs.push_back(p);
@@ -274,6 +280,15 @@ static void grow_hash_slots(lpa_handle *h, size_t need) {
   check(h, cudaMemsetAsync(h->d_hash, 0, need * sizeof(HashSlot), h->stream), "clear hash slots");
 }
 
+// Until a plan's lists are complete the handle has none: what is left of the
+// old ones may be freed, or index records of another scope.
+static void drop_lists(lpa_handle *h) {
+  h->plan_ready = false;
+  h->plan_version++;  // a captured iteration holds the old lists
+  h->n_heavy = h->n_light = h->n_packed = h->n_groups = h->n_rgroups = h->n_cblock = h->n_cwarp = h->n_hash = 0;
+  for (StreamRange &r : h->ranges) r.n_heavy = r.n_light = r.n_packed = r.n_groups = r.n_cblock = r.n_cwarp = 0;
+}
+
 static void upload_lists(lpa_handle *h) {
   h2d(h, h->d_seg_var, h->run_variant.data(), h->run_variant.size(), "upload variants");
   if (h->streamed) {
@@ -342,7 +357,6 @@ static void upload_lists(lpa_handle *h) {
   h->n_hash = out.n_hash;
   h->n_rgroups = out.n_rgroups;
   ensure_gtab(h);
-  h->plan_version++;
   // the resident blocks (the warps take decode groups from a work queue),
   // fewer when there are fewer groups than warps
   h->grid_decode = int(std::max<uint64_t>(
@@ -359,7 +373,6 @@ static void upload_range_lists(lpa_handle *h) {
     cap = need + need / 4 + 16;
     ptr = dalloc<std::remove_reference_t<decltype(*ptr)>>(h, cap, what);
   };
-  h->n_heavy = h->n_light = h->n_packed = h->n_groups = h->n_cblock = h->n_cwarp = h->n_hash = 0;
   for (size_t k = 0; k < h->ranges.size(); k++) {
     StreamRange &r = h->ranges[k];
     PlanInputs in{};
@@ -423,7 +436,6 @@ static void upload_range_lists(lpa_handle *h) {
     h->n_hash += out.n_hash;
   }
   ensure_gtab(h);
-  h->plan_version++;
 }
 
 // A vertex that only a block or the two-pass kernels can take (heavy bucket)
@@ -631,15 +643,50 @@ static void apply_run_variants(lpa_handle *h) {
       if (h->variant[s] == LPA_VARIANT_BLOCK && is_hub(h->segs[s])) h->run_variant[s] = LPA_VARIANT_TWO_PASS;
 }
 
+// The work lists of h->variant and h->tune.
+static void rebuild_lists(lpa_handle *h) {
+  drop_lists(h);
+  apply_run_variants(h);
+  upload_lists(h);
+  h->plan_ready = true;
+}
+
+// Lists for what the handle is to run, when a failed change left none.
+static void ensure_lists(lpa_handle *h) {
+  if (!h->plan_ready) rebuild_lists(h);
+}
+
+// Installs a plan and knobs.  When that fails the handle goes back to what it
+// ran before; without memory for those lists either, the next iteration
+// builds them (ensure_lists).
+static void install_plan(lpa_handle *h, std::vector<uint8_t> variant, const lpa_tune &tune) {
+  std::vector<uint8_t> before = std::move(h->variant);
+  const lpa_tune tune_before = h->tune;
+  h->variant = std::move(variant);
+  h->tune = tune;
+  try {
+    rebuild_lists(h);
+  } catch (const Fail &f) {
+    h->variant = std::move(before);
+    h->tune = tune_before;
+    if (f.st == LPA_ERR_OOM && h->variant.size() == h->segs.size()) {
+      try {
+        rebuild_lists(h);
+      } catch (const Fail &) {  // plan_ready says so
+      }
+    }
+    throw;
+  }
+}
+
 static void apply_dispatch(lpa_handle *h, int dispatch, int force) {
-  h->variant.resize(h->segs.size());
+  std::vector<uint8_t> variant(h->segs.size());
   for (size_t s = 0; s < h->segs.size(); s++) {
     int v = h->fixed[s];
     if (dispatch == LPA_DISPATCH_FORCE && variant_capable(force, h->segs[s], h->opts.cms_threshold)) v = force;
-    h->variant[s] = uint8_t(v);
+    variant[s] = uint8_t(v);
   }
-  apply_run_variants(h);
-  upload_lists(h);
+  install_plan(h, std::move(variant), h->tune);
 }
 
 // Ranges of a streamed handle: consecutive plan segments of the compressed
@@ -1354,6 +1401,7 @@ lpa_status lpa_iterate(lpa_handle *h, uint64_t *changed_out) {
   if (!h) return LPA_ERR_INVALID_ARG;
   try {
     check(h, cudaSetDevice(h->device), "cudaSetDevice");
+    ensure_lists(h);
     lpa_learner_before_iteration(h);
     unsigned long long *slot = h->d_changed;
     check(h, cudaMemsetAsync(slot, 0, sizeof(unsigned long long), h->stream), "clear counter");
@@ -1405,6 +1453,12 @@ lpa_status lpa_run(lpa_handle *h, int max_iter, int early_exit, int *iters_done)
     }
     if (iters_done) *iters_done = done;
     return LPA_OK;
+  }
+  try {
+    ensure_lists(h);
+  } catch (const Fail &f) {
+    if (iters_done) *iters_done = done;
+    return guard(h, f);
   }
   int rest = 0;
   lpa_status st = lpa_run_graph(h, max_iter - done, early_exit != 0, &rest);
@@ -1515,11 +1569,11 @@ lpa_status lpa_set_dispatch(lpa_handle *h, int dispatch, int force_variant) {
   if (!h || dispatch < 0 || dispatch > 2 || force_variant < 0 || force_variant > 3) return LPA_ERR_INVALID_ARG;
   try {
     check(h, cudaSetDevice(h->device), "cudaSetDevice");
+    lpa_learner_reset(h);
+    apply_dispatch(h, dispatch == LPA_DISPATCH_FORCE ? LPA_DISPATCH_FORCE : LPA_DISPATCH_FIXED, force_variant);
     h->opts.dispatch = dispatch;
     h->opts.force_variant = force_variant;
     if (dispatch == LPA_DISPATCH_LEARNED && h->opts.record_timings < 1) h->opts.record_timings = 1;
-    lpa_learner_reset(h);
-    apply_dispatch(h, dispatch == LPA_DISPATCH_FORCE ? LPA_DISPATCH_FORCE : LPA_DISPATCH_FIXED, force_variant);
     check(h, cudaStreamSynchronize(h->stream), "dispatch");
   } catch (const Fail &f) {
     return guard(h, f);
@@ -1594,8 +1648,7 @@ lpa_status lpa_set_tune(lpa_handle *h, const lpa_tune *t) {
   if (!h || !t || !tune_valid(*t)) return LPA_ERR_INVALID_ARG;
   try {
     check(h, cudaSetDevice(h->device), "cudaSetDevice");
-    h->tune = *t;
-    lpa_rt_apply_variants(h);
+    install_plan(h, h->variant, *t);
   } catch (const Fail &f) {
     return guard(h, f);
   }
@@ -1605,9 +1658,12 @@ lpa_status lpa_set_tune(lpa_handle *h, const lpa_tune *t) {
 lpa_status lpa_autotune(lpa_handle *h, const char *cache_path, int repeats, lpa_tune *out) {
   if (!h) return LPA_ERR_INVALID_ARG;
   if (repeats <= 0) repeats = 2;
+  const lpa_tune before = h->tune;
   try {
     check(h, cudaSetDevice(h->device), "cudaSetDevice");
+    ensure_lists(h);
     const std::string key = tune_key(h);
+    lpa_tune cached{};
     bool found = false;
     if (cache_path) {
       std::ifstream in(cache_path);
@@ -1619,13 +1675,13 @@ lpa_status lpa_autotune(lpa_handle *h, const char *cache_path, int repeats, lpa_
         if (ls >> k >> t.group_positions >> t.warp_positions >> t.warp_max_degree >> t.warp_claim >> t.bulk_stage >>
                 t.gather_cache >> t.stage_stream &&
             k == key && tune_valid(t)) {
-          h->tune = t;
+          cached = t;
           found = true;
         }
       }
     }
     if (found) {
-      lpa_rt_apply_variants(h);
+      install_plan(h, h->variant, cached);
     } else if (h->n_cblock + h->n_cwarp > 0) {
       // coordinate descent, two sweeps; a candidate must win by 0.5 %
       lpa_tune best = h->tune;
@@ -1648,8 +1704,7 @@ lpa_status lpa_autotune(lpa_handle *h, const char *cache_path, int repeats, lpa_
                                          : cand.stage_stream;
             if (slot == vals[i]) continue;
             slot = vals[i];
-            h->tune = cand;
-            lpa_rt_apply_variants(h);
+            install_plan(h, h->variant, cand);
             const double ms = tune_trial(h, repeats);
             if (ms < 0) throw Fail{LPA_ERR_CUDA, "autotune: " + h->last_error};
             if (ms < best_ms * 0.995) {
@@ -1659,8 +1714,7 @@ lpa_status lpa_autotune(lpa_handle *h, const char *cache_path, int repeats, lpa_
           }
         }
       }
-      h->tune = best;
-      lpa_rt_apply_variants(h);
+      install_plan(h, h->variant, best);
       if (cache_path) {
         std::ofstream o(cache_path, std::ios::app);
         o << key << ' ' << best.group_positions << ' ' << best.warp_positions << ' ' << best.warp_max_degree << ' '
@@ -1671,6 +1725,14 @@ lpa_status lpa_autotune(lpa_handle *h, const char *cache_path, int repeats, lpa_
     if (out) *out = h->tune;
   } catch (const Fail &f) {
     h->measure_busy = false;
+    if (std::memcmp(&h->tune, &before, sizeof(before)) != 0) {  // a candidate's
+      try {
+        install_plan(h, h->variant, before);
+      } catch (const Fail &) {
+        h->tune = before;
+        h->plan_ready = false;
+      }
+    }
     return guard(h, f);
   }
   return LPA_OK;
@@ -1682,10 +1744,9 @@ lpa_status lpa_set_plan(lpa_handle *h, const uint8_t *variant, size_t count) {
     if (variant[s] > 3 || !variant_capable(variant[s], h->segs[s], h->opts.cms_threshold)) return LPA_ERR_INVALID_ARG;
   try {
     check(h, cudaSetDevice(h->device), "cudaSetDevice");
-    h->opts.dispatch = LPA_DISPATCH_FORCE;
     lpa_learner_reset(h);
-    h->variant.assign(variant, variant + count);
-    lpa_rt_apply_variants(h);
+    install_plan(h, std::vector<uint8_t>(variant, variant + count), h->tune);
+    h->opts.dispatch = LPA_DISPATCH_FORCE;
     check(h, cudaStreamSynchronize(h->stream), "plan");
   } catch (const Fail &f) {
     return guard(h, f);
@@ -1763,8 +1824,15 @@ cudaError_t lpa_rt_launch_packed_loop(lpa_handle *h) {
   }
   return e;
 }
-void lpa_rt_apply_variants(lpa_handle *h) {
-  apply_run_variants(h);
-  upload_lists(h);
+bool lpa_rt_install_plan(lpa_handle *h, const std::vector<uint8_t> &variant) {
+  try {
+    install_plan(h, variant, h->tune);
+  } catch (const Fail &f) {
+    if (f.st != LPA_ERR_OOM) throw;
+    return false;
+  }
+  return true;
 }
+void lpa_rt_ensure_lists(lpa_handle *h) { ensure_lists(h); }
+extern "C" void lpa_test_refuse(const char *what) { refused_name = what ? what : ""; }
 lpa_status lpa_rt_take_error(lpa_handle *h) { return take_device_error(h); }

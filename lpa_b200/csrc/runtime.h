@@ -201,6 +201,7 @@ struct lpa_handle {
   void *graph_exec = nullptr;  // cudaGraphExec_t of the early-exit loop
   void *graph = nullptr;       // cudaGraph_t
   uint64_t launches_per_graph_iteration = 0;
+  bool plan_ready = false;  // the work lists are those of variant and tune
   uint64_t plan_version = 0, graph_plan_version = ~0ull;
 
   // learned dispatch (cost model), see dispatch.cu
@@ -228,7 +229,13 @@ void lpa_rt_enqueue_iteration(lpa_handle *h, unsigned long long *changed, uint32
 // Per-graph convergence of a lockstep batch, enqueued after every iteration
 // (2 launches).
 void lpa_rt_enqueue_track(lpa_handle *h);
-void lpa_rt_apply_variants(lpa_handle *h);
+// Installs a plan (variant per segment); false: no memory for it, the handle
+// keeps the plan before (whose lists lpa_rt_ensure_lists builds if need be).
+bool lpa_rt_install_plan(lpa_handle *h, const std::vector<uint8_t> &variant);
+void lpa_rt_ensure_lists(lpa_handle *h);
+// For tests: from now on the calling thread's device allocations of this name
+// fail as if the device had no memory left (nullptr: none).
+extern "C" void lpa_test_refuse(const char *what);
 constexpr int kPinnedSlots = 128;  // 64-bit words of lpa_handle::h_pinned
 void lpa_rt_prepare_branches(lpa_handle *h);
 int lpa_rt_packed_loop_grid(lpa_handle *h);

@@ -1,0 +1,126 @@
+"""Plans that the device has no memory for: the call says so, the handle goes on
+with the plan it had (or with the kernels that need less), and the labels stay
+right.  lpa_test_refuse makes allocations fail by name."""
+import contextlib
+
+import numpy as np
+import pytest
+
+import lpa_b200 as L
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+CMS = 1024
+
+
+@contextlib.contextmanager
+def refuse(name):
+    L.lib().lpa_test_refuse(name.encode())
+    try:
+        yield
+    finally:
+        L.lib().lpa_test_refuse(None)
+
+
+@pytest.fixture(scope="module")
+def case():
+    g = L.HostGraph.rmat(15, 16, seed=5)
+    row, clm = g.csr()
+    assert np.diff(row).max() > 4096  # hubs, above the block table too
+    g.compress(16, 128)
+    return g, {cms: oracle.lp_run(row, clm, 6, cms, 1) for cms in (0, CMS)}
+
+
+def _check(p, hist, changed, it):
+    assert p.iterate() == changed[it]
+    assert np.array_equal(p.labels(), hist[it])
+
+
+@pytest.mark.parametrize("cms", [0, CMS])
+@pytest.mark.parametrize("budget", [0, 4 << 20], ids=["resident", "streamed"])
+@pytest.mark.parametrize("name", ["work items", "decode groups", "record groups", "count items", "count block items",
+                                  "packed chunks", "two-pass scratch", "position index", "segment records"])
+def test_failed_switch(case, name, budget, cms):
+    g, want = case
+    hist, changed = want[cms]
+    if budget and name not in ("two-pass scratch", "position index", "segment records", "record groups"):
+        name = "range " + name
+    with L.Propagator(g, cms_threshold=cms, stream_budget=budget) as p:
+        assert p.run(2) == 2  # a captured iteration of the plan that stays
+        with refuse(name):
+            with contextlib.suppress(L.LpaError):
+                p.set_dispatch(L.Dispatch.FORCE, L.Variant.TWO_PASS)
+            try:
+                ch = p.iterate()
+            except L.LpaError as e:  # no memory for the old lists either
+                assert e.status == L.Status.OOM
+            else:
+                assert ch == changed[2] and np.array_equal(p.labels(), hist[2])
+                p.set_labels(hist[1])
+        _check(p, hist, changed, 2)
+        assert p.run(3) == 3
+        assert np.array_equal(p.labels(), hist[5])
+        p.set_dispatch(L.Dispatch.FORCE, L.Variant.TWO_PASS)  # there is memory now
+        p.init_labels()
+        for it in range(3):
+            _check(p, hist, changed, it)
+
+
+def test_failed_tune(case):
+    g, want = case
+    hist, changed = want[0]
+    with L.Propagator(g, dispatch=L.Dispatch.FORCE, force_variant=int(L.Variant.TWO_PASS)) as p:
+        before = p.get_tune()
+        with refuse("count items"):
+            with pytest.raises(L.LpaError) as e:
+                p.set_tune(1, 1, before.warp_max_degree, before.warp_claim)  # more items
+            assert e.value.status == L.Status.OOM
+        assert p.get_tune().as_tuple() == before.as_tuple()
+        for it in range(3):
+            _check(p, hist, changed, it)
+
+
+def test_learner_without_memory(case):
+    """Explorations that do not fit: the heuristic plan stays."""
+    g, want = case
+    hist, changed = want[CMS]
+    with L.Propagator(g, cms_threshold=CMS, dispatch=L.Dispatch.LEARNED) as p:
+        with refuse("two-pass scratch"):
+            for it in range(6):
+                _check(p, hist, changed, it)
+        p.init_labels()
+        p.run(6)
+        assert np.array_equal(p.labels(), hist[5])
+
+
+@pytest.mark.parametrize("cms", [0, CMS])
+@pytest.mark.parametrize("thresh", [0, 16])
+def test_hubs_without_scratch(case, thresh, cms):
+    """No memory for the hubs' labels: blocks of k_iterate decode and count them."""
+    g, want = case
+    hist, changed = want[cms]
+    row, clm = g.csr()
+    g2 = L.HostGraph.from_csr(row, clm).compress(thresh, 128)
+    with refuse("two-pass scratch"):
+        p = L.Propagator(g2, cms_threshold=cms)
+    with p:
+        for it in range(3):
+            _check(p, hist, changed, it)
+        p.init_labels()
+        p.run(6)
+        assert np.array_equal(p.labels(), hist[5])
+
+
+@pytest.mark.parametrize("gather", [0, 1, 2])
+@pytest.mark.parametrize("stage", [0, 1, 2])
+def test_without_records(case, stage, gather):
+    """No memory for the segment records: decode groups cover the residual segments."""
+    g, want = case
+    hist, changed = want[CMS]
+    with refuse("segment records"):
+        p = L.Propagator(g, cms_threshold=CMS, dispatch=L.Dispatch.FORCE, force_variant=int(L.Variant.TWO_PASS))
+    with p:
+        p.set_tune(*p.get_tune().as_tuple()[:5], gather, stage)
+        for it in range(3):
+            _check(p, hist, changed, it)
