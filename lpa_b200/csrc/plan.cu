@@ -63,6 +63,7 @@ struct PlanArgs {
   PackedChunk *packed;
   DecodeGroup *groups;
   RecGroup *rgroups;
+  uint32_t *heavy_exact;     // max: exact degrees of the heavy items above the shared table
   BlockItem *cblock;         // unsorted, with keys
   uint32_t *cblock_key;
   CountItem *cwarp;          // warp items, then group items from n_warp on
@@ -171,6 +172,8 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
     if (kEmit) {
       a.heavy[o[kLHeavy]] = make_item(a, s, si.begin, si.end, tp);
       a.heavy_key[o[kLHeavy]] = uint32_t(si.arcs < 0xFFFFFFFFull ? si.arcs : 0xFFFFFFFFull);
+    } else if (si.max_deg > kBlockMaxSmemDeg && (cms == 0 || si.max_deg < cms)) {
+      atomicMax(a.heavy_exact, si.max_deg);
     }
     c[kLHeavy] = 1;
   } else if (v == kVarPacked && si.max_deg <= kPackedMaxDeg) {
@@ -376,7 +379,7 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   const size_t scan_bytes = need;
   const auto pad = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t per_list = pad(size_t(kLists) * stride * 4), marks = pad(std::max<uint64_t>(1, in.n) * 4),
-               windows = pad((nwin + 1) * 4), totals = pad((kLists + 1) * 4);
+               windows = pad((nwin + 1) * 4), totals = pad((kLists + 2) * 4);
   PB_TRY(reserve(&count_ws, count_ws_cap, 2 * per_list + marks + 2 * windows + totals + scan_bytes), "plan counts");
   char *ws = static_cast<char *>(count_ws);
   const auto take = [&ws](size_t bytes) {
@@ -394,6 +397,7 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   PB_TRY(cudaMemsetAsync(cnt, 0, size_t(kLists) * stride * 4, st), "clear counts");
   PB_TRY(cudaMemsetAsync(win, 0, (nwin + 1) * 4, st), "clear windows");
   PB_TRY(cudaMemsetAsync(gmark, 0, std::max<uint64_t>(1, in.n) * 4, st), "clear marks");
+  PB_TRY(cudaMemsetAsync(tot, 0, (kLists + 2) * 4, st), "clear totals");
 
   PlanArgs a{};
   a.segs = in.segs;
@@ -424,6 +428,7 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   a.off = off;
   a.cnt = cnt;
   a.gmark = gmark;
+  a.heavy_exact = tot + kLists + 1;
   a.win_cnt = win;
   a.win_off = win_off;
   if (S) k_plan_count<<<grid_for(S, in.num_sms), 256, 0, st>>>(a);
@@ -438,8 +443,8 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   PB_TRY(cub::DeviceScan::ExclusiveSum(temp, t, win, win_off, nwin + 1, st), "window scan");
   k_plan_totals<<<1, 32, 0, st>>>(off, stride, win_off, nwin, tot);
   PB_TRY(cudaGetLastError(), "totals launch");
-  uint32_t h_tot[kLists + 1] = {};
-  PB_TRY(cudaMemcpyAsync(h_tot, tot, (kLists + 1) * 4, cudaMemcpyDeviceToHost, st), "read totals");
+  uint32_t h_tot[kLists + 2] = {};
+  PB_TRY(cudaMemcpyAsync(h_tot, tot, (kLists + 2) * 4, cudaMemcpyDeviceToHost, st), "read totals");
   PB_TRY(cudaStreamSynchronize(st), "plan totals");
   out.n_heavy = h_tot[kLHeavy];
   out.n_light = h_tot[kLLight];
@@ -449,6 +454,7 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   out.n_cwarp = h_tot[kLWarp] + h_tot[kLists];
   out.n_hash = h_tot[kLHash];
   out.n_rgroups = h_tot[kLRecs];
+  out.heavy_exact_deg = h_tot[kLists + 1];
 
   // outputs (the caller's buffers grow to fit) and sort staging
   PB_TRY(out.grow(out), "work lists");

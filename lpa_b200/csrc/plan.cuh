@@ -54,6 +54,7 @@ cudaError_t exclusive_sum(uint64_t *data, uint64_t n, void *temp, size_t &temp_b
 struct PlanOutputs {
   uint32_t n_heavy = 0, n_light = 0, n_packed = 0, n_groups = 0, n_cblock = 0, n_cwarp = 0, n_hash = 0,
            n_rgroups = 0;
+  uint32_t heavy_exact_deg = 0;  // largest exact degree of the heavy items above the shared table, 0: none
   WorkItem *items = nullptr;
   PackedChunk *packed = nullptr;
   DecodeGroup *groups = nullptr;

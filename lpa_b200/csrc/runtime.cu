@@ -259,16 +259,23 @@ static void build_segments(lpa_handle *h) {
 // few launches and one copy of the list sizes, not a host loop over n.
 static void upload_range_lists(lpa_handle *h);
 
-// Global exact-count tables, once a plan gives k_iterate heavy items: for its
-// exact vertices above the shared table, one table per block, at most 2 GiB.
-static void ensure_gtab(lpa_handle *h) {
-  if (h->d_gtab || h->n_heavy == 0 || h->max_exact_deg == 0) return;
-  h->gtab_slots = next_pow2_host(2 * uint64_t(h->max_exact_deg));
-  const uint64_t per_block = uint64_t(h->gtab_slots) * 2 * sizeof(uint32_t);
-  h->gtab_blocks = int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(h->grid), (2ull << 30) / per_block)));
-  h->d_gtab = dalloc<uint32_t>(h, uint64_t(h->gtab_blocks) * 2 * h->gtab_slots, "global count tables");
+// Global exact-count tables, for a plan that gives k_iterate exact vertices
+// above the shared table, the largest of degree max_deg (0: it has none): one
+// table per block, at most 2 GiB, and no more blocks than tables.
+static void ensure_gtab(lpa_handle *h, uint32_t max_deg) {
+  h->grid = h->num_sms * h->occ;
+  if (max_deg == 0) return;
+  const uint32_t slots = next_pow2_host(2 * uint64_t(max_deg));
+  if (!h->d_gtab || slots > h->gtab_slots) {
+    dfree(h, h->d_gtab);
+    const uint64_t per_block = uint64_t(slots) * 2 * sizeof(uint32_t);
+    const int blocks = int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(h->grid), (2ull << 30) / per_block)));
+    h->d_gtab = dalloc<uint32_t>(h, uint64_t(blocks) * 2 * slots, "global count tables");
+    h->gtab_slots = slots;
+    h->gtab_blocks = blocks;
+    check(h, cudaMemsetAsync(h->d_gtab, 0, uint64_t(blocks) * per_block, h->stream), "clear tables");
+  }
   h->grid = std::min(h->grid, h->gtab_blocks);
-  check(h, cudaMemsetAsync(h->d_gtab, 0, uint64_t(h->gtab_blocks) * per_block, h->stream), "clear tables");
 }
 
 static void grow_hash_slots(lpa_handle *h, size_t need) {
@@ -356,7 +363,7 @@ static void upload_lists(lpa_handle *h) {
   h->n_cwarp = out.n_cwarp;
   h->n_hash = out.n_hash;
   h->n_rgroups = out.n_rgroups;
-  ensure_gtab(h);
+  ensure_gtab(h, out.heavy_exact_deg);
   // the resident blocks (the warps take decode groups from a work queue),
   // fewer when there are fewer groups than warps
   h->grid_decode = int(std::max<uint64_t>(
@@ -373,6 +380,7 @@ static void upload_range_lists(lpa_handle *h) {
     cap = need + need / 4 + 16;
     ptr = dalloc<std::remove_reference_t<decltype(*ptr)>>(h, cap, what);
   };
+  uint32_t heavy_exact = 0;
   for (size_t k = 0; k < h->ranges.size(); k++) {
     StreamRange &r = h->ranges[k];
     PlanInputs in{};
@@ -434,8 +442,9 @@ static void upload_range_lists(lpa_handle *h) {
     h->n_cblock += r.n_cblock;
     h->n_cwarp += r.n_cwarp;
     h->n_hash += out.n_hash;
+    heavy_exact = std::max(heavy_exact, out.heavy_exact_deg);
   }
-  ensure_gtab(h);
+  ensure_gtab(h, heavy_exact);
 }
 
 // A vertex that only a block or the two-pass kernels can take (heavy bucket)
@@ -835,11 +844,6 @@ static void build_plan(lpa_handle *h) {
   check(h, cudaMemsetAsync(h->d_seg_cycles, 0, std::max<size_t>(1, h->segs.size()) * sizeof(long long), h->stream),
         "clear cycles");
 
-  for (uint64_t p = 0; p < h->n; p++) {
-    const uint32_t d = h->h_deg[p];
-    if (!(h->opts.cms_threshold != 0 && d >= h->opts.cms_threshold) && d > kBlockMaxSmemDeg)
-      h->max_exact_deg = std::max(h->max_exact_deg, d);
-  }
   apply_dispatch(h, h->opts.dispatch == LPA_DISPATCH_FORCE ? LPA_DISPATCH_FORCE : LPA_DISPATCH_FIXED,
                  h->opts.force_variant);
 }

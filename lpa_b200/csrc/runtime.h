@@ -178,7 +178,6 @@ struct lpa_handle {
   std::vector<void *> allocations, slabs;
   char *slab = nullptr;         // the rest of the last shared block
   uint64_t slab_left = 0;
-  uint32_t max_exact_deg = 0;   // largest exact degree above the shared table
 
   // out-of-core streaming (opts.stream_budget): the stream in pinned host
   // memory, two device buffers filled on copy_stream, the ranges

@@ -124,3 +124,28 @@ def test_without_records(case, stage, gather):
         p.set_tune(*p.get_tune().as_tuple()[:5], gather, stage)
         for it in range(3):
             _check(p, hist, changed, it)
+
+
+def test_count_tables_only_where_used(case):
+    """Exact hubs above the shared table run through the two-pass kernels: heavy
+    items of the small CSR (degree 1024 to 2047) need no global tables for them."""
+    g, want = case
+    hist, changed = want[0]
+    row, clm = g.csr()
+    deg = np.diff(row)
+    assert ((deg > 1023) & (deg < 2048)).any()
+    with refuse("global count tables"):
+        with L.Propagator(L.HostGraph.from_csr(row, clm).compress(2048, 2048)) as p:
+            for it in range(3):
+                _check(p, hist, changed, it)
+            p.set_dispatch(L.Dispatch.FORCE, L.Variant.BLOCK)
+            p.init_labels()
+            p.run(6)
+            assert np.array_equal(p.labels(), hist[5])
+        small = L.HostGraph.from_csr(row, clm).compress(8192, 8192)  # the hubs in the small CSR
+        with pytest.raises(L.LpaError) as e:
+            L.Propagator(small)
+        assert e.value.status == L.Status.OOM
+    with L.Propagator(small) as p:
+        for it in range(3):
+            _check(p, hist, changed, it)
