@@ -39,7 +39,7 @@ typedef enum lpa_status {
   LPA_ERR_CUDA = 1,        /* a CUDA runtime call failed */
   LPA_ERR_OOM = 2,         /* a device allocation failed */
   LPA_ERR_BAD_STREAM = 3,  /* the decoder left a vertex's bit range, or an id >= n */
-  LPA_ERR_TIMEOUT = 4,     /* a bounded device wait gave up */
+  LPA_ERR_TIMEOUT = 4,     /* a bounded device wait gave up; the labels are undefined until they are set */
   LPA_ERR_INVALID_ARG = 5, /* bad pointer, size or option */
   LPA_ERR_IO = 6,          /* a file is missing or malformed */
   LPA_ERR_NO_DEVICE = 7,   /* no usable CUDA device */
@@ -161,7 +161,10 @@ lpa_status lpa_set_labels(struct lpa_handle *h, const uint32_t *host, size_t n);
  * (baselines/novaplus/novaplus_propogator.cuh:131-199). */
 lpa_status lpa_iterate(struct lpa_handle *h, uint64_t *changed_out);
 /* Runs up to max_iter iterations; with early_exit it stops after an iteration
- * that changed nothing (device-side test inside a CUDA graph).  Replaces
+ * that changed nothing (device-side test inside a CUDA graph).  A plan of tiny
+ * segments alone (a road graph) runs as one cooperative launch: when other work
+ * on the device keeps part of its blocks from starting for 60 s, the call
+ * returns LPA_ERR_TIMEOUT.  Replaces
  * NovaPlusPropagator::run (baselines/novaplus/novaplus_propogator.cuh:100-129). */
 lpa_status lpa_run(struct lpa_handle *h, int max_iter, int early_exit, int *iters_done);
 /* Per-iteration changed counts of the last lpa_run (count entries). */

@@ -119,7 +119,7 @@ lpa_status lpa_run_graph(lpa_handle *h, int max_iter, bool early_exit, int *iter
   const uint32_t start = uint32_t(h->cur);
   lpa_dev::PackedLoop *ctl = reinterpret_cast<lpa_dev::PackedLoop *>(h->h_pinned);
   lpa_dev::PackedLoop *back = ctl + 1;
-  *ctl = lpa_dev::PackedLoop{start, start + uint32_t(max_iter), early_exit ? 1u : 0u, start, 0u, 0u};
+  *ctl = lpa_dev::PackedLoop{start, start + uint32_t(max_iter), early_exit ? 1u : 0u, start, 0u, 0u, h->loop_wait_ns};
   e = cudaMemsetAsync(h->d_changed, 0, size_t(max_iter + 2) * sizeof(unsigned long long), h->stream);
   if (e != cudaSuccess) return fail(e, "clear counters");
   e = cudaMemcpyAsync(h->d_loop_it, ctl, sizeof(*ctl), cudaMemcpyHostToDevice, h->stream);

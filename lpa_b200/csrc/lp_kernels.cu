@@ -1277,17 +1277,21 @@ __global__ void __launch_bounds__(kThreads) k_packed(IterArgs a) {
 // Waits until every block of the launch has arrived for the k-th time (k from
 // 1).  Bounded: when the others do not arrive, the error word is set and
 // every block gives up.  The launch is cooperative, so all blocks are resident.
-__device__ __forceinline__ bool grid_barrier(PackedLoop *lp, uint32_t k, uint32_t *err) {
+__device__ __forceinline__ bool grid_barrier(PackedLoop *lp, uint32_t k, uint64_t limit, uint32_t *err) {
   __shared__ uint32_t s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(&lp->arrived, 1u);
     const volatile uint32_t *seen = &lp->arrived, *gone = &lp->gone;
-    uint32_t tries = 0;
+    unsigned long long t0 = 0;
     bool ok = true;
-    while (*seen < k * gridDim.x) {
-      if (*gone || ++tries > kBarrierTries) {
+    // the clock on one poll in 64: reading it on each took 0.25 us an iteration
+    for (uint32_t polls = 1; *seen < k * gridDim.x; polls++) {
+      if ((polls & 63u) && limit) continue;
+      const unsigned long long now = global_ns();
+      if (t0 == 0) t0 = now;
+      if (*gone || now - t0 >= limit) {
         ok = false;
         break;
       }
@@ -1308,14 +1312,15 @@ __device__ __forceinline__ bool grid_barrier(PackedLoop *lp, uint32_t k, uint32_
 // the work (road grid 64^2),
 // a barrier of the resident blocks 2 to 3 (lpa_run, 20 iterations: 207 -> 120 us;
 // 362^2: 261 -> 195 us).
-// Iterations lp->it .. lp->stop - 1 (lp->early: until nothing changes); the
-// last block's thread leaves the next iteration's number in lp->it.
+// Iterations lp->it .. lp->stop - 1 (lp->early: until nothing changes); block 0
+// leaves the number of the iteration after the last in lp->it_end.
 __global__ void __launch_bounds__(kThreads) k_packed_loop(IterArgs a, PackedLoop *lp) {
   __shared__ uint32_t slab[kThreads * kPackedMaxDeg];
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   const uint32_t first = lp->it, stop = lp->stop;
   const bool early = lp->early != 0u;
+  const uint64_t limit = lp->wait_ns;
   uint32_t it = first;
   bool ok = true;
   while (it < stop) {
@@ -1338,7 +1343,7 @@ __global__ void __launch_bounds__(kThreads) k_packed_loop(IterArgs a, PackedLoop
     }
     flush_changed(c.changed, changed);
     it++;
-    if (!grid_barrier(lp, it - first, a.err)) {
+    if (!grid_barrier(lp, it - first, limit, a.err)) {
       ok = false;
       break;
     }

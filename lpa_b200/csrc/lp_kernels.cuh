@@ -309,8 +309,12 @@ struct PackedLoop {
   uint32_t it, stop, early;
   uint32_t it_end;         // out: the iteration after the last
   uint32_t arrived, gone;  // the barrier's arrivals; a block that gave up
+  uint64_t wait_ns;        // how long a block waits at the barrier before it gives up
 };
-constexpr uint32_t kBarrierTries = 1u << 24;  // polls (of an L2 round trip) before a barrier gives up
+// A block waits for the longest share of an iteration (below 1 ms) and for
+// blocks that have no SM yet, as long as other streams' kernels hold it: a
+// time on the GPU's clock, far above both, not a number of polls.
+constexpr uint64_t kBarrierWaitNs = 60ull * 1000 * 1000 * 1000;
 cudaError_t occupancy_packed_loop(int *blocks);
 cudaError_t launch_packed_loop(int grid, cudaStream_t s, IterArgs a, PackedLoop *lp);
 

@@ -1838,5 +1838,6 @@ bool lpa_rt_install_plan(lpa_handle *h, const std::vector<uint8_t> &variant) {
   return true;
 }
 void lpa_rt_ensure_lists(lpa_handle *h) { ensure_lists(h); }
+extern "C" void lpa_test_loop_wait(lpa_handle *h, uint64_t ns) { h->loop_wait_ns = ns; }
 extern "C" void lpa_test_refuse(const char *what) { refused_name = what ? what : ""; }
 lpa_status lpa_rt_take_error(lpa_handle *h) { return take_device_error(h); }

@@ -196,6 +196,7 @@ struct lpa_handle {
   // CUDA-graph loop: while set, kernels take their parity and counter slot from it
   const uint32_t *loop_it = nullptr;
   uint32_t *d_loop_it = nullptr;  // a lpa_dev::PackedLoop; the graph's step kernel uses its first three words
+  uint64_t loop_wait_ns = lpa_dev::kBarrierWaitNs;
   int occ_packed_loop = -1;       // resident blocks per SM of k_packed_loop (-1: not asked yet)
   void *graph_exec = nullptr;  // cudaGraphExec_t of the early-exit loop
   void *graph = nullptr;       // cudaGraph_t
@@ -235,6 +236,8 @@ void lpa_rt_ensure_lists(lpa_handle *h);
 // For tests: from now on the calling thread's device allocations of this name
 // fail as if the device had no memory left (nullptr: none).
 extern "C" void lpa_test_refuse(const char *what);
+// For tests: the handle's PackedLoop::wait_ns.
+extern "C" void lpa_test_loop_wait(lpa_handle *h, uint64_t ns);
 constexpr int kPinnedSlots = 128;  // 64-bit words of lpa_handle::h_pinned
 void lpa_rt_prepare_branches(lpa_handle *h);
 int lpa_rt_packed_loop_grid(lpa_handle *h);
