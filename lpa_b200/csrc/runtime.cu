@@ -88,6 +88,28 @@ void dfree(lpa_handle *h, T *&p) {
   p = nullptr;
 }
 
+// Device memory of one call.
+template <class T>
+struct TempBuf {
+  T *p = nullptr;
+  cudaError_t alloc(uint64_t count) {
+    const cudaError_t e = cudaMalloc(&p, std::max<uint64_t>(count, 1) * sizeof(T));
+    if (e != cudaSuccess) {
+      p = nullptr;
+      cudaGetLastError();
+    }
+    return e;
+  }
+  void release() {
+    if (p) cudaFree(p);
+    p = nullptr;
+  }
+  ~TempBuf() { release(); }
+  TempBuf() = default;
+  TempBuf(const TempBuf &) = delete;
+  TempBuf &operator=(const TempBuf &) = delete;
+};
+
 template <class T>
 void h2d(lpa_handle *h, T *dst, const T *src, uint64_t count, const char *what) {
   if (count == 0) return;
@@ -451,23 +473,6 @@ static void upload_range_lists(lpa_handle *h) {
 // in the compressed region.
 static bool is_hub(const SegInfo &s) { return s.region == 0 && s.bucket == kHeavy; }
 
-// Device memory of one call.
-template <class T>
-struct TempBuf {
-  T *p = nullptr;
-  cudaError_t alloc(uint64_t count) {
-    const cudaError_t e = cudaMalloc(&p, std::max<uint64_t>(count, 1) * sizeof(T));
-    if (e != cudaSuccess) {
-      p = nullptr;
-      cudaGetLastError();
-    }
-    return e;
-  }
-  ~TempBuf() {
-    if (p) cudaFree(p);
-  }
-};
-
 static void build_records(lpa_handle *h, bool full);
 
 // The two-pass kernels' scratch and position index, for the hubs alone (a
@@ -745,13 +750,11 @@ static void build_ranges(lpa_handle *h) {
 static void build_plan(lpa_handle *h) {
   // degrees, decoded once on the device (validates the stream as well)
   h->d_deg = dalloc<uint32_t>(h, h->n, "degrees");
-  uint32_t *d_itv = nullptr;
-  check(h, cudaMalloc(&d_itv, std::max<uint64_t>(1, h->n) * sizeof(uint32_t)), "interval counts");
+  TempBuf<uint32_t> itv_buf, hubs_buf;
+  check(h, itv_buf.alloc(h->n), "interval counts");
   // the positions left to k_degree_hubs, after their number
-  uint32_t *d_hubs = nullptr;
-  cudaError_t he = cudaMalloc(&d_hubs, (h->n_c + 1) * sizeof(uint32_t));
-  if (he != cudaSuccess) cudaFree(d_itv);
-  check(h, he, "hub list");
+  check(h, hubs_buf.alloc(h->n_c + 1), "hub list");
+  uint32_t *const d_itv = itv_buf.p, *const d_hubs = hubs_buf.p;
   const int threads = 128;
   auto degree_pass = [&](const DevGraph &g, uint64_t p0, uint64_t p1) {
     if (p1 <= p0) return;
@@ -803,8 +806,8 @@ static void build_plan(lpa_handle *h) {
         "read degrees");
   std::vector<uint32_t> itv(h->n);
   check(h, cudaMemcpy(itv.data(), d_itv, h->n * sizeof(uint32_t), cudaMemcpyDeviceToHost), "read interval counts");
-  cudaFree(d_itv);
-  cudaFree(d_hubs);
+  itv_buf.release();
+  hubs_buf.release();
   h->m = 0;
   h->max_deg = 0;
   for (uint64_t p = 0; p < h->n; p++) {

@@ -5,6 +5,7 @@ import contextlib
 
 import numpy as np
 import pytest
+import torch
 
 import lpa_b200 as L
 import oracle
@@ -149,3 +150,17 @@ def test_count_tables_only_where_used(case):
     with L.Propagator(small) as p:
         for it in range(3):
             _check(p, hist, changed, it)
+
+
+def test_refused_graph_leaves_no_memory():
+    """A malformed stream is refused after the degree pass: all its memory comes back."""
+    arr = L.HostGraph.road(1000, 1000, seed=3).compress(0, 128).arrays()
+    mid = len(arr["words"]) // 2
+    arr["words"][mid:mid + 8] = 0
+    free = []
+    for _ in range(6):  # 4 MB of interval counts and 4 MB of hub list each
+        with pytest.raises(L.LpaError) as e:
+            L.Propagator(L.desc_from_arrays(arr))
+        assert e.value.status == L.Status.BAD_STREAM
+        free.append(torch.cuda.mem_get_info(0)[0])
+    assert free[0] - free[-1] < 4 << 20
