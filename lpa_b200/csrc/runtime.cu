@@ -1627,7 +1627,8 @@ static double tune_trial(lpa_handle *h, int repeats) {
   return best;
 }
 
-// The cache key: GPU, graph, sketch threshold and plan.
+// The cache key: the kernels the knobs were found for (raised with them), GPU,
+// graph, sketch threshold and plan.
 static std::string tune_key(const lpa_handle *h) {
   cudaDeviceProp pr{};
   if (cudaGetDeviceProperties(&pr, h->device) != cudaSuccess) cudaGetLastError();
@@ -1639,7 +1640,7 @@ static std::string tune_key(const lpa_handle *h) {
   uint64_t arcs = 0;
   for (const auto &sg : h->segs) arcs += sg.arcs;
   char buf[512];
-  std::snprintf(buf, sizeof(buf), "v5|%s|sm%d|n%llu|nc%llu|arcs%llu|cms%u|plan%016llx", gpu.c_str(), pr.multiProcessorCount,
+  std::snprintf(buf, sizeof(buf), "v6|%s|sm%d|n%llu|nc%llu|arcs%llu|cms%u|plan%016llx", gpu.c_str(), pr.multiProcessorCount,
                 (unsigned long long)h->n, (unsigned long long)h->n_c, (unsigned long long)arcs,
                 h->opts.cms_threshold, (unsigned long long)fnv);
   return buf;
