@@ -469,10 +469,6 @@ static void upload_range_lists(lpa_handle *h) {
   ensure_gtab(h, heavy_exact);
 }
 
-// A vertex that only a block or the two-pass kernels can take (heavy bucket)
-// in the compressed region.
-static bool is_hub(const SegInfo &s) { return s.region == 0 && s.bucket == kHeavy; }
-
 static void build_records(lpa_handle *h, bool full);
 
 // The two-pass kernels' scratch and position index, for the hubs alone (a
@@ -489,8 +485,7 @@ static void ensure_two_pass_scratch(lpa_handle *h, bool full) {
   if (first) {
     std::vector<uint8_t> hub(h->n_c, 0);
     if (!h->streamed)
-      for (const SegInfo &s : h->segs)
-        if (is_hub(s)) std::fill(hub.begin() + s.begin, hub.begin() + s.end, uint8_t(1));
+      for (const uint32_t s : h->hub_segs) std::fill(hub.begin() + h->segs[s].begin, hub.begin() + h->segs[s].end, uint8_t(1));
     off.assign(h->n_c + 1, 0);
     uint64_t at = 0;
     for (int pass = 0; pass < 2; pass++) {
@@ -574,8 +569,11 @@ static void build_records(lpa_handle *h, bool full) {
   dfree(h, h->d_seg_rec);
   const uint32_t nseg = uint32_t(h->segs.size());
   if (h->streamed || h->n_c == 0 || h->total_bits + 1024 >= kSegMaxBit || h->h_arc_off[h->n_c] >= kSegMaxIndex) return;
+  uint32_t region0 = 0;  // the compressed region's segments come first
+  while (region0 < nseg && h->segs[region0].region == 0) region0++;
   std::vector<uint8_t> use(nseg);
-  for (uint32_t s = 0; s < nseg; s++) use[s] = h->segs[s].region == 0 && (full || is_hub(h->segs[s]));
+  if (full) std::fill(use.begin(), use.begin() + region0, uint8_t(1));
+  else for (const uint32_t s : h->hub_segs) use[s] = 1;
   // working memory, two allocations: {position sums, indices, scope, scan}, {count sums, scan}
   struct Piece { uint64_t *p = nullptr; } roff, csum, index;
   TempBuf<uint64_t> w1, w2;
@@ -618,8 +616,6 @@ static void build_records(lpa_handle *h, bool full) {
   k_seg_counts<<<blocks, 256, 0, h->stream>>>(dev_graph(h), h->d_pidx, roff.p, csum.p, h->d_err);
   check(h, exclusive_sum(csum.p, total + 1, scan2, t2, h->stream), "record scan");
   k_seg_records<<<blocks, 256, 0, h->stream>>>(dev_graph(h), h->d_pidx, roff.p, csum.p, index.p, recs);
-  uint32_t region0 = 0;  // the compressed region's segments come first
-  while (region0 < nseg && h->segs[region0].region == 0) region0++;
   if (region0)
     k_seg_ranges<<<int(std::min<uint32_t>((region0 + 255) / 256, uint32_t(blocks))), 256, 0, h->stream>>>(
         h->d_segs, region0, roff.p, seg_rec);
@@ -637,11 +633,10 @@ static void build_records(lpa_handle *h, bool full) {
 // 0.82 to 1.86 ms in k_iterate, 7 ms of work on one of 296 blocks.  Without
 // memory for the hubs' labels k_iterate's blocks decode them.
 static void apply_run_variants(lpa_handle *h) {
-  bool two = false, hubs = false;
-  for (size_t s = 0; s < h->segs.size(); s++) {
-    two |= h->variant[s] == LPA_VARIANT_TWO_PASS;
-    hubs |= h->variant[s] == LPA_VARIANT_BLOCK && is_hub(h->segs[s]);
-  }
+  const std::vector<uint8_t> &v = h->variant;
+  const bool two = !v.empty() && std::memchr(v.data(), LPA_VARIANT_TWO_PASS, v.size()) != nullptr;
+  bool hubs = false;
+  for (const uint32_t s : h->hub_segs) hubs |= v[s] == LPA_VARIANT_BLOCK;
   if (two) ensure_two_pass_scratch(h, true);
   if (hubs && h->hubs_two_pass) {
     try {
@@ -651,10 +646,10 @@ static void apply_run_variants(lpa_handle *h) {
       h->hubs_two_pass = false;
     }
   }
-  h->run_variant = h->variant;
+  h->run_variant = v;
   if (hubs && h->hubs_two_pass)
-    for (size_t s = 0; s < h->segs.size(); s++)
-      if (h->variant[s] == LPA_VARIANT_BLOCK && is_hub(h->segs[s])) h->run_variant[s] = LPA_VARIANT_TWO_PASS;
+    for (const uint32_t s : h->hub_segs)
+      if (v[s] == LPA_VARIANT_BLOCK) h->run_variant[s] = LPA_VARIANT_TWO_PASS;
 }
 
 // The work lists of h->variant and h->tune.
@@ -820,6 +815,11 @@ static void build_plan(lpa_handle *h) {
     for (uint32_t p = sg.begin; p < sg.end; p++) iv += itv[p];
     sg.intervals = uint32_t(std::min<uint64_t>(iv, 0xFFFFFFFFull));
   }
+  // vertices of the compressed region that only a block or the two-pass kernels
+  // can take, as a list: a walk over all segments took most of a plan change
+  // (1.5M segments, R-MAT scale 24)
+  for (size_t s = 0; s < h->segs.size() && h->segs[s].region == 0; s++)
+    if (h->segs[s].bucket == kHeavy) h->hub_segs.push_back(uint32_t(s));
   if (h->streamed) build_ranges(h);
   h->fixed.resize(h->segs.size());
   for (size_t s = 0; s < h->segs.size(); s++) h->fixed[s] = uint8_t(fixed_variant(h->segs[s]));

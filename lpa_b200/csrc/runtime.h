@@ -101,6 +101,7 @@ struct lpa_handle {
   // plan
   std::vector<uint32_t> h_deg;
   std::vector<lpa_rt::SegInfo> segs;
+  std::vector<uint32_t> hub_segs;  // the heavy bucket's segments of the compressed region
   std::vector<uint8_t> variant;  // per segment
   std::vector<uint8_t> run_variant;          // what the kernels run for it (apply_run_variants)
   std::vector<uint8_t> fixed;    // per segment, the heuristic's choice
