@@ -97,7 +97,8 @@ typedef struct lpa_opts {
    * copied from host memory on a second stream while the previous range is
    * processed.  The ranges are cut so that two stream buffers (a quarter of
    * the budget each) and the two-pass label scratch (half) fit in this many
-   * bytes; per-vertex arrays, labels and the small CSR stay resident.
+   * bytes; per-vertex arrays (the two-pass kernels' arrays by position among
+   * them, see lpa_create), labels and the small CSR stay resident.
    * LPA_ERR_CAPACITY when one vertex alone does not fit.  Single graphs only:
    * lpa_batch_create rejects it. */
   uint64_t stream_budget;
@@ -114,7 +115,7 @@ typedef struct lpa_info {
   uint64_t num_segments;
   uint64_t max_degree;
   uint64_t bytes_algorithmic; /* one iteration's compulsory bytes (see lpa_info docs) */
-  uint64_t device_bytes;      /* device memory held by the handle */
+  uint64_t device_bytes;      /* device memory held by the handle (see lpa_create) */
 } lpa_info;
 
 typedef struct lpa_stats {
@@ -144,7 +145,17 @@ void lpa_opts_default(lpa_opts *o);
 
 /* --------------------------------------------------- propagator handle ---- */
 /* Copies the graph to the device, derives every compressed vertex's degree by
- * decoding it once, and builds the dispatch plan.  Replaces
+ * decoding it once, and builds the dispatch plan.
+ *
+ * Device memory: the compressed graph, 16 bytes per vertex (ids, degrees, two
+ * label buffers), 2.5 MB of counters, the plan's work lists, and for what runs
+ * through the two-pass kernels their labels (4 bytes per arc), 16 bytes per
+ * 256-bit segment of residuals and 28 bytes per compressed position.  Under
+ * every plan those are at least the hubs of the bitstream, the vertices of
+ * degree above 1023 or at the sketch threshold; a plan with two-pass segments
+ * has them for every compressed position.  Where the device has no room for
+ * the hubs' labels, blocks decode and count the hubs instead; lpa_create does
+ * not leave room for allocations that the caller makes later.  Replaces
  * NovaPlusPropagator::preprocess / transfer_data
  * (baselines/novaplus/novaplus_propogator.cuh:201-204,340-373). */
 lpa_status lpa_create(const lpa_graph_desc *g, const lpa_opts *o, struct lpa_handle **out);

@@ -71,6 +71,7 @@ T *dalloc(lpa_handle *h, uint64_t count, const char *what) {
       throw Fail{LPA_ERR_OOM, std::string("cudaMalloc ") + what + " (" + std::to_string(bytes) + " bytes)"};
     }
     h->allocations.push_back(p);
+    h->alloc_bytes[p] = bytes;
   }
   h->device_bytes += bytes;
   return static_cast<T *>(p);
@@ -83,6 +84,11 @@ void dfree(lpa_handle *h, T *&p) {
   const auto it = std::find(h->allocations.begin(), h->allocations.end(), (void *)p);
   if (it != h->allocations.end()) {
     h->allocations.erase(it);
+    const auto b = h->alloc_bytes.find(p);
+    if (b != h->alloc_bytes.end()) {
+      h->device_bytes -= b->second;
+      h->alloc_bytes.erase(b);
+    }
     cudaFree(p);
   }
   p = nullptr;
@@ -475,11 +481,12 @@ static void build_records(lpa_handle *h, bool full);
 // plan whose block-variant hubs run through them) or for every compressed
 // position.  The hubs' labels have an allocation of their own, so that a
 // handle that goes from one to the other holds no more than the whole: index
-// arc_off[p] of d_scratch reaches into either.
+// arc_off[p] of d_scratch reaches into either.  A streamed handle has one
+// range's labels at a time, after up to 3 words of alignment, in either case.
+// The arrays by position (28 bytes each) end 32 positions after the last hub,
+// as far as the pre-pass reads them, unless every position is in the scope.
 static void ensure_two_pass_scratch(lpa_handle *h, bool full) {
   if (h->scratch_scope >= (full ? 2 : 1)) return;
-  if (h->streamed) full = true;  // one range's labels at a time, after up to 3 words of alignment
-  const uint64_t nc = std::max<uint64_t>(1, h->n_c);
   const bool first = h->scratch_scope == 0;
   std::vector<uint64_t> &off = h->h_arc_off;  // streamed: in position order, else the hubs' labels first
   if (first) {
@@ -498,62 +505,61 @@ static void ensure_two_pass_scratch(lpa_handle *h, bool full) {
     }
     off[h->n_c] = at;
   }
-  uint64_t *d_arc_off = h->d_arc_off;
+  const uint64_t hub_end = h->hub_segs.empty() ? 0 : h->segs[h->hub_segs.back()].end;
+  const uint64_t np = full ? h->n_c : std::min<uint64_t>(h->n_c, hub_end + 32);
+  uint64_t *d_arc_off = nullptr;
   uint32_t *d_scratch = h->d_scratch, *d_rest = nullptr;
-  uint4 *d_pidx = h->d_pidx;
-  uint32_t *d_cursor = h->d_cursor;
+  uint4 *d_pidx = nullptr;
+  uint32_t *d_cursor = nullptr;
   try {
-    if (first) {
-      // + 4: a 16-byte-aligned bulk copy may read up to 12 bytes past the last label
-      d_scratch = dalloc<uint32_t>(h, h->streamed ? h->scratch_words : h->hub_arcs + 4, "two-pass scratch");
-      d_arc_off = dalloc<uint64_t>(h, h->n_c + 1, "arc offsets");
-      d_pidx = dalloc<uint4>(h, nc, "position index");
-      d_cursor = dalloc<uint32_t>(h, nc, "pre-pass cursors");
-    }
+    // + 4: a 16-byte-aligned bulk copy may read up to 12 bytes past the last label
+    if (first) d_scratch = dalloc<uint32_t>(h, h->streamed ? h->scratch_words : h->hub_arcs + 4, "two-pass scratch");
     if (full && !h->streamed) d_rest = dalloc<uint32_t>(h, off[h->n_c] - h->hub_arcs + 4, "two-pass scratch");
+    d_arc_off = dalloc<uint64_t>(h, np + 1, "arc offsets");
+    d_pidx = dalloc<uint4>(h, np, "position index");
+    d_cursor = dalloc<uint32_t>(h, np, "pre-pass cursors");
   } catch (const Fail &) {
-    if (first) {
-      dfree(h, d_scratch);
-      dfree(h, d_arc_off);
-      dfree(h, d_pidx);
-      dfree(h, d_cursor);
-    }
+    if (first) dfree(h, d_scratch);
+    dfree(h, d_rest);
+    dfree(h, d_arc_off);
+    dfree(h, d_pidx);
+    dfree(h, d_cursor);
     throw;
   }
-  std::vector<uint64_t> dev = off;
+  std::vector<uint64_t> dev(off.begin(), off.begin() + np + 1);
   if (d_rest) {
     // both allocations are 256-byte aligned, so indices keep their 16-byte alignment
     const uint64_t shift = uint64_t((reinterpret_cast<int64_t>(d_rest) - reinterpret_cast<int64_t>(d_scratch)) / 4);
     for (uint64_t p = 0; p < h->n_c; p++)
       if (off[p] >= h->hub_arcs) dev[p] = off[p] - h->hub_arcs + shift;
   }
+  dfree(h, h->d_arc_off);
+  dfree(h, h->d_pidx);
+  dfree(h, h->d_cursor);
   h->d_arc_off = d_arc_off;
   h->d_scratch = d_scratch;
   if (d_rest) h->d_scratch_rest = d_rest;
   h->d_pidx = d_pidx;
   h->d_cursor = d_cursor;
   h->scratch_scope = full ? 2 : 1;
-  h2d(h, h->d_arc_off, dev.data(), h->n_c + 1, "upload arc offsets");
+  h2d(h, h->d_arc_off, dev.data(), np + 1, "upload arc offsets");
   check(h, cudaStreamSynchronize(h->stream), "arc offsets");
-  if (!first) {
-    build_records(h, full);
-    return;
-  }
-  // where every compressed position's segments start, for the pre-pass
-  check(h, cudaMemsetAsync(h->d_cursor, 0, nc * sizeof(uint32_t), h->stream), "clear cursors");
+  // where every position's segments start, for the pre-pass
+  check(h, cudaMemsetAsync(h->d_cursor, 0, std::max<uint64_t>(1, np) * sizeof(uint32_t), h->stream), "clear cursors");
   if (h->streamed) {
     for (const StreamRange &r : h->ranges) {
-      if (r.p1 <= r.p0) continue;
+      const uint64_t p1 = std::min(r.p1, np);
+      if (p1 <= r.p0) continue;
       DevGraph g = dev_graph(h);
       g.words = stage_words(h, 0, r.w0, r.w1, h->stream);
-      const int blocks = int(std::min<uint64_t>((r.p1 - r.p0 + 127) / 128, uint64_t(h->num_sms) * 32));
-      k_pos_index<<<std::max(blocks, 1), 128, 0, h->stream>>>(g, h->d_pidx, h->d_err, r.p0, r.p1);
+      const int blocks = int(std::min<uint64_t>((p1 - r.p0 + 127) / 128, uint64_t(h->num_sms) * 32));
+      k_pos_index<<<std::max(blocks, 1), 128, 0, h->stream>>>(g, h->d_pidx, h->d_err, r.p0, p1);
       check(h, cudaGetLastError(), "position index launch");
       check(h, cudaStreamSynchronize(h->stream), "position index");  // the buffer is reused by the next range
     }
-  } else if (h->n_c) {
-    const int blocks = int(std::min<uint64_t>((h->n_c + 127) / 128, uint64_t(h->num_sms) * 32));
-    k_pos_index<<<std::max(blocks, 1), 128, 0, h->stream>>>(dev_graph(h), h->d_pidx, h->d_err, 0, h->n_c);
+  } else if (np) {
+    const int blocks = int(std::min<uint64_t>((np + 127) / 128, uint64_t(h->num_sms) * 32));
+    k_pos_index<<<std::max(blocks, 1), 128, 0, h->stream>>>(dev_graph(h), h->d_pidx, h->d_err, 0, np);
     check(h, cudaGetLastError(), "position index launch");
   }
   lpa_status st = take_device_error(h);

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -177,6 +178,7 @@ struct lpa_handle {
   uint64_t device_bytes = 0;
   char *d_csr_ws = nullptr;     // lpa_decode_csr's memory, kept by small handles
   std::vector<void *> allocations, slabs;
+  std::map<void *, uint64_t> alloc_bytes;  // of the allocations counted in device_bytes
   char *slab = nullptr;         // the rest of the last shared block
   uint64_t slab_left = 0;
 

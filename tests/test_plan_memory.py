@@ -164,3 +164,30 @@ def test_refused_graph_leaves_no_memory():
         assert e.value.status == L.Status.BAD_STREAM
         free.append(torch.cuda.mem_get_info(0)[0])
     assert free[0] - free[-1] < 4 << 20
+
+
+def test_position_arrays_end_at_the_last_hub():
+    """One hub, first in position order, among 200,000 compressed vertices: what the
+    two-pass kernels keep by position (28 bytes each) does not cover them all."""
+    n, d = 200000, 2000
+    v = np.arange(n)
+    lists = [np.arange(1, 1 + d)] + [np.array([x - 1]) for x in v[1:]]
+    row = np.concatenate([[0], np.cumsum([len(x) for x in lists])]).astype(np.uint64)
+    clm = np.concatenate(lists).astype(np.uint32)
+    hist, changed = oracle.lp_run(row, clm, 3, 0, 1)
+    g = L.HostGraph.from_csr(row, clm).compress(0, 128)
+    with refuse("two-pass scratch"):
+        with L.Propagator(g) as p:
+            without = p.get_info().device_bytes
+    for budget in (0, 1 << 20):
+        with L.Propagator(g, stream_budget=budget) as p:
+            if not budget:
+                assert p.get_info().device_bytes - without < 1 << 20
+            for it in range(3):
+                _check(p, hist, changed, it)
+            drow, dclm = p.decode_csr()  # of a streamed handle: needs every position's
+            assert np.array_equal(drow, row) and np.array_equal(dclm, clm)
+            p.set_dispatch(L.Dispatch.FORCE, L.Variant.TWO_PASS)
+            p.init_labels()
+            for it in range(3):
+                _check(p, hist, changed, it)
