@@ -27,6 +27,7 @@
 // zeroed stream.  Only the reference's parameters (zeta k = 3, intervals of
 // >= 4, 256-bit segments for both sections) are supported.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <cub/device/device_scan.cuh>
 
@@ -34,7 +35,6 @@
 #include <cstdint>
 #include <stdexcept>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "lpa/cgr_format.h"
@@ -423,27 +423,16 @@ struct DevBuf {
   DevBuf &operator=(const DevBuf &) = delete;
 };
 
-// v.resize(n) of an empty vector, its pages touched by several threads first:
-// a fresh page costs more than copying into it (45 MB of stream: 16 ms by one
-// thread).
+// v.resize(n) of an empty vector, in huge pages where the system has them: a
+// fresh page costs more than copying into it (45 MB of stream: 14 ms in 4 KB
+// pages, 6 in 2 MB ones, 7 in 4 KB pages touched by 16 threads).
 template <class T>
 void grow(std::vector<T> &v, size_t n) {
+  constexpr uintptr_t kHuge = 2u << 20;
   v.reserve(n);
-  char *p = reinterpret_cast<char *>(v.data());
-  const size_t bytes = n * sizeof(T), page = 4096;
-  const size_t nt = std::min<size_t>({16, std::max(1u, std::thread::hardware_concurrency()), bytes >> 21});
-  if (nt > 1) {
-    std::vector<std::thread> pool;
-    try {
-      for (size_t t = 0; t < nt; t++)
-        pool.emplace_back([=]() {
-          for (size_t i = bytes * t / nt; i < bytes * (t + 1) / nt; i += page)
-            *reinterpret_cast<volatile char *>(p + i) = 0;
-        });
-    } catch (...) {  // no more threads: resize touches what is left
-    }
-    for (auto &th : pool) th.join();
-  }
+  const uintptr_t p = reinterpret_cast<uintptr_t>(v.data());
+  const uintptr_t a = (p + kHuge - 1) & ~(kHuge - 1), e = (p + n * sizeof(T)) & ~(kHuge - 1);
+  if (e > a) madvise(reinterpret_cast<void *>(a), e - a, MADV_HUGEPAGE);  // advice: nothing to do when refused
   v.resize(n);
 }
 
