@@ -1831,7 +1831,9 @@ cudaError_t lpa_rt_launch_packed_loop(lpa_handle *h) {
   a.ktime = nullptr;
   a.seg_cycles = nullptr;
   const cudaError_t e =
-      launch_packed_loop(lpa_rt_packed_loop_grid(h), h->stream, a, reinterpret_cast<PackedLoop *>(h->d_loop_it));
+      refused("packed loop")
+          ? cudaErrorCooperativeLaunchTooLarge
+          : launch_packed_loop(lpa_rt_packed_loop_grid(h), h->stream, a, reinterpret_cast<PackedLoop *>(h->d_loop_it));
   if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs for this process than the device has
     cudaGetLastError();
     h->occ_packed_loop = 0;

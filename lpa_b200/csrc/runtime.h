@@ -237,7 +237,8 @@ void lpa_rt_enqueue_track(lpa_handle *h);
 bool lpa_rt_install_plan(lpa_handle *h, const std::vector<uint8_t> &variant);
 void lpa_rt_ensure_lists(lpa_handle *h);
 // For tests: from now on the calling thread's device allocations of this name
-// fail as if the device had no memory left (nullptr: none).
+// fail as if the device had no memory left, and "packed loop" as if its grid
+// did not fit (nullptr: none).
 extern "C" void lpa_test_refuse(const char *what);
 // For tests: the handle's PackedLoop::wait_ns.
 extern "C" void lpa_test_loop_wait(lpa_handle *h, uint64_t ns);
