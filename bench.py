@@ -649,7 +649,7 @@ def main():
     ms_per_step = total_ms / args.steps
 
     # roofline of one iteration: its kernels (two-pass decode, two-pass
-    # count, persistent iteration kernel) together read the compressed graph
+    # count, lane, warp and block kernels) together read the compressed graph
     # and the labels and write the labels once; the algorithmic bytes of the
     # iteration over its device time
     kern_avg = kern_ms / args.steps
@@ -699,14 +699,14 @@ def main():
                        "l2": "L2 flushed between iterations" if flush else "inputs larger than L2",
                        "parallelism": f"replicas x{world}"},
             "roofline": {"bound": "hbm",
-                         "kernel": "iteration (k_decode_two_pass + k_count_two_pass + k_packed + k_iterate)",
+                         "kernel": "iteration (k_decode_two_pass + k_count_two_pass + k_packed + k_light + k_iterate)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": peak_kind,
                          "bytes_per_launch": b_alg, "ms_per_launch": ms_per_step,
                          "traffic": traffic_summary(args.workload),
                          "kernel_ms": None if loop == "graph" else
                          {"k_decode_two_pass": float(kern_avg[0]), "k_count_two_pass": float(kern_avg[1]),
-                          "k_packed": float(kern_avg[2]), "k_iterate": float(kern_avg[3])}},
+                          "k_packed": float(kern_avg[2]), "k_light + k_iterate": float(kern_avg[3])}},
             "dispatch": {"mode": args.dispatch,
                          "fixed_value": arcs * args.steps * world / (fixed_ms / 1e3),
                          "fixed_ms_per_step": fixed_ms / args.steps,

@@ -131,7 +131,7 @@ typedef struct lpa_stats {
   int learned_active;               /* 1 when the learned plan is in use */
   uint64_t launches;                /* kernel launches enqueued by this handle */
   double decode_ms;                 /* two-pass decode kernel, last iteration */
-  double iterate_ms;                /* persistent iteration kernel, last iteration */
+  double iterate_ms;                /* block and warp kernels (k_iterate, k_light), last iteration */
   double count_ms;                  /* two-pass count kernel, last iteration */
   double packed_ms;                 /* lane-per-vertex kernel of the tiny bucket, last iteration */
   uint64_t stream_ranges;           /* out-of-core streaming: ranges per iteration (0: resident) */
@@ -222,7 +222,8 @@ typedef struct lpa_tune {
                                 0 (default) not at all (per-lane loads); 1 a bulk prefetch of the next
                                 group's span into L2; 2 a bulk copy of the next group's span into one of
                                 the warp's two shared-memory buffers (mbarrier-completed), overlapping the
-                                current group's decode */
+                                current group's decode.  On resident handles the groups are the interval
+                                segments only; the residual segments have records and read the stream */
 } lpa_tune;
 lpa_status lpa_get_tune(struct lpa_handle *h, lpa_tune *out);
 /* Installs the knobs (out of range: LPA_ERR_INVALID_ARG) and rebuilds the work lists. */

@@ -75,13 +75,6 @@ struct StagedWords {
   }
 };
 
-// Shared-memory word source: words [base_word, base_word + len) staged at s.
-struct SWords {
-  const uint32_t *s;
-  uint64_t base_word;
-  __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return s[i - base_word]; }
-};
-
 // gamma (graph_utils.cuh:63-67): z zeros, then the z+1 bits of x+1.
 template <class W>
 __device__ __forceinline__ uint32_t dec_gamma(W w, uint64_t &pos, bool &bad) {
@@ -575,8 +568,6 @@ __device__ __forceinline__ uint32_t warp_mode(const uint32_t *lab, uint32_t d) {
 __device__ __forceinline__ bool one_by_one(uint32_t lists, uint32_t dmax) {
   return lists * 128u < dmax * (dmax + 16u);
 }
-
-__device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
 // The GPU's nanosecond clock (the same for every SM).
 __device__ __forceinline__ unsigned long long global_ns() {

@@ -48,7 +48,9 @@ constexpr float kLr = 3e-3f;
 // predicted cheaper by more than this (log2 cost / 32: 1.6 times the cost).
 // Per-segment costs do not see what running one more kernel takes: on a road
 // grid joined with R-MAT scale 18 the plain argmin left the R-MAT graph's large
-// segments, a few percent apart, on k_iterate, 268 us per iteration against 204.
+// segments, a few percent apart, on k_light, 268 us per iteration against 204.
+// On single graphs (road grids, R-MAT scale 14 to 22, copy models) the plan and
+// the time are the same without it: the merged candidate wins there.
 constexpr float kTwoPassMargin = 0.02f;
 
 __device__ __forceinline__ uint32_t mix32(uint32_t x) {

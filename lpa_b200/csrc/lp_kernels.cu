@@ -1246,8 +1246,8 @@ __device__ __forceinline__ uint32_t packed_vertex(const IterArgs &a, const Ctx &
 }
 
 // V2 (several vertices per warp) at its limit for the tiny bucket: one lane
-// per position (packed_vertex), 32 vertices per warp.  No shared memory, no
-// warp-wide steps.
+// per position (packed_vertex), 32 vertices per warp; the lanes share nothing
+// but the count of changed labels.
 __global__ void __launch_bounds__(kThreads) k_packed(IterArgs a) {
   // per thread kPackedMaxDeg label slots: a per-thread array indexed at run
   // time would live in local memory
@@ -1473,8 +1473,13 @@ __device__ __forceinline__ void decode_records(const IterArgs &a, const Ctx &c, 
   }
 }
 
-// Two-pass variant, pass 1.  Every 256-bit segment of the two-pass positions
-// is decoded by one lane, which writes the labels of its ids (not the ids) to
+// Two-pass variant, pass 1, in two parts: decode groups, then record groups
+// (decode_records).  Where the handle has segment records those take the
+// residual segments and the decode groups the interval segments alone; without
+// them (streamed handles, no memory for the records, streams or scratches beyond
+// a record's fields) the decode groups take both.
+//
+// Decode groups: every 256-bit segment is decoded by one lane, which writes the labels of its ids (not the ids) to
 // the scratch, so pass 2 only counts.  A warp takes one decode group (32
 // segments) at a time from the iteration's work queue (IterArgs::work slot
 // kWqGroups, zeroed before the launch).  Lane l finds its position with a warp scan of the positions'
@@ -1500,7 +1505,11 @@ __device__ __forceinline__ void decode_records(const IterArgs &a, const Ctx &c, 
 // multicast), completed on that buffer's mbarrier with a bounded wait, so the
 // copy of group k + 1 overlaps the decode of group k; the lanes then read
 // their words from the buffer (words outside the copied span, if any, from
-// the stream itself).
+// the stream itself).  Record groups read the stream directly; a group of
+// interval segments alone has the residual segments between them in its span,
+// so with records the knob moves words that no lane reads: an iteration at R-MAT
+// scale 22 takes 1055 / 1094 / 1364 us with 0 / 1 / 2, of a 4M-vertex copy
+// model 691 / 737 / 1073, at scale 14 to 20 the same with 0 and 1 within 2 %.
 //
 // kPack (n <= 2^27, unstaged forms): a staged id carries its lane in its top
 // 5 bits, so the window needs no owner bytes (one shared store per id fewer:
@@ -2050,8 +2059,8 @@ __device__ __forceinline__ uint64_t block_max_u64(uint64_t v, uint64_t *red) {
 // degrees up to kCountBlockMax in a 4096-slot block table, or the sketch;
 // the warps stream disjoint 256-label blocks of the vertex.  Warp items: up
 // to 4 (tunable) positions of degree <= kCountWarpMax, one vertex at a time in the
-// warp's 512-slot table, or up to 32 positions of degree <= 32 on G-lane
-// groups.  The same shared memory serves the warp tables, the block table
+// warp's 512-slot table, or up to 32 positions of degree <= 32, a lane each
+// (few left to count: the warp one by one).  The same shared memory serves the warp tables, the block table
 // (block epochs, disjoint from the warps') and the sketch (cleared before and
 // after use).  Every position's pre-pass cursor is reset here.
 // kHash: the plan has kCountHash items (the call in the item loop costs the

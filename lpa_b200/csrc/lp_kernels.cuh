@@ -103,7 +103,7 @@ constexpr uint32_t kSpanSmemBytes = kWarps * 2 * kSpanWords * 4;  // its two buf
 // p0 + np - 1, all of one kind, whose labels the pre-pass wrote to the
 // scratch.  seg is the plan segment the cycles are booked to.
 enum CountKind : uint32_t {
-  kCountGroups = 0,  // np <= 32 positions of degree <= 32: G-lane groups, several vertices per round
+  kCountGroups = 0,  // np <= 32 positions of degree <= 32: a lane per vertex
   kCountWarp = 1,    // np <= 4 positions of degree <= kCountWarpMax: warp per vertex, 512-slot table
   kCountBlock = 2,   // one position, degree <= kCountBlockMax: block per vertex, 4096-slot table
   kCountSketch = 3,  // one position at or above the sketch threshold: block per vertex

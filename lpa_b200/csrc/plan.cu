@@ -1,7 +1,7 @@
 // Work lists of a plan, built on the device.
 //
 // A plan (one kernel variant per segment) becomes the kernels' work lists:
-// k_iterate's heavy and light items, k_packed's chunks, the two-pass
+// k_iterate's heavy items, k_light's items, k_packed's chunks, the two-pass
 // pre-pass's decode groups and the count pass's block, warp and group items
 // (lp_kernels.cuh).  Building them is a walk over every segment's positions.
 // Here one thread walks one segment (at most 256 positions, or one hub), twice:
@@ -110,7 +110,7 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
   const uint32_t cms = a.cms;
   const bool tp = v == kVarTwoPass;
   // a block-variant segment whose vertices one warp holds runs as warp
-  // chunks (one vertex per warp at a time, k_iterate's light loop) instead of
+  // chunks (one vertex per warp at a time, k_light) instead of
   // one vertex per block: its vertices have at most 64 segments of 256 bits,
   // too few to keep a block busy, and block items wait at barriers
   const bool block = (v == kVarBlock || tp) && !warp_capable(si, cms);

@@ -1083,7 +1083,7 @@ static void collect_times(lpa_handle *h) {
     return double(t);
   };
   for (int v = 0; v < 4; v++) h->variant_ms[v] = 0;
-  double k_ms[4] = {0, 0, 0, 0};  // pre-pass, count pass, k_packed, k_iterate
+  double k_ms[4] = {0, 0, 0, 0};  // pre-pass, count pass, k_packed, k_light and k_iterate
   for (int e = 1; e < h->ev_used; e++)
     if (h->ev_kernel[e] >= 0 && h->ev_kernel[e] < 4) k_ms[h->ev_kernel[e]] = ms(e - 1, e);
   h->decode_ms = k_ms[0];

@@ -172,7 +172,7 @@ struct lpa_handle {
   double decode_ms = 0, iterate_ms = 0, count_ms = 0, packed_ms = 0;
   bool collect_cycles = false;  // per-segment cycles for the cost model
   cudaEvent_t ev[5] = {};  // iteration start, then one after each kernel that ran
-  int ev_kernel[5] = {};   // which kernel each event follows (0 pre-pass, 1 count, 2 k_packed, 3 k_iterate)
+  int ev_kernel[5] = {};   // which kernel each event follows (0 pre-pass, 1 count, 2 k_packed, 3 k_light and k_iterate)
   int ev_used = 0;
   bool events_ready = false;
   uint64_t device_bytes = 0;
