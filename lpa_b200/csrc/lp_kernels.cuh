@@ -107,7 +107,7 @@ enum CountKind : uint32_t {
   kCountWarp = 1,    // np <= 4 positions of degree <= kCountWarpMax: warp per vertex, 512-slot table
   kCountBlock = 2,   // one position, degree <= kCountBlockMax: block per vertex, 4096-slot table
   kCountSketch = 3,  // one position at or above the sketch threshold: block per vertex
-  kCountHash = 4,    // one position, exact, degree <= kCountHashMax: a block per share of the labels' hashes
+  kCountHash = 4,    // one position, exact, degree <= PlanInputs::hash_max: a block per share of the labels' hashes
 };
 struct CountItem {
   uint32_t p0, np, seg, kind;
@@ -129,6 +129,24 @@ struct BlockItem {
 constexpr uint32_t kCountHashLoad = 2048;
 constexpr uint32_t kCountHashMaxLog = 12;
 constexpr uint64_t kCountHashMax = uint64_t(kCountHashLoad) << kCountHashMaxLog;
+// log2 of the shares of an exact vertex of degree d.
+__host__ __device__ inline uint32_t hash_share_log(uint32_t d) {
+  uint32_t lg = 1;
+  while ((uint64_t(kCountHashLoad) << lg) < d) lg++;
+  return lg;
+}
+// Shares read a vertex's labels once each, so their work grows with the square
+// of the degree, where a table in global memory (k_iterate, one block a vertex)
+// reads them once: the shares win by their blocks until a graph has many
+// vertices of several 100,000 neighbours.  100 of degree 1M: 60 to 70 ms in
+// shares, 6 (all labels equal) / 10 (zipf) / 38 (all different) in tables;
+// 300 of 300,000: 28 to 35 against 5.5 / 9.9 / 38; 1000 of 100,000: 8.4 / 9.3
+// / 23 against 3.0 / 8.4 / 27; 10 of 1M: 6.7 to 8 against 6.2 / 8.6 / 22.
+// hash_share_limit (runtime.cu) weighs the two with these rates, in ns a label:
+constexpr double kShareNs = 1.17e-3;      // a label read by one share, the whole GPU on it
+constexpr double kTableLatencyNs = 8.0;   // a label counted by one block
+constexpr double kTableNs = 0.1;          // a label, all blocks counting
+constexpr double kTableMargin = 1.5;      // the tables have to be faster by this
 struct HashSlot {
   unsigned long long best;  // pack_best over the finished shares
   uint32_t done, pad;       // finished shares

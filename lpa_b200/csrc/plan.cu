@@ -49,6 +49,7 @@ struct PlanArgs {
   const uint32_t *words, *small_nbr, *scratch;
   uint64_t n, n_c;
   uint32_t cms, wmax, warp_positions, group_positions;
+  uint64_t hash_max;
   uint64_t c_begin, c_end, s_begin, s_end;  // positions of the group items (compressed, small CSR)
   uint64_t win0;             // windows of the compressed positions; the rest cover the small CSR
   const uint32_t *off;       // kLists x (nseg + 1) exclusive offsets, by segment - seg_begin
@@ -117,7 +118,7 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
   bool counted = tp;  // the two-pass count pass takes the segment's positions
   if (tp) {
     // exact above the count pass's reach (a hub is alone in its segment)
-    if (si.max_deg > kCountHashMax && (cms == 0 || si.max_deg < cms)) counted = false;
+    if (si.max_deg > a.hash_max && (cms == 0 || si.max_deg < cms)) counted = false;
     // the small CSR is counted by warp and group items only
     if (si.region == 1 && ((cms != 0 && si.max_deg >= cms) || si.max_deg > a.wmax)) counted = false;
   }
@@ -131,8 +132,7 @@ __device__ void plan_segment(const PlanArgs &a, uint32_t i) {
       const uint32_t d = a.deg[p];
       const bool sk = cms != 0 && d >= cms;
       if (!sk && d > kCountBlockMax) {
-        uint32_t lg = 1;
-        while ((uint64_t(kCountHashLoad) << lg) < d) lg++;
+        const uint32_t lg = hash_share_log(d);
         if (kEmit) {
           for (uint32_t k = 0; k < 1u << lg; k++) {
             const uint32_t at = o[kLBlock] + c[kLBlock] + k;
@@ -421,6 +421,7 @@ cudaError_t PlanBuilder::build(const PlanInputs &in, PlanOutputs &out, cudaStrea
   a.n = in.n;
   a.n_c = in.n_c;
   a.cms = in.cms;
+  a.hash_max = in.hash_max;
   a.wmax = in.wmax;
   a.warp_positions = in.warp_positions;
   a.group_positions = uint32_t(G);

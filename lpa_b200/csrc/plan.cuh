@@ -40,6 +40,7 @@ struct PlanInputs {
   uint32_t wmax;             // lpa_tune.warp_max_degree
   uint32_t warp_positions;   // lpa_tune.warp_positions
   uint32_t group_positions;  // lpa_tune.group_positions
+  uint64_t hash_max;         // largest exact degree counted in hash shares
   int num_sms;
 };
 

@@ -223,6 +223,13 @@ bool variant_capable(int v, const SegInfo &s, uint32_t cms_thr) {
   }
 }
 
+// Global count tables of 2 GiB for vertices of up to max_deg neighbours, at most
+// one per block.
+static int count_tables(uint32_t max_deg, int blocks) {
+  const uint64_t table = uint64_t(next_pow2_host(2 * uint64_t(max_deg))) * 2 * sizeof(uint32_t);
+  return int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(blocks), (2ull << 30) / table)));
+}
+
 // The reference's degree buckets: <16 packed warp, <128 warp, >=128 block
 // (baselines/novaplus/novaplus_propogator.cuh:219-220, include/decoder.cuh:50-58).
 int fixed_variant(const SegInfo &s) {
@@ -234,6 +241,38 @@ int fixed_variant(const SegInfo &s) {
     default:
       return LPA_VARIANT_BLOCK;
   }
+}
+
+// Degrees above the limit go to the tables, the others to hash shares: the
+// largest degrees first, as many as make the sum of both the least (the shares'
+// and the tables' kernels run one after the other).
+uint64_t hash_share_limit(std::vector<uint32_t> deg, int blocks) {
+  std::sort(deg.begin(), deg.end(), std::greater<uint32_t>());
+  const auto share_ns = [](uint32_t d) { return double(d) * double(1u << hash_share_log(d)) * kShareNs; };
+  size_t k0 = 0;  // beyond the shares' reach whatever they cost
+  while (k0 < deg.size() && deg[k0] > kCountHashMax) k0++;
+  double rest = 0;
+  for (size_t i = k0; i < deg.size(); i++) rest += share_ns(deg[i]);
+  double table = 0, best = 0, none = 0;  // table: labels in the tables
+  for (size_t i = 0; i < k0; i++) table += deg[i];
+  size_t best_k = k0;
+  for (size_t k = k0;; k++) {
+    if (k == k0 || k == deg.size() || deg[k] != deg[k - 1]) {
+      const double at = k ? double(std::min(blocks, count_tables(deg[0], blocks))) : 1.0;
+      const double ns =
+          rest + (k ? std::max(kTableLatencyNs * deg[0], table * std::max(kTableNs, kTableLatencyNs / at)) : 0.0);
+      if (k == k0) best = none = ns;
+      if (ns < best) {
+        best = ns;
+        best_k = k;
+      }
+    }
+    if (k == deg.size()) break;
+    table += deg[k];
+    rest -= share_ns(deg[k]);
+  }
+  if (best * kTableMargin > none) best_k = k0;
+  return best_k == k0 ? kCountHashMax : best_k == deg.size() ? uint64_t(kCountBlockMax) : uint64_t(deg[best_k]);
 }
 
 }  // namespace lpa_rt
@@ -297,7 +336,7 @@ static void ensure_gtab(lpa_handle *h, uint32_t max_deg) {
   if (!h->d_gtab || slots > h->gtab_slots) {
     dfree(h, h->d_gtab);
     const uint64_t per_block = uint64_t(slots) * 2 * sizeof(uint32_t);
-    const int blocks = int(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(h->grid), (2ull << 30) / per_block)));
+    const int blocks = count_tables(max_deg, h->grid);
     h->d_gtab = dalloc<uint32_t>(h, uint64_t(blocks) * 2 * slots, "global count tables");
     h->gtab_slots = slots;
     h->gtab_blocks = blocks;
@@ -356,6 +395,7 @@ static void upload_lists(lpa_handle *h) {
   in.warp_positions = h->tune.warp_positions;
   in.group_positions = h->tune.group_positions;
   in.num_sms = h->num_sms;
+  in.hash_max = h->hash_max;
   auto regrow = [&](auto *&ptr, size_t &cap, size_t need, const char *what) {
     if (need <= cap && ptr) return;
     dfree(h, ptr);
@@ -436,6 +476,7 @@ static void upload_range_lists(lpa_handle *h) {
     in.warp_positions = h->tune.warp_positions;
     in.group_positions = h->tune.group_positions;
     in.num_sms = h->num_sms;
+  in.hash_max = h->hash_max;
     PlanOutputs out{};
     out.grow = [&](PlanOutputs &o) -> cudaError_t {
       regrow(r.items, r.items_cap, size_t(o.n_heavy) + o.n_light, "range work items");
@@ -662,7 +703,14 @@ static void apply_run_variants(lpa_handle *h) {
 static void rebuild_lists(lpa_handle *h) {
   drop_lists(h);
   apply_run_variants(h);
-  upload_lists(h);
+  try {
+    upload_lists(h);
+  } catch (const Fail &f) {
+    if (f.st != LPA_ERR_OOM || h->hash_max == kCountHashMax) throw;
+    h->hash_max = kCountHashMax;  // the shares need no tables
+    drop_lists(h);
+    upload_lists(h);
+  }
   h->plan_ready = true;
 }
 
@@ -826,6 +874,12 @@ static void build_plan(lpa_handle *h) {
   // (1.5M segments, R-MAT scale 24)
   for (size_t s = 0; s < h->segs.size() && h->segs[s].region == 0; s++)
     if (h->segs[s].bucket == kHeavy) h->hub_segs.push_back(uint32_t(s));
+  std::vector<uint32_t> exact;
+  for (const uint32_t s : h->hub_segs) {
+    const uint32_t d = h->segs[s].max_deg;
+    if (d > kCountBlockMax && (h->opts.cms_threshold == 0 || d < h->opts.cms_threshold)) exact.push_back(d);
+  }
+  h->hash_max = hash_share_limit(std::move(exact), h->num_sms * h->occ);
   if (h->streamed) build_ranges(h);
   h->fixed.resize(h->segs.size());
   for (size_t s = 0; s < h->segs.size(); s++) h->fixed[s] = uint8_t(fixed_variant(h->segs[s]));
@@ -1850,6 +1904,9 @@ bool lpa_rt_install_plan(lpa_handle *h, const std::vector<uint8_t> &variant) {
   return true;
 }
 void lpa_rt_ensure_lists(lpa_handle *h) { ensure_lists(h); }
+extern "C" uint64_t lpa_test_hash_share_limit(const uint32_t *deg, size_t n, int blocks) {
+  return hash_share_limit(std::vector<uint32_t>(deg, deg + n), blocks);
+}
 extern "C" void lpa_test_loop_wait(lpa_handle *h, uint64_t ns) { h->loop_wait_ns = ns; }
 extern "C" void lpa_test_refuse(const char *what) { refused_name = what ? what : ""; }
 lpa_status lpa_rt_take_error(lpa_handle *h) { return take_device_error(h); }

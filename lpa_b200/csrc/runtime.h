@@ -42,6 +42,9 @@ inline uint32_t next_pow2_host(uint64_t x) {
 
 bool variant_capable(int variant, const SegInfo &s, uint32_t cms_thr);
 int fixed_variant(const SegInfo &s);
+// The largest degree to count in hash shares, for a graph's exact vertices above
+// the count pass's block table and k_iterate's blocks.
+uint64_t hash_share_limit(std::vector<uint32_t> deg, int blocks);
 // Segment cutting limits: positions per bucket, and arcs.
 struct SegLimits {
   uint32_t positions[kNumBuckets];
@@ -102,6 +105,7 @@ struct lpa_handle {
   // plan
   std::vector<uint32_t> h_deg;
   std::vector<lpa_rt::SegInfo> segs;
+  uint64_t hash_max = 0;           // hash_share_limit of the graph
   std::vector<uint32_t> hub_segs;  // the heavy bucket's segments of the compressed region
   std::vector<uint8_t> variant;  // per segment
   std::vector<uint8_t> run_variant;          // what the kernels run for it (apply_run_variants)
@@ -240,6 +244,7 @@ void lpa_rt_ensure_lists(lpa_handle *h);
 // fail as if the device had no memory left, and "packed loop" as if its grid
 // did not fit (nullptr: none).
 extern "C" void lpa_test_refuse(const char *what);
+extern "C" uint64_t lpa_test_hash_share_limit(const uint32_t *deg, size_t n, int blocks);  // hash_share_limit
 // For tests: the handle's PackedLoop::wait_ns.
 extern "C" void lpa_test_loop_wait(lpa_handle *h, uint64_t ns);
 constexpr int kPinnedSlots = 128;  // 64-bit words of lpa_handle::h_pinned
