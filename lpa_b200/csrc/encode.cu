@@ -33,6 +33,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <numeric>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -412,27 +413,54 @@ void ck(cudaError_t e, const char *what) {
   }
 }
 
-template <class T>
-struct DevBuf {
-  T *p = nullptr;
-  explicit DevBuf(size_t n) { ck(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)), "cudaMalloc"); }
-  ~DevBuf() {
-    if (p) cudaFree(p);
+// Device arrays of one call, those added between two alloc()s in one allocation
+// (400 us each above 1 MB, whatever the size).
+class DevArrays {
+ public:
+  DevArrays() = default;
+  DevArrays(const DevArrays &) = delete;
+  DevArrays &operator=(const DevArrays &) = delete;
+  ~DevArrays() {
+    for (char *p : blocks_)
+      if (p) cudaFree(p);
   }
-  DevBuf(const DevBuf &) = delete;
-  DevBuf &operator=(const DevBuf &) = delete;
+  template <class T>
+  void add(T **p, size_t count) {
+    want_.push_back({reinterpret_cast<void **>(p), total_});
+    total_ += (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~size_t(255);
+  }
+  void alloc() {
+    blocks_.push_back(nullptr);
+    ck(cudaMalloc(&blocks_.back(), total_), "cudaMalloc");
+    for (const Want &w : want_) *w.p = blocks_.back() + w.at;
+    want_.clear();
+    total_ = 0;
+  }
+
+ private:
+  struct Want {
+    void **p;
+    size_t at;
+  };
+  std::vector<Want> want_;
+  std::vector<char *> blocks_;
+  size_t total_ = 0;
 };
 
-// v.resize(n) of an empty vector, in huge pages where the system has them: a
-// fresh page costs more than copying into it (45 MB of stream: 14 ms in 4 KB
-// pages, 6 in 2 MB ones, 7 in 4 KB pages touched by 16 threads).
+// Storage for n elements of an empty vector, in huge pages where the system has
+// them: a fresh page costs more than copying into it (45 MB of stream: 14 ms in
+// 4 KB pages, 6 in 2 MB ones, 7 in 4 KB pages touched by 16 threads).
 template <class T>
-void grow(std::vector<T> &v, size_t n) {
+void in_huge_pages(std::vector<T> &v, size_t n) {
   constexpr uintptr_t kHuge = 2u << 20;
   v.reserve(n);
   const uintptr_t p = reinterpret_cast<uintptr_t>(v.data());
   const uintptr_t a = (p + kHuge - 1) & ~(kHuge - 1), e = (p + n * sizeof(T)) & ~(kHuge - 1);
   if (e > a) madvise(reinterpret_cast<void *>(a), e - a, MADV_HUGEPAGE);  // advice: nothing to do when refused
+}
+template <class T>
+void grow(std::vector<T> &v, size_t n) {
+  in_huge_pages(v, n);
   v.resize(n);
 }
 
@@ -458,112 +486,121 @@ void cgr_encode_gpu(const CsrView &g, const CgrParams &p, int small_thresh, int 
   ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "attribute");
   const int wide = sms * 8;
 
-  // the CSR on the device, once, for both the encoder and the small CSR
-  // few allocations: what n and m size, what n_c sizes, the stream, the small CSR
-  size_t total = 0;
-  const auto piece = [&total](size_t bytes) {
-    const size_t at = total;
-    total += (bytes + 255) & ~size_t(255);
-    return at;
-  };
+  // position order: large by id, mid by id, small by id (as the host encoder)
+  DevArrays mem;
+  uint64_t *d_row, *d_class;
+  uint32_t *d_vert;
+  char *d_scan;
   size_t scan_bytes = 0;  // of the longest scan, over n + 1
   ck(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, static_cast<uint64_t *>(nullptr), static_cast<uint64_t *>(nullptr),
                                    n + 1), "scan");
-  const size_t o_row = piece((n + 1) * 8), o_clm = piece(m * 4), o_class = piece((n + 1) * 8), o_vert = piece(n * 4),
-               o_scan = piece(scan_bytes);
-  DevBuf<char> mem_n(total);
-  struct { uint64_t *p; } d_row{reinterpret_cast<uint64_t *>(mem_n.p + o_row)},
-      d_class{reinterpret_cast<uint64_t *>(mem_n.p + o_class)};
-  struct { uint32_t *p; } d_clm{reinterpret_cast<uint32_t *>(mem_n.p + o_clm)},
-      d_vert{reinterpret_cast<uint32_t *>(mem_n.p + o_vert)};
-  ck(cudaMemcpy(d_row.p, g.row, (n + 1) * 8, cudaMemcpyHostToDevice), "upload row");
-  if (m) ck(cudaMemcpy(d_clm.p, g.clm, m * 4, cudaMemcpyHostToDevice), "upload clm");
-
-  // position order: large by id, mid by id, small by id (as the host encoder)
+  mem.add(&d_row, n + 1);
+  mem.add(&d_class, n + 1);
+  mem.add(&d_vert, n);
+  mem.add(&d_scan, scan_bytes);
+  mem.alloc();
+  ck(cudaMemcpy(d_row, g.row, (n + 1) * 8, cudaMemcpyHostToDevice), "upload row");
   auto scan = [&](uint64_t *data, uint64_t count) {  // exclusive, in place; count <= n + 1
     size_t bytes = 0;
     ck(cub::DeviceScan::ExclusiveSum(nullptr, bytes, data, data, count), "scan");
     if (bytes > scan_bytes) throw std::runtime_error("cgr_encode_gpu: scan memory");
-    ck(cub::DeviceScan::ExclusiveSum(mem_n.p + o_scan, bytes, data, data, count), "scan");
+    ck(cub::DeviceScan::ExclusiveSum(d_scan, bytes, data, data, count), "scan");
   };
+  k_class<<<wide, 256>>>(d_row, n, uint64_t(large_thresh), uint64_t(small_thresh), d_class);
+  ck(cudaGetLastError(), "position order");
+  scan(d_class, n + 1);
   uint64_t num = 0;
-  {
-    k_class<<<wide, 256>>>(d_row.p, n, uint64_t(large_thresh), uint64_t(small_thresh), d_class.p);
-    ck(cudaGetLastError(), "position order");
-    scan(d_class.p, n + 1);
-    k_place<<<wide, 256>>>(d_row.p, n, uint64_t(large_thresh), uint64_t(small_thresh), d_class.p, d_vert.p);
-    ck(cudaGetLastError(), "position order");
-    ck(cudaMemcpy(&num, d_class.p + n, 8, cudaMemcpyDeviceToHost), "class sizes");
-  }
+  ck(cudaMemcpy(&num, d_class + n, 8, cudaMemcpyDeviceToHost), "class sizes");
   out.n_large = num >> 32;
   const uint64_t n_c = out.n_c = out.n_large + (num & 0xFFFFFFFFull), ns = n - n_c;
-  const uint32_t *d_small = d_vert.p + n_c;
+  if (n_c == 0) {
+    // nothing to compress: the small CSR is the graph (road grid 300^2 with
+    // threshold 16: 2.5 ms by the passes below, 0.9 ms here)
+    if (m > 0xFFFFFFFFull) throw std::invalid_argument("cgr_encode_gpu: small CSR exceeds 2^32 arcs");
+    out.offsets.assign(1, 0);
+    out.words.assign(4, 0u);
+    if (n == 0) return;
+    grow(out.vertices, n);
+    std::iota(out.vertices.begin(), out.vertices.end(), 0u);
+    grow(out.small_offset, n + 1);
+    for (uint64_t v = 0; v <= n; v++) out.small_offset[v] = uint32_t(g.row[v] - g.row[0]);
+    in_huge_pages(out.small_graph, m);
+    out.small_graph.assign(g.clm + g.row[0], g.clm + m);
+    return;
+  }
+  k_place<<<wide, 256>>>(d_row, n, uint64_t(large_thresh), uint64_t(small_thresh), d_class, d_vert);
+  ck(cudaGetLastError(), "position order");
+  const uint32_t *d_small = d_vert + n_c;
 
   // d_bits: the bit lengths, then their sums, the offsets
-  total = 0;
-  const size_t o_ctr = piece(2 * 8 + 4), o_bits = piece((n_c + 1) * 8), o_itv = piece(n_c * 8), o_nsi = piece(n_c * 4),
-               o_nsr = piece(n_c * 4), o_nres = piece(n_c * 4), o_nitv = piece(n_c * 4), o_work = piece(n_c ? m * 4 : 0),
-               o_so64 = piece((ns + 1) * 8), o_so = piece((ns + 1) * 4);
-  DevBuf<char> mem_c(total);
-  struct { uint64_t *p; } d_bits{reinterpret_cast<uint64_t *>(mem_c.p + o_bits)},
-      d_itv{reinterpret_cast<uint64_t *>(mem_c.p + o_itv)}, d_so64{reinterpret_cast<uint64_t *>(mem_c.p + o_so64)};
-  struct { uint32_t *p; } d_nsi{reinterpret_cast<uint32_t *>(mem_c.p + o_nsi)},
-      d_nsr{reinterpret_cast<uint32_t *>(mem_c.p + o_nsr)}, d_nres{reinterpret_cast<uint32_t *>(mem_c.p + o_nres)},
-      d_nitv{reinterpret_cast<uint32_t *>(mem_c.p + o_nitv)}, d_work{reinterpret_cast<uint32_t *>(mem_c.p + o_work)},
-      d_so{reinterpret_cast<uint32_t *>(mem_c.p + o_so)}, d_err{reinterpret_cast<uint32_t *>(mem_c.p + o_ctr + 16)};
-  struct { unsigned long long *p; } d_ctr{reinterpret_cast<unsigned long long *>(mem_c.p + o_ctr)};  // one per pass
-  ck(cudaMemset(d_ctr.p, 0, 16), "clear work counters");
-  ck(cudaMemset(d_err.p, 0, 4), "clear error");
-  EncodeArgs ea{d_row.p, d_clm.p, d_vert.p, d_work.p, n_c, out.n_large, d_bits.p, d_itv.p,
-                d_nsi.p, d_nsr.p, d_nres.p, d_nitv.p, d_ctr.p, d_err.p};
-  const int blocks = int(std::max<uint64_t>(1, std::min<uint64_t>((n_c + kEncWarps - 1) / kEncWarps, uint64_t(wide))));
-  if (n_c) k_encode_size<<<blocks, kEncThreads>>>(ea);
+  uint32_t *d_clm, *d_work, *d_nsi, *d_nsr, *d_nres, *d_nitv, *d_so, *d_err;
+  uint64_t *d_bits, *d_itv, *d_so64;
+  unsigned long long *d_ctr;  // one per pass
+  mem.add(&d_clm, m);
+  mem.add(&d_work, m);
+  mem.add(&d_bits, n_c + 1);
+  mem.add(&d_itv, n_c);
+  mem.add(&d_nsi, n_c);
+  mem.add(&d_nsr, n_c);
+  mem.add(&d_nres, n_c);
+  mem.add(&d_nitv, n_c);
+  mem.add(&d_so64, ns + 1);
+  mem.add(&d_so, ns + 1);
+  mem.add(&d_ctr, 2);
+  mem.add(&d_err, 1);
+  mem.alloc();
+  if (m) ck(cudaMemcpy(d_clm, g.clm, m * 4, cudaMemcpyHostToDevice), "upload clm");
+  ck(cudaMemset(d_ctr, 0, 16), "clear work counters");
+  ck(cudaMemset(d_err, 0, 4), "clear error");
+  EncodeArgs ea{d_row, d_clm, d_vert, d_work, n_c, out.n_large, d_bits, d_itv,
+                d_nsi, d_nsr, d_nres, d_nitv, d_ctr, d_err};
+  const int blocks = int(std::min<uint64_t>((n_c + kEncWarps - 1) / kEncWarps, uint64_t(wide)));
+  k_encode_size<<<blocks, kEncThreads>>>(ea);
   ck(cudaGetLastError(), "size pass");
   grow(out.vertices, n);
-  if (n) ck(cudaMemcpy(out.vertices.data(), d_vert.p, n * 4, cudaMemcpyDeviceToHost), "read positions");
+  ck(cudaMemcpy(out.vertices.data(), d_vert, n * 4, cudaMemcpyDeviceToHost), "read positions");
   uint32_t err = 0;
-  ck(cudaMemcpy(&err, d_err.p, 4, cudaMemcpyDeviceToHost), "read error");
+  ck(cudaMemcpy(&err, d_err, 4, cudaMemcpyDeviceToHost), "read error");
   if (err) throw std::invalid_argument("cgr_encode_gpu: neighbour lists must be strictly ascending");
-  ck(cudaMemset(d_bits.p + n_c, 0, 8), "clear last size");
-  scan(d_bits.p, n_c + 1);
-  ck(cudaMemcpy(&out.total_bits, d_bits.p + n_c, 8, cudaMemcpyDeviceToHost), "read total");
+  ck(cudaMemset(d_bits + n_c, 0, 8), "clear last size");
+  scan(d_bits, n_c + 1);
+  ck(cudaMemcpy(&out.total_bits, d_bits + n_c, 8, cudaMemcpyDeviceToHost), "read total");
   // 4 zero words of tail, as the host encoder
   const uint64_t nwords = (out.total_bits + 31) / 32 + 4;
-  DevBuf<uint32_t> d_words(nwords);
-  ck(cudaMemset(d_words.p, 0, nwords * 4), "clear stream");
-  ea.ctr = d_ctr.p + 1;
-  if (n_c) k_encode_write<<<blocks, kEncThreads>>>(ea, d_bits.p, d_words.p, nwords);
-  ck(cudaGetLastError(), "write pass");
-
-  // small CSR (src/compressor.cpp:267-282)
+  // the small CSR's offsets (src/compressor.cpp:267-282)
   uint64_t acc = 0;
   if (ns) {
-    k_small_degrees<<<wide, 256>>>(d_row.p, d_small, ns, d_so64.p);
+    k_small_degrees<<<wide, 256>>>(d_row, d_small, ns, d_so64);
     ck(cudaGetLastError(), "small offsets");
-    scan(d_so64.p, ns + 1);
-    k_narrow<<<wide, 256>>>(d_so64.p, ns + 1, d_so.p);
+    scan(d_so64, ns + 1);
+    k_narrow<<<wide, 256>>>(d_so64, ns + 1, d_so);
     ck(cudaGetLastError(), "small offsets");
-    // the host's pages while the device writes
-    grow(out.words, nwords);
-    grow(out.small_offset, ns + 1);
-    ck(cudaMemcpy(&acc, d_so64.p + ns, 8, cudaMemcpyDeviceToHost), "read small total");
+    ck(cudaMemcpy(&acc, d_so64 + ns, 8, cudaMemcpyDeviceToHost), "read small total");
     if (acc > 0xFFFFFFFFull) throw std::invalid_argument("cgr_encode_gpu: small CSR exceeds 2^32 arcs");
-  } else {
-    grow(out.words, nwords);
   }
-  DevBuf<uint32_t> d_sg(acc);
+  uint32_t *d_words, *d_sg;
+  mem.add(&d_words, nwords);
+  mem.add(&d_sg, acc);
+  mem.alloc();
+  ck(cudaMemset(d_words, 0, nwords * 4), "clear stream");
+  ea.ctr = d_ctr + 1;
+  k_encode_write<<<blocks, kEncThreads>>>(ea, d_bits, d_words, nwords);
+  ck(cudaGetLastError(), "write pass");
   if (acc) {
-    k_gather_small<<<wide, 256>>>(d_row.p, d_clm.p, d_small, d_so.p, ns, d_sg.p);
+    k_gather_small<<<wide, 256>>>(d_row, d_clm, d_small, d_so, ns, d_sg);
     ck(cudaGetLastError(), "small CSR gather");
-    grow(out.small_graph, acc);
   }
+  // the host's pages while the device writes
+  grow(out.words, nwords);
+  if (ns) grow(out.small_offset, ns + 1);
+  if (acc) grow(out.small_graph, acc);
   out.offsets.resize(n_c + 1);
-  ck(cudaMemcpy(out.offsets.data(), d_bits.p, (n_c + 1) * 8, cudaMemcpyDeviceToHost), "read offsets");
-  ck(cudaMemcpy(&err, d_err.p, 4, cudaMemcpyDeviceToHost), "read error");
+  ck(cudaMemcpy(out.offsets.data(), d_bits, (n_c + 1) * 8, cudaMemcpyDeviceToHost), "read offsets");
+  ck(cudaMemcpy(&err, d_err, 4, cudaMemcpyDeviceToHost), "read error");
   if (err) throw std::runtime_error("cgr_encode_gpu: a vertex's bits did not end at its offset");
-  ck(cudaMemcpy(out.words.data(), d_words.p, nwords * 4, cudaMemcpyDeviceToHost), "read stream");
-  if (ns) ck(cudaMemcpy(out.small_offset.data(), d_so.p, (ns + 1) * 4, cudaMemcpyDeviceToHost), "read small offsets");
-  if (acc) ck(cudaMemcpy(out.small_graph.data(), d_sg.p, acc * 4, cudaMemcpyDeviceToHost), "read small CSR");
+  ck(cudaMemcpy(out.words.data(), d_words, nwords * 4, cudaMemcpyDeviceToHost), "read stream");
+  if (ns) ck(cudaMemcpy(out.small_offset.data(), d_so, (ns + 1) * 4, cudaMemcpyDeviceToHost), "read small offsets");
+  if (acc) ck(cudaMemcpy(out.small_graph.data(), d_sg, acc * 4, cudaMemcpyDeviceToHost), "read small CSR");
 }
 
 }  // namespace lpa
