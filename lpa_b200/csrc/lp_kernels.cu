@@ -1401,15 +1401,14 @@ __device__ __forceinline__ void decode_records(const IterArgs &a, const Ctx &c, 
     const uint32_t incl = warp_incl_scan(cnt, lane);
     const uint32_t excl = incl - cnt;
     const uint32_t tot = __shfl_sync(kFull, incl, 31);
-    // window item f of lane l goes to sc[drel_l + f] (32-bit arithmetic) when
-    // every lane's items lie within 2^31 of lane 0's first
+    // window item f of lane l goes to sc[drel_l + f].  32 bits do: the records of
+    // a group are neighbours in one plan segment, so their items lie within its
+    // 16384 arcs, or, of a hub, within the group's own residual labels
     const uint64_t i0 = (uint64_t(__shfl_sync(kFull, uint32_t(index >> 32), 0)) << 32) |
                         __shfl_sync(kFull, uint32_t(index), 0);
     uint32_t *sb = i0 >= a.hub_arcs ? a.scratch_rest : a.scratch;  // a plan segment is all hub or none
     uint32_t *sc = sb + i0;
-    const int64_t away = int64_t(index - i0);
-    const bool rel32 = __all_sync(kFull, cnt == 0u || (away > -(1ll << 30) && away < (1ll << 30))) && tot < 1u << 30;
-    const int32_t drel = int32_t(away) - int32_t(excl);
+    const int32_t drel = int32_t(index - i0) - int32_t(excl);
     uint32_t done = 0, v = 0;
     for (uint32_t w0 = 0; w0 < tot; w0 += kDecodeWindow) {
       const uint32_t w1 = min(w0 + kDecodeWindow, tot);
@@ -1444,24 +1443,12 @@ __device__ __forceinline__ void decode_records(const IterArgs &a, const Ctx &c, 
                   : (kGather == 2 || (kGather == 0 && id < hot)) ? __ldg(c.lab_in + id)
                                                                   : ld_cg_keep(c.lab_in + id, keep_pol);
         }
-        if (rel32) {
 #pragma unroll
-          for (int u = 0; u < 8; u++) {
-            const uint32_t f = f0 + 32u * u + lane;
-            const uint32_t ol = f < w1 ? (kPack ? wst[f - w0] >> 27 : wown[f - w0]) : 0u;
-            const int32_t rel = __shfl_sync(kFull, drel, ol) + int32_t(f);
-            if (f < w1) __stcs(sc + rel, lv[u]);
-          }
-        } else {
-#pragma unroll
-          for (int u = 0; u < 8; u++) {
-            const uint32_t f = f0 + 32u * u + lane;
-            const uint32_t ol = f < w1 ? (kPack ? wst[f - w0] >> 27 : wown[f - w0]) : 0u;
-            const uint64_t ob = (uint64_t(__shfl_sync(kFull, uint32_t(index >> 32), ol)) << 32) |
-                                __shfl_sync(kFull, uint32_t(index), ol);
-            const uint32_t ox = __shfl_sync(kFull, excl, ol);
-            if (f < w1) __stcs(sb + ob + (f - ox), lv[u]);
-          }
+        for (int u = 0; u < 8; u++) {
+          const uint32_t f = f0 + 32u * u + lane;
+          const uint32_t ol = f < w1 ? (kPack ? wst[f - w0] >> 27 : wown[f - w0]) : 0u;
+          const int32_t rel = __shfl_sync(kFull, drel, ol) + int32_t(f);
+          if (f < w1) __stcs(sc + rel, lv[u]);
         }
       }
       __syncwarp();
