@@ -1977,13 +1977,12 @@ __device__ __forceinline__ void sketch_count(uint32_t *cms, const uint32_t *__re
 }
 
 // One share of an exact vertex's labels (BlockItem, kCountHash) by the whole
-// block: best is this thread's best of them.  keys and counts: kCountBlockSlots
-// each, zero before and after.  A share whose labels overfill the table is
+// block: best is this thread's best of them.  keys and counts (kCountBlockSlots
+// each) and *top (the count of kTopLabel) are zero before and after.  A share whose labels overfill the table is
 // counted again in 4, 16, ... parts of itself, told apart by further bits of
 // the hash (a bijection of the label: 20 bits leave at most 4096 labels).
-__device__ __noinline__ uint64_t count_share(uint32_t *keys, const uint32_t *src, uint32_t d, uint32_t lg,
-                                             uint32_t share) {
-  __shared__ uint32_t top;
+__device__ __noinline__ uint64_t count_share(uint32_t *keys, uint32_t *top, const uint32_t *src, uint32_t d,
+                                             uint32_t lg, uint32_t share) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint32_t *cnts = keys + kCountBlockSlots;
   uint64_t best = 0;
@@ -1992,9 +1991,7 @@ __device__ __noinline__ uint64_t count_share(uint32_t *keys, const uint32_t *src
     bool full = false;
     for (uint32_t part = 0; part < 1u << more && !full; part++) {
       const uint32_t want = share << more | part, sh = 32u - lg - more;
-      if (threadIdx.x == 0) top = 0;
-      __syncthreads();
-      const auto ins = [&](uint32_t lab, uint32_t c) { full |= !table_add(keys, cnts, kCountBlockSlots, &top, lab, c); };
+      const auto ins = [&](uint32_t lab, uint32_t c) { full |= !table_add(keys, cnts, kCountBlockSlots, top, lab, c); };
       WarpRun run;
       warp_stream<true, 4>(src, d, warp, kWarps, [&](bool ok, uint32_t lab) {
         ok = ok && slot_hash(lab) >> sh == want;
@@ -2015,9 +2012,10 @@ __device__ __noinline__ uint64_t count_share(uint32_t *keys, const uint32_t *src
           cnts[k] = 0u;
         }
       }
-      if (threadIdx.x == 0 && top) {
-        const uint64_t cand = pack_best(top, kTopLabel);
+      if (threadIdx.x == 0 && *top) {
+        const uint64_t cand = pack_best(*top, kTopLabel);
         best = cand > best ? cand : best;
+        *top = 0u;
       }
       __syncthreads();
     }
@@ -2058,6 +2056,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_count_two_pass(IterArgs a) {
   __shared__ uint64_t red[kWarps];
   __shared__ uint64_t s_bar[kWarps];  // per warp: completion of its bulk copies
   __shared__ uint32_t s_has, s_epoch;
+  __shared__ uint32_t s_top;  // kHash: a share's count of kTopLabel
   __shared__ BlockItem s_bi;
   const DevGraph &g = a.g;
   const Ctx c = resolve(a);
@@ -2119,8 +2118,9 @@ __global__ void __launch_bounds__(kThreads, 5) k_count_two_pass(IterArgs a) {
     } else if (kHash && (it.kind & 15u) == kCountHash) {
       uint32_t *keys = reinterpret_cast<uint32_t *>(cslots);
       for (uint32_t k = t; k < 2 * kCountBlockSlots; k += kThreads) keys[k] = 0u;
+      if (t == 0) s_top = 0u;
       __syncthreads();
-      best = block_max_u64(count_share(keys, src, d, (it.kind >> 4) & 15u, it.kind >> 8), red);
+      best = block_max_u64(count_share(keys, &s_top, src, d, (it.kind >> 4) & 15u, it.kind >> 8), red);
     } else {
       // blocks small enough that every warp takes one: the critical path of
       // a vertex of 512..1024 labels is one block of 64 or 128, not 256
